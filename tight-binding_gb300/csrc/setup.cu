@@ -512,13 +512,13 @@ __global__ void k_segments(DevPairs pr, int npairs, int natoms, int2 *seg)
     if (last) seg[(long)a * natoms + b].y = p + 1;
 }
 
-// Bloch phases for a chunk of k points: ph[kk][p] = e^{2 pi i k.(dlv - q_j + q_i)}
+// Bloch phases for a chunk of k points: ph[p][kk] = e^{2 pi i k.(dlv - q_j + q_i)}
 __global__ void k_phases(DevStructure S, DevPairs pr, int npairs, const double *kq, int nk, double2 *ph)
 {
     const double tpi = 6.283185307179586;
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (t >= (long)npairs * nk) return;
-    const int p = (int)(t % npairs), kk = (int)(t / npairs);
+    const int kk = (int)(t % nk), p = (int)(t / nk);
     const int a1 = pr.jatm[2 * p] - 1, a2 = pr.jatm[2 * p + 1] - 1;
     double q[3];
     for (int c = 0; c < 3; ++c)
@@ -526,19 +526,27 @@ __global__ void k_phases(DevStructure S, DevPairs pr, int npairs, const double *
     const double dot = kq[3 * kk] * q[0] + kq[3 * kk + 1] * q[1] + kq[3 * kk + 2] * q[2];
     double sn, cs;
     sincos(tpi * dot, &sn, &cs);
-    ph[(long)kk * npairs + p] = make_double2(cs, sn);
+    ph[(long)p * nk + kk] = make_double2(cs, sn);
 }
 
 // Dense Hermitian matrices for a chunk of k points; `which0` selects H/S (0) or
 // dH/dS (2).  Column-major, leading dimension nv.  One CTA per pair of 32 x 32
-// tiles (R, C), R <= C: thread (row tr, column tc) forms elements (32 R + tr,
-// 32 C + tc + 8 q), q < 4.  Element (r, c) is the sum over the images of its
-// atom pair taken in the reference's upper storage (min-atom row, max-atom
-// column) and conjugated when (r, c) is the lower one, so the two elements of
-// a mirrored pair are conjugates of one sum: off the diagonal tiles each sum is
-// formed once and its conjugate written to (c, r) through a shared-memory
-// transpose (coalesced both ways), halving the FP64 work; diagonal tiles form
-// every element.  The values are those of one thread per element.
+// tiles (R, C), R <= C, and per group of BLOCH_K k points: thread (row tr,
+// column tc) forms elements (32 R + tr, 32 C + tc + 8 q), q < 4.  Element (r, c)
+// is the sum over the images of its atom pair taken in the reference's upper
+// storage (min-atom row, max-atom column) and conjugated when (r, c) is the
+// lower one, so the two elements of a mirrored pair are conjugates of one sum:
+// off the diagonal tiles each sum is formed once and its conjugate written to
+// (c, r) through a shared-memory transpose (coalesced both ways), halving the
+// FP64 work; diagonal tiles form every element.  The values are those of one
+// thread per element.
+// Bound: the FP64 pipe (4 FMAs per element, image and k).  The k points are
+// spread over the grid because a small cell has few tiles: with every k in one
+// CTA an 8-atom sp3 cell (N = 32) took 5.0 ms a call for 125 k against 0.17
+// spread, and a one-atom cell's 1728 k 197 ms.  BLOCH_K = 4 k of one element
+// share the loads of its Slater-Koster entries, whose latency (not the FMAs)
+// set the pace of larger cells too: N = 288, 64 k 1.42 -> 0.61 ms a call,
+// N = 1152, 27 k 0.86 -> 0.62.
 __device__ __forceinline__ void bloch_elem(const DevStructure &S, const DevSK &sk, int npairs, const int2 *seg,
                                            const int *orb_atom, const int *ksk, int r, int c, int which0,
                                            int &a1, int &a2, int &oi, int &oj, bool &conjg, int2 &sg, double &on1,
@@ -564,9 +572,10 @@ k_bloch_build(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, co
               const int *orb_atom, const int *ksk, const double2 *ph, int nk, int nv, int which0,
               double2 *M1, double2 *M2, int jsover)
 {
-    __shared__ double2 t1[32][33], t2[32][33];   // [row in R][column in C]
-    // tile pair of this CTA: blockIdx.x = C (C + 1) / 2 + R
-    const int u = blockIdx.x;
+    __shared__ double2 t[2][BLOCH_K][32][9];   // [matrix][k][row in R][8 columns of C], conjugated
+    // k group and tile pair of this CTA: blockIdx.x = pairs x group + C (C + 1) / 2 + R
+    const int tiles = (nv + 31) / 32, tpairs = tiles * (tiles + 1) / 2;
+    const int kg = blockIdx.x / tpairs, u = blockIdx.x - kg * tpairs;
     int C = (int)((sqrtf(8.f * u + 1.f) - 1.f) * 0.5f);
     while ((C + 1) * (C + 2) / 2 <= u) ++C;
     while (C * (C + 1) / 2 > u) --C;
@@ -574,64 +583,69 @@ k_bloch_build(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, co
     const bool diag = R == C;
     const int tr = threadIdx.x & 31, tc = threadIdx.x >> 5;
     const int r = 32 * R + tr;
+    const int kk0 = kg * BLOCH_K, kn = min(BLOCH_K, nk - kk0);
     const double *E1 = sk.E + (long)which0 * npairs * 81;
     const double *E2 = sk.E + (long)(which0 + 1) * npairs * 81;
-    int a1[4], a2[4], oi[4], oj[4];
-    bool conjg[4], ok[4];
-    int2 sg[4];
-    double on1[4], on2[4];
-#pragma unroll
+    const long nn = (long)nv * nv;
+    double2 *m1 = M1 + kk0 * nn, *m2 = M2 + kk0 * nn;
+#pragma unroll 1
     for (int q = 0; q < 4; ++q) {
         const int c = 32 * C + tc + 8 * q;
-        ok[q] = r < nv && c < nv;
-        if (ok[q]) bloch_elem(S, sk, npairs, seg, orb_atom, ksk, r, c, which0, a1[q], a2[q], oi[q], oj[q], conjg[q],
-                              sg[q], on1[q], on2[q]);
-    }
-    for (int kk = 0; kk < nk; ++kk) {
-        const double2 *phk = ph + (long)kk * npairs;
-        double2 *m1 = M1 + (long)kk * nv * nv, *m2 = M2 + (long)kk * nv * nv;
+        if (32 * C + 8 * q >= nv) break;   // uniform
+        if (r < nv && c < nv) {
+            int a1, a2, oi, oj;
+            bool conjg;
+            int2 sg;
+            double on1, on2;
+            bloch_elem(S, sk, npairs, seg, orb_atom, ksk, r, c, which0, a1, a2, oi, oj, conjg, sg, on1, on2);
+            double h_re[BLOCH_K], h_im[BLOCH_K], s_re[BLOCH_K], s_im[BLOCH_K];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (!ok[q]) continue;
-            const int c = 32 * C + tc + 8 * q;
-            double h_re = 0, h_im = 0, s_re = 0, s_im = 0;
-            for (int p = sg[q].x; p < sg[q].y; ++p) {
-                const double2 z = phk[p];
-                const double e1 = E1[(long)p * 81 + oi[q] * 9 + oj[q]];
-                h_re += e1 * z.x;
-                h_im += e1 * z.y;
-                if (jsover) {
-                    const double e2 = E2[(long)p * 81 + oi[q] * 9 + oj[q]];
-                    s_re += e2 * z.x;
-                    s_im += e2 * z.y;
+            for (int kk = 0; kk < BLOCH_K; ++kk) h_re[kk] = h_im[kk] = s_re[kk] = s_im[kk] = 0;
+            for (int p = sg.x; p < sg.y; ++p) {
+                const double2 *phk = ph + (long)p * nk + kk0;
+                const double e1 = E1[(long)p * 81 + oi * 9 + oj];
+                const double e2 = jsover ? E2[(long)p * 81 + oi * 9 + oj] : 0.0;
+#pragma unroll
+                for (int kk = 0; kk < BLOCH_K; ++kk) {
+                    if (kk >= kn) break;   // uniform
+                    const double2 z = phk[kk];
+                    h_re[kk] += e1 * z.x;
+                    h_im[kk] += e1 * z.y;
+                    if (jsover) {
+                        s_re[kk] += e2 * z.x;
+                        s_im[kk] += e2 * z.y;
+                    }
                 }
             }
-            h_re += on1[q];
-            if (jsover) s_re += on2[q];
-            else s_re = (r == c && which0 == 0) ? 1.0 : 0.0;
-            if (conjg[q]) { h_im = -h_im; s_im = -s_im; }
             const long off = r + (long)c * nv;
-            m1[off] = make_double2(h_re, h_im);
-            m2[off] = make_double2(s_re, s_im);
-            if (!diag) {
-                t1[tr][tc + 8 * q] = make_double2(h_re, -h_im);
-                t2[tr][tc + 8 * q] = make_double2(s_re, -s_im);
-            }
-        }
-        if (!diag) {
-            // (c, r) = conj (r, c): rows 32 C + tr, columns 32 R + tc + 8 q
-            __syncthreads();
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int rr = 32 * C + tr, cc = 32 * R + tc + 8 * q;
-                if (rr < nv && cc < nv) {
-                    const long off = rr + (long)cc * nv;
-                    m1[off] = t1[tc + 8 * q][tr];
-                    m2[off] = t2[tc + 8 * q][tr];
+            for (int kk = 0; kk < BLOCH_K; ++kk) {
+                if (kk >= kn) break;
+                h_re[kk] += on1;
+                if (jsover) s_re[kk] += on2;
+                else s_re[kk] = (r == c && which0 == 0) ? 1.0 : 0.0;
+                if (conjg) { h_im[kk] = -h_im[kk]; s_im[kk] = -s_im[kk]; }
+                m1[kk * nn + off] = make_double2(h_re[kk], h_im[kk]);
+                m2[kk * nn + off] = make_double2(s_re[kk], s_im[kk]);
+                if (!diag) {
+                    t[0][kk][tr][tc] = make_double2(h_re[kk], -h_im[kk]);
+                    t[1][kk][tr][tc] = make_double2(s_re[kk], -s_im[kk]);
                 }
             }
-            __syncthreads();
         }
+        if (diag) continue;   // uniform
+        // (c, r) = conj (r, c): eight rows c of column r per k, 128 bytes together
+        __syncthreads();
+        const int cl = threadIdx.x & 7, rl = threadIdx.x >> 3;
+        const int rr = 32 * C + 8 * q + cl, cc = 32 * R + rl;
+        if (rr < nv && cc < nv) {
+            const long off = rr + (long)cc * nv;
+            for (int kk = 0; kk < kn; ++kk) {
+                m1[kk * nn + off] = t[0][kk][rl][cl];
+                m2[kk * nn + off] = t[1][kk][rl][cl];
+            }
+        }
+        __syncthreads();
     }
 }
 
