@@ -52,8 +52,16 @@ int nrltb_bench_cgemm_run(nrltb_ctx *ctx, int method, int m, int n, int k, int o
                           int triB, int triC, const float alpha[2], const float beta[2], const float *A,
                           int lda, const float *B, int ldb, float *C, int ldc);
 
+/* One FP64 complex GEMM of the eigensolver on caller data, for accuracy checks:
+ * C = alpha op(A) op(B) + beta C for `batch` matrices stored one after another,
+ * real alpha and beta, op and triangle flags as above; method 1 = the library's
+ * dispatch (the digit products, the FMA pipe for small shapes), 2 = the FMA pipe. */
+int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, int k, int batch, int opA, int opB, int triA,
+                          int triB, int triC, double alpha, double beta, const double *A, int lda, const double *B,
+                          int ldb, double *C, int ldc);
+
 /* Fault flags of the tcgen05 kernels: bit 0 the FP32 GEMM, bit 1 the
- * refinement's digit product; a bit is set once a bounded barrier wait inside
+ * refinement's digit product, bit 2 the FP64 GEMM's; a bit is set once a bounded barrier wait inside
  * that kernel ran out (the kernel then leaves its output untouched).
  * clear = 1 resets both. */
 int nrltb_bench_umma_fault(int clear);

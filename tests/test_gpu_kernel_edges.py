@@ -1,5 +1,7 @@
 """Kernels at the sizes where their tiling can go wrong: edges of tiles, remainders, the smallest and the
 largest of a range."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -27,3 +29,101 @@ def test_bloch_sums_over_k_groups_and_tiles(ctx, natoms, basis, nk):
         want = oracle.setham(st, par, km, which)
         for g, o in zip(got, want):
             assert np.abs(g - o).max() <= 1e-13 * max(np.abs(o).max(), 1e-300)
+
+
+def _cplx(rng, shape):
+    return rng.normal(size=shape) + 1j * rng.normal(size=shape)
+
+
+def _zgemm(ctx, method, opA, opB, tri, alpha, beta, A, B, Cm):
+    """C = alpha op(A) op(B) + beta C; A, B, C as (batch, column, row) arrays."""
+    m, n = Cm.shape[2], Cm.shape[1]
+    k = A.shape[2] if opA else A.shape[1]
+    A, B, out = np.ascontiguousarray(A), np.ascontiguousarray(B), np.ascontiguousarray(Cm).copy()
+    rc = ctx.lib.nrltb_bench_zgemm_run(ctx.h, method, m, n, k, out.shape[0], opA, opB, *tri, alpha, beta,
+                                       C.c_void_p(A.ctypes.data), A.shape[2], C.c_void_p(B.ctypes.data), B.shape[2],
+                                       C.c_void_p(out.ctypes.data), m)
+    assert rc == 0 and ctx.lib.nrltb_bench_umma_fault(0) == 0
+    return out
+
+
+def _zgemm_check(got, M, N, Cm, tri, alpha, beta):
+    """Bound of the digit products: the operands' rounding (2^-56 of a power of two that is at most twice the row's
+    or column's largest part, for both factors), the pairs dropped and the unit of the 64-bit sums, below
+    K 2^-51 row maximum x column maximum in all; and two roundings of the result.  Held by 200 elements against
+    extended precision, by all against double precision with that reference's own K 2^-52 |M| |N|."""
+    K = M.shape[2]
+    want = alpha * (M @ N) + beta * Cm.transpose(0, 2, 1)
+    part = lambda x: np.maximum(np.abs(x.real), np.abs(x.imag))
+    bound = K * 2.0 ** -51 * part(M).max(2)[:, :, None] * part(N).max(1)[:, None, :]
+    bound = bound + 2.0 ** -52 * (np.abs(want) + np.abs(M @ N))
+    m, n = want.shape[1:]
+    use = np.tril(np.ones((m, n), bool)) if tri[2] == 1 else np.triu(np.ones((m, n), bool)) if tri[2] == 2 else \
+        np.ones((m, n), bool)
+    got = got.transpose(0, 2, 1)
+    assert ((np.abs(got - want) <= bound + K * 2.0 ** -52 * (np.abs(M) @ np.abs(N))) | ~use).all()
+    rng = np.random.default_rng(0)
+    at = np.argwhere(np.broadcast_to(use, want.shape))
+    L = np.clongdouble
+    for b, i, j in at[rng.integers(0, len(at), 200)]:
+        v = alpha * (M[b, i].astype(L) * N[b, :, j].astype(L)).sum() + beta * Cm[b, j, i]
+        assert abs(complex(got[b, i, j] - v)) <= bound[b, i, j]
+
+
+@pytest.mark.parametrize("m,n,k,batch", [(16, 16, 16, 3), (128, 64, 32, 1), (129, 65, 33, 2), (127, 63, 31, 2),
+                                         (300, 200, 257, 2), (15, 16, 16, 1), (700, 33, 64, 5)])
+@pytest.mark.parametrize("opA,opB", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_fp64_product_shapes(ctx, m, n, k, batch, opA, opB):
+    """The digit products at the edges of their 128 x 64 x 32 tiles and of the rule that selects them."""
+    rng = np.random.default_rng(m + n + k)
+    A, B = _cplx(rng, (batch, m, k) if opA else (batch, k, m)), _cplx(rng, (batch, k, n) if opB else (batch, n, k))
+    Cm = _cplx(rng, (batch, n, m))
+    M = A.conj() if opA else A.transpose(0, 2, 1)
+    N = B.conj() if opB else B.transpose(0, 2, 1)
+    for alpha, beta in ((1.0, 0.0), (-1.0, 1.0)):
+        _zgemm_check(_zgemm(ctx, 1, opA, opB, (0, 0, 0), alpha, beta, A, B, Cm), M, N, Cm, (0, 0, 0), alpha, beta)
+
+
+@pytest.mark.parametrize("n,batch", [(65, 1), (200, 6), (385, 5)])
+@pytest.mark.parametrize("tri", [(1, 0, 0), (2, 0, 0), (0, 1, 0), (0, 2, 0), (0, 0, 1), (0, 0, 2), (1, 0, 1), (2, 0, 2)])
+def test_fp64_product_triangles(ctx, n, batch, tri):
+    """Every triangle form: the other half of a triangular operand is never read (NaN there)."""
+    rng = np.random.default_rng(n)
+    A, B, Cm = (_cplx(rng, (batch, n, n)) for _ in range(3))
+    M, N = A.transpose(0, 2, 1).copy(), B.transpose(0, 2, 1).copy()
+    low = np.tril(np.ones((n, n), bool))
+    if tri[0]:
+        M[:, ~(low if tri[0] == 1 else low.T)] = np.nan
+    if tri[1]:
+        N[:, ~(low.T if tri[1] == 1 else low)] = np.nan
+    got = _zgemm(ctx, 1, 0, 0, tri, 1.0, 0.0, M.transpose(0, 2, 1), N.transpose(0, 2, 1), Cm)
+    _zgemm_check(got, np.nan_to_num(M), np.nan_to_num(N), Cm, tri, 1.0, 0.0)
+
+
+@pytest.mark.parametrize("scale", [0.0, 1e-320, 1e-160, 1e-30, 1e150, 1e300])
+def test_fp64_product_scales_and_specials(ctx, scale):
+    """Row scales from subnormal to near overflow; zero rows; one large element; infinities and NaN reach every
+    element of their row and column and no other."""
+    rng = np.random.default_rng(3)
+    A, B, Cm = _cplx(rng, (1, 70, 150)), _cplx(rng, (1, 80, 70)), np.zeros((1, 80, 150), complex)
+    A[0, :, 7] *= scale
+    A[0, 3, 9] = 1e6
+    M, N = A.transpose(0, 2, 1), B.transpose(0, 2, 1)
+    got = _zgemm(ctx, 1, 0, 0, (0, 0, 0), 1.0, 0.0, A, B, Cm).transpose(0, 2, 1)
+    # (the scaled row against itself unscaled: digits and sums depend on the scale by an exponent only)
+    unit = scale if scale else 1.0
+    by_unit = lambda x: x.real / unit + 1j * (x.imag / unit)   # (numpy's complex quotient overflows at 1e-320)
+    want = np.vstack([M[0, :7] @ N[0], by_unit(M[0, 7:8]) @ N[0], M[0, 8:] @ N[0]])
+    have = got[0].copy()
+    have[7] = by_unit(have[7])
+    size = np.abs(M[0]).max(1) * np.abs(N).max()
+    size[7] /= unit
+    tiny = 70 * 2.0 ** -1073 / unit * np.abs(N).max()   # a subnormal row has no more bits
+    assert (np.abs(have - want) <= (70 * 2.0 ** -49 * size + (np.arange(150) == 7) * tiny)[:, None]).all()
+    for special in (np.inf, np.nan):
+        A2, B2 = A.copy(), B.copy()
+        A2[0, 5, 140], B2[0, 11, 20] = special, complex(0, special)
+        got = _zgemm(ctx, 1, 0, 0, (0, 0, 0), 1.0, 0.0, A2, B2, Cm).transpose(0, 2, 1)[0]
+        hit = np.zeros((150, 80), bool)
+        hit[140], hit[:, 11] = True, True
+        assert (np.isfinite(got) == ~hit).all()

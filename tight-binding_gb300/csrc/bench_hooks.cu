@@ -320,7 +320,41 @@ extern "C" int nrltb_bench_cgemm_run(nrltb_ctx *ctx, int method, int m, int n, i
     return cudaGetLastError() == cudaSuccess ? NRLTB_OK : NRLTB_E_CUDA;
 }
 
+extern "C" int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, int k, int batch, int opA, int opB,
+                                     int triA, int triB, int triC, double alpha, double beta, const double *A,
+                                     int lda, const double *B, int ldb, double *C, int ldc)
+{
+    if (!ctx || m < 1 || n < 1 || k < 1 || batch < 1 || !A || !B || !C || method < 1 || method > 2) return NRLTB_E_ARG;
+    const long ra = opA ? k : m, ca = opA ? m : k, rb = opB ? n : k, cb = opB ? k : n;
+    if (lda < ra || ldb < rb || ldc < m) return NRLTB_E_ARG;
+    const long na = (long)lda * ca, nb = (long)ldb * cb, nc = (long)ldc * n;
+    cudaStream_t s = nrltb_ctx_stream_internal(ctx);
+    DevBufs d;
+    ZScratch zs;
+    zs.bytes = zgemm64_scratch_bytes(std::max(m, std::max(n, k)), batch);
+    void *z = nullptr;
+    if (cudaMalloc(&d.p[0], sizeof(double2) * na * batch) != cudaSuccess ||
+        cudaMalloc(&d.p[1], sizeof(double2) * nb * batch) != cudaSuccess ||
+        cudaMalloc(&d.p[2], sizeof(double2) * nc * batch) != cudaSuccess || cudaMalloc(&z, zs.bytes + 256) != cudaSuccess)
+        return NRLTB_E_NOMEM;
+    zs.p = z;
+    const double2 al = make_double2(alpha, 0), be = make_double2(beta, 0);
+    const double2 *dA = (const double2 *)d.p[0], *dB = (const double2 *)d.p[1];
+    double2 *dC = (double2 *)d.p[2];
+    bool ok = cudaMemcpyAsync(d.p[0], A, sizeof(double2) * na * batch, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+              cudaMemcpyAsync(d.p[1], B, sizeof(double2) * nb * batch, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+              cudaMemcpyAsync(d.p[2], C, sizeof(double2) * nc * batch, cudaMemcpyHostToDevice, s) == cudaSuccess;
+    if (ok) {
+        if (method == 2) zs = ZScratch();
+        zgemm<double>(s, m, n, k, batch, al, dA, lda, na, opA, dB, ldb, nb, opB, be, dC, ldc, nc, triA, triB, triC, zs);
+        ok = cudaMemcpyAsync(C, dC, sizeof(double2) * nc * batch, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+        ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
+    }
+    cudaFree(z);
+    return ok && cudaGetLastError() == cudaSuccess ? NRLTB_OK : NRLTB_E_CUDA;
+}
+
 extern "C" int nrltb_bench_umma_fault(int clear)
 {
-    return (int)(zgemm_umma_fault(clear != 0) | (ozaki_fault(clear != 0) << 1));
+    return (int)(zgemm_umma_fault(clear != 0) | (ozaki_fault(clear != 0) << 1) | (zgemm64_fault(clear != 0) << 2));
 }

@@ -1070,9 +1070,9 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
         if (rem > 0) {
             C2 *P = w.L + (j0 + jb) + (long)j0 * ld;
             zgemm<T>(s, rem, jb, jb, B, one, P, ld, ms, 0, w.Wi + j0 + (long)j0 * ld, ld, ms, 1, zero, P, ld, ms,
-                     0, 1, 0);
+                     0, 1, 0, w.zs);
             zgemm<T>(s, rem, rem, jb, B, mone, P, ld, ms, 0, P, ld, ms, 1, one,
-                     w.L + (j0 + jb) + (long)(j0 + jb) * ld, ld, ms, 0, 0, 1);
+                     w.L + (j0 + jb) + (long)(j0 + jb) * ld, ld, ms, 0, 0, 1, w.zs);
         }
     }
     // 2. Wi = L^{-1}, bottom-up blocked: the 32 x 32 diagonal blocks are already
@@ -1089,20 +1089,20 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
             if (rem <= 0) continue;
             const long ldx = n;
             zgemm<T>(s, rem, jb, rem, B, one, w.Wi + (long)(j0 + jb) * (ld + 1), ld, ms, 0,
-                     w.L + (j0 + jb) + (long)j0 * ld, ld, ms, 0, zero, w.Xt, ldx, (long)NB2 * n, 1, 0, 0);
+                     w.L + (j0 + jb) + (long)j0 * ld, ld, ms, 0, zero, w.Xt, ldx, (long)NB2 * n, 1, 0, 0, w.zs);
             zgemm<T>(s, rem, jb, jb, B, mone, w.Xt, ldx, (long)NB2 * n, 0, w.Wi + (long)j0 * (ld + 1), ld, ms, 0,
-                     zero, w.Wi + (j0 + jb) + (long)j0 * ld, ld, ms, 0, 2, 0);
+                     zero, w.Wi + (j0 + jb) + (long)j0 * ld, ld, ms, 0, 2, 0, w.zs);
         }
     }
     // 3. A = Wi H Wi^H (lower tiles); FP32: Wi^H formed explicitly in L (free
     //    after step 2) so that both tensor-core GEMMs stream stored operands
     if (sizeof(T) == 4) {
         conj_transpose<T>(s, w.Wi, w.L, n, B);
-        zgemm<T>(s, n, n, n, B, one, w.A, ld, ms, 0, w.L, ld, ms, 0, zero, w.Y, ld, ms, 0, 1, 0);
+        zgemm<T>(s, n, n, n, B, one, w.A, ld, ms, 0, w.L, ld, ms, 0, zero, w.Y, ld, ms, 0, 1, 0, w.zs);
     } else {
-        zgemm<T>(s, n, n, n, B, one, w.A, ld, ms, 0, w.Wi, ld, ms, 1, zero, w.Y, ld, ms, 0, 1, 0);
+        zgemm<T>(s, n, n, n, B, one, w.A, ld, ms, 0, w.Wi, ld, ms, 1, zero, w.Y, ld, ms, 0, 1, 0, w.zs);
     }
-    zgemm<T>(s, n, n, n, B, one, w.Wi, ld, ms, 0, w.Y, ld, ms, 0, zero, w.A, ld, ms, 1, 0, 1);
+    zgemm<T>(s, n, n, n, B, one, w.Wi, ld, ms, 0, w.Y, ld, ms, 0, zero, w.A, ld, ms, 1, 0, 1, w.zs);
     if (tri_start) cudaEventRecord(tri_start, s);
     // 4. tridiagonalisation: one cluster launch per panel (tri_panel.cuh); the
     //    per-column launch chain below is the path for devices or sizes where
@@ -1135,10 +1135,10 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
                 NRLTB_LAUNCH(k_copy_vpanel<C2>, dim3(cdiv((long)rem * jb, 256), B), 256, 0, s, w.V, ld, ms, w.VW,
                              (long)n, w.wps, t0, j0, jb, rem);
                 zgemm<T>(s, rem, rem, 2 * EIG_NB, B, mone, w.VW + t0, n, w.wps, 0, w.VW + t0 + (long)n * EIG_NB, n,
-                         w.wps, 1, one, At, ld, ms, 0, 0, 1);
+                         w.wps, 1, one, At, ld, ms, 0, 0, 1, w.zs);
             } else {
-                zgemm<T>(s, rem, rem, jb, B, mone, Vp, ld, ms, 0, Wpp, n, w.wps, 1, one, At, ld, ms, 0, 0, 1);
-                zgemm<T>(s, rem, rem, jb, B, mone, Wpp, n, w.wps, 0, Vp, ld, ms, 1, one, At, ld, ms, 0, 0, 1);
+                zgemm<T>(s, rem, rem, jb, B, mone, Vp, ld, ms, 0, Wpp, n, w.wps, 1, one, At, ld, ms, 0, 0, 1, w.zs);
+                zgemm<T>(s, rem, rem, jb, B, mone, Wpp, n, w.wps, 0, Vp, ld, ms, 1, one, At, ld, ms, 0, 0, 1, w.zs);
             }
         }
     }
@@ -1153,7 +1153,7 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
         C2 *const G = w.Tt + (long)g * sG * B;
         const int jb = std::min(nbw, nref - j0), mb = n - j0 - 1;
         const C2 *Vb = w.V + (j0 + 1) + (long)j0 * ld;
-        zgemm<T>(st, jb, jb, mb, B, one, Vb, ld, ms, 1, Vb, ld, ms, 0, zero, G, nbw, sG);
+        zgemm<T>(st, jb, jb, mb, B, one, Vb, ld, ms, 1, Vb, ld, ms, 0, zero, G, nbw, sG, 0, 0, 0, w.zs);
         if (sizeof(T) == 4) {
             const int sm = (int)(sizeof(C2) * EIG_WY * (EIG_WY + 1));
             smem_attr_at_least((const void *)k_larft_wy<T, true>, sm);
@@ -1220,20 +1220,20 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
                 // Vb^H formed explicitly in Xt: the tensor-core GEMM streams an A
                 // operand in its stored orientation twice as fast
                 conj_transpose<T>(s, Vb, ld, ms, w.Xt, nbw, sX, mb, jb, B);
-                zgemm<T>(s, jb, n, mb, B, one, w.Xt, nbw, sX, 0, Yb, ld, ms, 0, zero, w.A, nbw, sX);
+                zgemm<T>(s, jb, n, mb, B, one, w.Xt, nbw, sX, 0, Yb, ld, ms, 0, zero, w.A, nbw, sX, 0, 0, 0, w.zs);
             } else {
-                zgemm<T>(s, jb, n, mb, B, one, Vb, ld, ms, 1, Yb, ld, ms, 0, zero, w.A, nbw, sX);
+                zgemm<T>(s, jb, n, mb, B, one, Vb, ld, ms, 1, Yb, ld, ms, 0, zero, w.A, nbw, sX, 0, 0, 0, w.zs);
             }
-            zgemm<T>(s, jb, n, jb, B, one, Tf, nbw, sG, 0, w.A, nbw, sX, 0, zero, w.L, nbw, sX, 2, 0, 0);
-            zgemm<T>(s, mb, n, jb, B, mone, Vb, ld, ms, 0, w.L, nbw, sX, 0, one, Yb, ld, ms);
+            zgemm<T>(s, jb, n, jb, B, one, Tf, nbw, sG, 0, w.A, nbw, sX, 0, zero, w.L, nbw, sX, 2, 0, 0, w.zs);
+            zgemm<T>(s, mb, n, jb, B, mone, Vb, ld, ms, 0, w.L, nbw, sX, 0, one, Yb, ld, ms, 0, 0, 0, w.zs);
         }
         if (sizeof(T) == 4) {
             // Wi^H formed explicitly in L (free again): the tensor-core GEMM
             // streams an A operand in its stored orientation twice as fast
             conj_transpose<T>(s, w.Wi, w.L, n, B);
-            zgemm<T>(s, n, n, n, B, one, w.L, ld, ms, 0, w.Y, ld, ms, 0, zero, X, ld, ms, 2, 0, 0);
+            zgemm<T>(s, n, n, n, B, one, w.L, ld, ms, 0, w.Y, ld, ms, 0, zero, X, ld, ms, 2, 0, 0, w.zs);
         } else {
-            zgemm<T>(s, n, n, n, B, one, w.Wi, ld, ms, 1, w.Y, ld, ms, 0, zero, X, ld, ms, 2, 0, 0);
+            zgemm<T>(s, n, n, n, B, one, w.Wi, ld, ms, 1, w.Y, ld, ms, 0, zero, X, ld, ms, 2, 0, 0, w.zs);
         }
     }
 }

@@ -59,6 +59,7 @@ template <typename T> struct EigWork {
     int *perm;                      // eigenvalue -> block bookkeeping, 3 n per matrix
     unsigned *counter;              // per-matrix ticket counters (last-CTA pattern)
     int *status;                    // per-matrix status
+    ZScratch zs;                    // FP64 form: digit scratch of the GEMMs (set by the caller, may be empty)
 };
 
 template <typename T> size_t eig_work_bytes(int n, int batch);

@@ -11,9 +11,9 @@
 // that touch the lower (upper) triangle of C.
 //
 // SIMT register-tiled kernel: a BM x BN tile per CTA, BK-deep k slices staged
-// through shared memory, TM x TN complex outputs per thread.  FP64 runs here
-// (GB300 has no FP64 tensor path); FP32 goes to the tensor cores
-// (gemm_umma.cu, gemm_tc.cu).
+// through shared memory, TM x TN complex outputs per thread.  The small shapes run
+// here; FP64 products go to the tensor cores as digit products (zgemm64.cu), FP32
+// ones as 3xTF32 (gemm_umma.cu, gemm_tc.cu).
 #pragma once
 #include <algorithm>
 #include "common.cuh"
@@ -278,13 +278,28 @@ void zgemm_simt(cudaStream_t s, int m, int n, int k, int batch, typename cplx<T>
     if (ev) kt_end(ev, s, KC_GEMM_SIMT, 8.0 * gemm_useful_macs(m, n, k, triA, triB, triC) * batch);
 }
 
-// FP64: SIMT FMA pipe; FP32: tensor cores (3xTF32, FP32-class accuracy)
+// FP64 products as exact digit products on the bf16 tensor cores (zgemm64.cu),
+// with caller-owned scratch for the operands' digits (zgemm64_scratch_bytes for
+// products of order up to n in every dimension); without scratch, or where one
+// matrix's digits exceed it, the FMA-pipe kernel runs
+struct ZScratch {
+    void *p = nullptr;
+    size_t bytes = 0;
+};
+constexpr size_t ZGEMM64_SCRATCH_MAX = (size_t)6 << 30;
+size_t zgemm64_scratch_bytes(int n, int batch);
+bool zgemm64_supported(const GemmArgs<double> &g);
+bool zgemm64_launch(cudaStream_t s, const GemmArgs<double> &g, const ZScratch &zs);
+unsigned zgemm64_fault(bool clear);
+
+// FP64: digit products, FMA pipe for the small shapes; FP32: tensor cores
+// (3xTF32, FP32-class accuracy)
 template <typename T>
 void zgemm(cudaStream_t s, int m, int n, int k, int batch, typename cplx<T>::t alpha,
            const typename cplx<T>::t *A, long lda, long sA, int opA,
            const typename cplx<T>::t *B, long ldb, long sB, int opB,
            typename cplx<T>::t beta, typename cplx<T>::t *C, long ldc, long sC,
-           int triA = 0, int triB = 0, int triC = 0)
+           int triA = 0, int triB = 0, int triC = 0, const ZScratch &zs = ZScratch())
 {
     if (m <= 0 || n <= 0 || batch <= 0) return;
     // tensor cores for m >= 128, n >= 64: tcgen05 (op(A) = A) from k = 32,
@@ -303,6 +318,14 @@ void zgemm(cudaStream_t s, int m, int n, int k, int batch, typename cplx<T>::t a
         else zgemm_tc_launch(s, g);
         if (ev) kt_end(ev, s, KC_GEMM_TC, 8.0 * gemm_useful_macs(m, n, k, triA, triB, triC) * batch);
     } else {
+        const GemmArgs<double> g = gemm_args<T>(m, n, k, batch, alpha, A, lda, sA, opA, B, ldb, sB, opB, beta, C,
+                                                ldc, sC, triA, triB, triC);
+        if (zgemm64_supported(g)) {
+            cudaEvent_t ev = kt_begin(s);
+            const bool done = zgemm64_launch(s, g, zs);
+            if (ev && done) kt_end(ev, s, KC_DIGIT_GEMM, 8.0 * gemm_useful_macs(m, n, k, triA, triB, triC) * batch);
+            if (done) return;
+        }
         zgemm_simt<T>(s, m, n, k, batch, alpha, A, lda, sA, opA, B, ldb, sB, opB, beta, C, ldc, sC, triA, triB,
                       triC);
     }

@@ -133,6 +133,7 @@ struct nrltb_ctx {
     DBuf d_sk, d_seg, d_ph;
     // k-chunk matrices and solver
     DBuf d_H, d_S, d_X, d_work, d_ref, d_hf, d_np, d_qw;
+    DBuf d_zs;   // digits of the FP64 products' operands (zgemm64.cu)
     DBuf d_dH, d_dS, d_ph2, d_oa;   // side stream: dH, dS, their phases, the prepared digits
     std::vector<std::pair<int, int>> nonpd;   // (k, chunk) of k points whose S is not positive definite
     // results
@@ -575,12 +576,23 @@ static int run_bloch(nrltb_ctx *c, int k0, int nk, int which0, double2 *M1, doub
 // aligned offset (double2 accesses need 16-byte alignment).
 static size_t zoff(size_t nn, int nk) { return (sizeof(float2) * nn * nk + 255) & ~size_t(255); }
 
+// digit scratch of the FP64 products of nk matrices of order nv
+static int z_scratch(nrltb_ctx *c, int nv, int nk, ZScratch &zs)
+{
+    const size_t bytes = zgemm64_scratch_bytes(nv, nk);
+    RET(c->d_zs.ensure(bytes));
+    zs.p = c->d_zs.p;
+    zs.bytes = bytes;
+    return NRLTB_OK;
+}
+
 static size_t per_k_bytes(int nv, int prec)
 {
     size_t nn = (size_t)nv * nv;
     size_t w = (prec == NRLTB_PREC_FP64) ? eig_work_bytes<double>(nv, 1) : eig_work_bytes<float>(nv, 1);
     size_t x = (prec == NRLTB_PREC_FP64) ? 16 * nn : 8 * nn;
     size_t ref = (prec == NRLTB_PREC_FP64) ? 0 : refine_work_bytes(nv, 1);
+    if (prec == NRLTB_PREC_FP64) w += zgemm64_scratch_bytes(nv, 1);
     return 32 * nn + w + x + ref + hf_scratch_bytes(nv, 1) + 64 * (size_t)nv;
 }
 
@@ -616,11 +628,13 @@ static int run_solve(nrltb_ctx *c, int nv, int nkc, int prec, const double2 *H, 
         RET(c->d_work.ensure(eig_work_bytes<double>(nv, nkc)));
         EigWork<double> w;
         eig_work_carve<double>(w, c->d_work.p, nv, nkc);
+        RET(z_scratch(c, nv, nkc, w.zs));
         // one stream: the WY factors and the tridiagonal solve both load the
         // FP64 pipe, and overlapping them measured slower
         eig_solve<double>(s, w, H, S, eig, Zout, vectors);
         CKL();
         CK(cudaMemcpyAsync(status, w.status, sizeof(int) * nkc, cudaMemcpyDeviceToDevice, s));
+        fault_mark(s, status, nkc);
     } else {
         if (!refine_available()) { set_err("mixed-precision form not built"); return NRLTB_E_UNSUPPORTED; }
         RET(c->d_work.ensure(eig_work_bytes<float>(nv, nkc)));
@@ -706,12 +720,15 @@ static int run_lowdin(nrltb_ctx *c, int nv, int nkc, const double2 *S, const dou
         RET(c->d_work.ensure(eig_work_bytes<double>(nv, nkc)));
         EigWork<double> w;
         eig_work_carve<double>(w, c->d_work.p, nv, nkc);
+        RET(z_scratch(c, nv, nkc, w.zs));
         eig_solve<double>(s, w, A, B, o, V, true);
         CKL();
         const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
-        zgemm<double>(s, nv, nv, nv, nkc, one, V, nv, (long)nn, 1, Z, nv, (long)nn, 0, zero, A, nv, (long)nn);
+        zgemm<double>(s, nv, nv, nv, nkc, one, V, nv, (long)nn, 1, Z, nv, (long)nn, 0, zero, A, nv, (long)nn, 0, 0, 0,
+                      w.zs);
         NRLTB_LAUNCH(k_lowdin_scale, cdiv(tot, 256), 256, 0, s, A, o, nv, nkc);
-        zgemm<double>(s, nv, nv, nv, nkc, one, V, nv, (long)nn, 0, A, nv, (long)nn, 0, zero, B, nv, (long)nn);
+        zgemm<double>(s, nv, nv, nv, nkc, one, V, nv, (long)nn, 0, A, nv, (long)nn, 0, zero, B, nv, (long)nn, 0, 0, 0,
+                      w.zs);
         W = B;
     }
     NRLTB_LAUNCH(k_lowdin_charges, cdiv(tot, 256), 256, 0, s, W, status, orb, nv, nkc);
@@ -737,6 +754,7 @@ static int fix_nonpd(nrltb_ctx *c, int nv, const std::vector<int> &bad, const do
     RET(c->d_work.ensure(eig_work_bytes<double>(nv, nb)));
     EigWork<double> w;
     eig_work_carve<double>(w, c->d_work.p, nv, nb);
+    RET(z_scratch(c, nv, nb, w.zs));
     eig_solve<double>(s, w, Hp, Sp, ep, nullptr, false);
     CKL();
     for (int j = 0; j < nb; ++j)
@@ -871,6 +889,7 @@ static int run_all(nrltb_ctx *c)
                 if (lqlmt && (rc = run_lowdin(c, nv, nkc, c->d_S.as<double2>(), Z, status,
                                               c->d_orbq.as<double>() + (size_t)r0 * nn)))
                     break;
+                if (lqlmt || !bad.empty()) fault_mark(s, status, nkc);   // the FP64 products of the two above
                 if (lspdir) {
                     const long nt = (long)nkc * nv * S.natoms;
                     NRLTB_LAUNCH(k_spin_expect, cdiv(nt, 256), 256, 0, s, Z, nv, nkc, S.natoms, c->d_ksk.as<int>(),
@@ -889,8 +908,10 @@ static int run_all(nrltb_ctx *c)
                     if ((rc = c->d_hf.ensure(hf_scratch_bytes(nv, nkc)))) break;
                     const double2 *dH = overlap ? c->d_dH.as<double2>() : c->d_H.as<double2>();
                     const double2 *dS = overlap ? c->d_dS.as<double2>() : c->d_S.as<double2>();
+                    ZScratch zs;
+                    if (o.precision == NRLTB_PREC_FP64 && (rc = z_scratch(c, nv, nkc, zs))) break;
                     if ((rc = run_hf(s, nv, nkc, o.precision, dH, dS, Z, eig, c->d_deig.as<double>() + (size_t)r0 * nv,
-                                     c->d_hf.p, overlap ? pre + 2 : nullptr)))
+                                     c->d_hf.p, overlap ? pre + 2 : nullptr, zs)))
                         { set_err("hf failed"); break; }
                     CKL();
                     fault_mark(s, status, nkc);
@@ -1067,7 +1088,7 @@ int nrltb_ctx_destroy(nrltb_ctx *c)
                     &c->d_sk, &c->d_seg, &c->d_ph, &c->d_H, &c->d_S, &c->d_X, &c->d_work, &c->d_ref, &c->d_hf, &c->d_np,
                     &c->d_qw, &c->d_eig, &c->d_deig, &c->d_ncut, &c->d_status, &c->d_fjob, &c->d_fout,
                     &c->d_orbq, &c->d_spev, &c->d_spdir, &c->d_fault, &c->d_dH, &c->d_dS, &c->d_ph2,
-                    &c->d_oa};
+                    &c->d_oa, &c->d_zs};
     for (DBuf *b : bufs) b->release();
     if (c->kt) {
         for (cudaEvent_t e : c->kt->pool) cudaEventDestroy(e);

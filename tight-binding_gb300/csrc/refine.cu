@@ -724,7 +724,7 @@ void launch_to_f32(cudaStream_t s, const double2 *src, float2 *dst, long count)
 }
 
 int run_hf(cudaStream_t s, int n, int nkc, int prec, const double2 *dH, const double2 *dS, const double2 *Z,
-           const double *eig, double *deig, void *scratch, const OzakiA *pre)
+           const double *eig, double *deig, void *scratch, const OzakiA *pre, const ZScratch &zs)
 {
     const long nn = (long)n * n;
     double2 *P = (double2 *)scratch;
@@ -732,8 +732,8 @@ int run_hf(cudaStream_t s, int n, int nkc, int prec, const double2 *dH, const do
     if (prec == NRLTB_PREC_FP64) {
         const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
         // P = triu(dH) Z, Q = triu(dS) Z
-        zgemm<double>(s, n, n, n, nkc, one, dH, n, nn, 0, Z, n, nn, 0, zero, P, n, nn, 2, 0, 0);
-        zgemm<double>(s, n, n, n, nkc, one, dS, n, nn, 0, Z, n, nn, 0, zero, Q, n, nn, 2, 0, 0);
+        zgemm<double>(s, n, n, n, nkc, one, dH, n, nn, 0, Z, n, nn, 0, zero, P, n, nn, 2, 0, 0, zs);
+        zgemm<double>(s, n, n, n, nkc, one, dS, n, nn, 0, Z, n, nn, 0, zero, Q, n, nn, 2, 0, 0, zs);
         launch_hf_dots(s, Z, P, Q, dH, dS, eig, deig, n, nkc);
     } else {
         // Mixed form: P = dH Z', Q = dS Z' by the tensor-core digit product with

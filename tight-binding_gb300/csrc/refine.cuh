@@ -2,6 +2,7 @@
 // eigenpairs, and the Hellmann-Feynman products of both forms.
 #pragma once
 #include "common.cuh"
+#include "gemm.cuh"
 #include "ozaki.cuh"
 
 namespace nrltb {
@@ -44,9 +45,10 @@ void refine_eigen(cudaStream_t s, RefineWork &w, const double2 *H, const double2
 // Hellmann-Feynman shifts deig = diag(Z^H dH Z) - eig * diag(Z^H dS Z) for nkc
 // matrices; scratch must hold hf_scratch_bytes(n, nkc), 256-byte aligned.
 // pre (optional, mixed form): the 3-digit forms of dH and dS from
-// ozaki_prepare_a (dH, dS are then not read).
+// ozaki_prepare_a (dH, dS are then not read).  zs (FP64 form): digit scratch.
 int run_hf(cudaStream_t s, int n, int nkc, int prec, const double2 *dH, const double2 *dS, const double2 *Z,
-           const double *eig, double *deig, void *scratch, const OzakiA *pre = nullptr);
+           const double *eig, double *deig, void *scratch, const OzakiA *pre = nullptr,
+           const ZScratch &zs = ZScratch());
 size_t hf_scratch_bytes(int n, int nkc);
 
 }  // namespace nrltb

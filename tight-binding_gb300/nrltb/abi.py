@@ -117,6 +117,8 @@ GPU_SYMBOLS = [
     ("nrltb_bench_kernel_stats", C.c_int, [_vp, C.c_int, _dp, _dp, C.POINTER(C.c_int)]),
     ("nrltb_bench_cgemm_run", C.c_int, [_vp] + [C.c_int] * 9 + [_vp, _vp, _vp, C.c_int, _vp, C.c_int, _vp,
                                                                   C.c_int]),
+    ("nrltb_bench_zgemm_run", C.c_int, [_vp] + [C.c_int] * 10 + [C.c_double] * 2 + [_vp, C.c_int, _vp, C.c_int, _vp,
+                                                                                C.c_int]),
     ("nrltb_bench_umma_fault", C.c_int, [C.c_int]),
     ("nrltb_bench_raise_fault_word", C.c_int, [_vp]),
 ]
