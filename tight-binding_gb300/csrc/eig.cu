@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cfloat>
 #include "eig.cuh"
+#include "tri_col.cuh"
 #include "tri_panel.cuh"
 
 namespace nrltb {
@@ -26,7 +27,6 @@ template <typename T> void eig_work_carve(EigWork<T> &w, void *base, int n, int 
     char *b = (char *)base;
     auto take = [&](size_t bytes) { void *p = b + off; off = align256(off + bytes); return p; };
     const size_t nn = (size_t)n * n, nb = (size_t)batch;
-    const int ncta = cdiv(n, EIG_ROWS) + 1;
     w.n = n; w.batch = batch; w.ld = n; w.mstride = (long)nn;
     w.L = (C2 *)take(sizeof(C2) * nn * nb);
     w.Wi = (C2 *)take(sizeof(C2) * nn * nb);
@@ -39,9 +39,10 @@ template <typename T> void eig_work_carve(EigWork<T> &w, void *base, int n, int 
     w.wq = (C2 *)take(sizeof(C2) * n * nb);
     w.col = (C2 *)take(sizeof(C2) * n * nb);
     w.tau = (C2 *)take(sizeof(C2) * n * nb);
-    w.pp = (C2 *)take(sizeof(C2) * 2 * EIG_NB * nb);
-    w.part = (C2 *)take(sizeof(C2) * (2 * EIG_NB + 2) * ncta * nb);
-    w.sc = (C2 *)take(sizeof(C2) * 4 * nb);
+    w.npart = (long)tc_part_count(n);
+    w.part = (C2 *)take(sizeof(C2) * w.npart * nb);
+    w.nyp = (long)tc_y_count(n);
+    w.yp = (C2 *)take(sizeof(C2) * w.nyp * nb);
     const size_t nbw = (size_t)std::min(EIG_WY, n), nblk = n > 1 ? (size_t)cdiv(n - 1, (int)nbw) : 0;
     w.Tt = (C2 *)take(sizeof(C2) * (EIG_NAUX + nblk) * nbw * nbw * nb);   // G per aux stream | T of each block
     w.Xt = (C2 *)take(sizeof(C2) * std::max(EIG_NB, (int)nbw) * (size_t)n * nb);
@@ -52,7 +53,6 @@ template <typename T> void eig_work_carve(EigWork<T> &w, void *base, int n, int 
     w.ylu = (double *)take(sizeof(double) * 4 * (size_t)n * (64 * (size_t)cdiv(n, 64)) * nb);
     w.yvec = (double *)take(sizeof(double) * nn * nb);
     w.perm = (int *)take(sizeof(int) * 4 * n * nb);
-    w.counter = (unsigned *)take(sizeof(unsigned) * nb);
     w.status = (int *)take(sizeof(int) * nb);
     if (!base) w.status = (int *)(uintptr_t)off;  // size query
 }
@@ -157,274 +157,6 @@ __global__ void __launch_bounds__(256) k_potrf_diag(EigWork<T> w, int j0, int jb
             Wi[r + (long)c * w.ld] = (r >= c) ? x[c][r] : z;
         }
     if (tid == 0 && bad) w.status[b] = 1;
-}
-
-// ---------------------------------------------------------------------------
-// Tridiagonalisation, column i of the panel starting at j0 (c = i - j0).
-// KA: finalize W[:, c-1]; update column i; reflector (last CTA).
-template <typename T>
-__global__ void __launch_bounds__(EIG_ROWS) k_tri_colupd(EigWork<T> w, int i, int j0, int ncta)
-{
-    typedef typename cplx<T>::t C2;
-    __shared__ C2 vi[EIG_NB], wi[EIG_NB];
-    __shared__ T red[EIG_ROWS / 32];
-    __shared__ unsigned ticket;
-    const int b = blockIdx.y, n = w.n, c = i - j0, tid = threadIdx.x;
-    const long ld = w.ld;
-    C2 *A = w.A + b * w.mstride, *V = w.V + b * w.mstride;
-    C2 *Wp = w.Wp + (long)b * w.wps, *wq = w.wq + (long)b * n, *col = w.col + (long)b * n;
-    const C2 alpha_prev = w.sc[b * 4 + 1];
-    // row i of the panel's V and W (W[i, c-1] recomputed from w', never read from Wp)
-    if (tid < c) {
-        vi[tid] = V[i + (long)(j0 + tid) * ld];
-        if (tid < c - 1) wi[tid] = Wp[i + (long)tid * n];
-        else wi[tid] = cadd(wq[i], cmul(alpha_prev, V[i + (long)(i - 1) * ld]));
-    }
-    __syncthreads();
-    const int r = i + blockIdx.x * EIG_ROWS + tid;
-    T nrm2 = T(0);
-    if (r < n) {
-        C2 wlast = cmk<T>(0, 0);
-        if (c > 0) {
-            wlast = cadd(wq[r], cmul(alpha_prev, V[r + (long)(i - 1) * ld]));
-            Wp[r + (long)(c - 1) * n] = wlast;
-        }
-        C2 a = A[r + (long)i * ld];
-        for (int j = 0; j < c; ++j) {
-            C2 vrj = V[r + (long)(j0 + j) * ld];
-            C2 wrj = (j < c - 1) ? Wp[r + (long)j * n] : wlast;
-            a = csub(a, cmul(vrj, cconj(wi[j])));
-            a = csub(a, cmul(wrj, cconj(vi[j])));
-        }
-        col[r] = a;
-        if (r == i) w.d[(long)b * n + i] = (double)a.x;
-        if (r >= i + 2) nrm2 = a.x * a.x + a.y * a.y;
-    }
-    __threadfence();   // col[] is read by the last CTA
-    nrm2 = block_sum(nrm2, red);
-    if (tid == 0) {
-        C2 p; p.x = nrm2; p.y = T(0);
-        w.part[((long)b * ncta + blockIdx.x) * (2 * EIG_NB + 2)] = p;
-        __threadfence();
-        ticket = atomicAdd(&w.counter[b], 1u);
-    }
-    __syncthreads();
-    if (ticket != (unsigned)(ncta - 1) || tid != 0) return;
-    // last CTA: Householder reflector (zlarfg) from col[i+1:]
-    __threadfence();
-    T xn2 = T(0);
-    for (int q = 0; q < ncta; ++q) xn2 += __ldcg(&w.part[((long)b * ncta + q) * (2 * EIG_NB + 2)].x);
-    C2 tau = cmk<T>(0, 0), scale = cmk<T>(0, 0);
-    double beta = 0.0;
-    if (i + 1 < n) {
-        C2 al;
-        al.x = __ldcg(&col[i + 1].x);
-        al.y = __ldcg(&col[i + 1].y);
-        T xnorm = sqrt(xn2);
-        if (xnorm == T(0) && al.y == T(0)) {
-            beta = (double)al.x;
-        } else {
-            T bb = sqrt(al.x * al.x + al.y * al.y + xnorm * xnorm);
-            bb = (al.x >= T(0)) ? -bb : bb;
-            tau = cmk<T>((bb - al.x) / bb, -al.y / bb);
-            C2 den = cmk<T>(al.x - bb, al.y);         // 1 / (alpha - beta)
-            T dd = den.x * den.x + den.y * den.y;
-            scale = cmk<T>(den.x / dd, -den.y / dd);
-            beta = (double)bb;
-        }
-        w.e[(long)b * n + i] = beta;
-    }
-    w.tau[(long)b * n + i] = tau;
-    w.sc[b * 4 + 0] = scale;
-    w.counter[b] = 0;
-}
-
-// KB: v = scaled column; p1 = W^H v, p2 = V^H v over the panel's previous columns.
-template <typename T>
-__global__ void __launch_bounds__(EIG_ROWS) k_tri_vdots(EigWork<T> w, int i, int j0, int ncta)
-{
-    typedef typename cplx<T>::t C2;
-    __shared__ C2 sv[EIG_ROWS];
-    __shared__ unsigned ticket;
-    const int b = blockIdx.y, n = w.n, c = i - j0, tid = threadIdx.x;
-    const long ld = w.ld;
-    C2 *V = w.V + b * w.mstride, *Wp = w.Wp + (long)b * w.wps, *col = w.col + (long)b * n;
-    const C2 scale = w.sc[b * 4 + 0];
-    const int r = i + 1 + blockIdx.x * EIG_ROWS + tid;
-    C2 v = cmk<T>(0, 0);
-    if (r < n) {
-        v = (r == i + 1) ? cmk<T>(1, 0) : cmul(col[r], scale);
-        V[r + (long)i * ld] = v;
-    }
-    if (blockIdx.x == 0)
-        for (int q = tid; q <= i; q += EIG_ROWS) V[q + (long)i * ld] = cmk<T>(0, 0);
-    sv[tid] = v;
-    __syncthreads();
-    // partial dots: thread j < c sums W[:, j]^H v, thread EIG_NB + j sums V[:, j0+j]^H v
-    C2 *part = w.part + ((long)b * ncta + blockIdx.x) * (2 * EIG_NB + 2);
-    if (tid < 2 * EIG_NB) {
-        int j = tid % EIG_NB;
-        bool isV = tid >= EIG_NB;
-        C2 s = cmk<T>(0, 0);
-        if (j < c) {
-            int r0 = i + 1 + blockIdx.x * EIG_ROWS;
-            for (int q = 0; q < EIG_ROWS && r0 + q < n; ++q) {
-                C2 m = isV ? V[r0 + q + (long)(j0 + j) * ld] : Wp[r0 + q + (long)j * n];
-                cfmac(s, m, sv[q]);
-            }
-        }
-        part[tid] = s;
-        __threadfence();
-    }
-    __syncthreads();
-    if (tid == 0) {
-        ticket = atomicAdd(&w.counter[b], 1u);
-    }
-    __syncthreads();
-    if (ticket != (unsigned)(ncta - 1)) return;
-    __threadfence();
-    if (tid < 2 * EIG_NB) {
-        C2 s = cmk<T>(0, 0);
-        for (int q = 0; q < ncta; ++q) {
-            const C2 *p = w.part + ((long)b * ncta + q) * (2 * EIG_NB + 2) + tid;
-            s.x += __ldcg(&p->x);
-            s.y += __ldcg(&p->y);
-        }
-        w.pp[b * 2 * EIG_NB + tid] = s;
-    }
-    __syncthreads();
-    if (tid == 0) w.counter[b] = 0;
-}
-
-// KC: y = A[i+1:, i+1:] v with A stored in its lower triangle.  32-row blocks,
-// 32 x 32 tiles through shared memory, 8 column slices per row.
-template <typename T>
-__global__ void __launch_bounds__(256) k_tri_hemv(EigWork<T> w, int i)
-{
-    typedef typename cplx<T>::t C2;
-    __shared__ C2 tile[32][33];
-    __shared__ C2 vs[32];
-    __shared__ C2 red[8][33];
-    const int b = blockIdx.y, n = w.n, tid = threadIdx.x;
-    const long ld = w.ld;
-    const C2 *A = w.A + b * w.mstride, *V = w.V + b * w.mstride;
-    const int base = i + 1, m = n - base;
-    const int rb = blockIdx.x, r0 = base + 32 * rb;
-    const int tr = tid & 31, tc = tid >> 5;
-    C2 acc = cmk<T>(0, 0);
-    const int ntile = cdiv(m, 32);
-    for (int t = 0; t < ntile; ++t) {
-        const int s0 = base + 32 * t;
-        __syncthreads();
-        if (tid < 32) vs[tid] = (s0 + tid < n) ? V[s0 + tid + (long)i * ld] : cmk<T>(0, 0);
-        if (t <= rb) {
-            // tile[rr][ss] = A[r0+rr, s0+ss], coalesced along rr
-            for (int e = tid; e < 1024; e += 256) {
-                int rr = e & 31, ss = e >> 5;
-                int rg = r0 + rr, sg = s0 + ss;
-                tile[rr][ss] = (rg < n && sg < n && sg <= rg) ? A[rg + (long)sg * ld] : cmk<T>(0, 0);
-            }
-        } else {
-            // tile[rr][ss] = conj(A[s0+ss, r0+rr]), coalesced along ss
-            for (int e = tid; e < 1024; e += 256) {
-                int ss = e & 31, rr = e >> 5;
-                int rg = r0 + rr, sg = s0 + ss;
-                tile[rr][ss] = (rg < n && sg < n) ? cconj(A[sg + (long)rg * ld]) : cmk<T>(0, 0);
-            }
-        }
-        __syncthreads();
-        if (t == rb) {
-            // diagonal tile: only the lower half was loaded; mirror it
-            for (int e = tid; e < 1024; e += 256) {
-                int rr = e & 31, ss = e >> 5;
-                if (ss > rr) tile[rr][ss] = cconj(tile[ss][rr]);
-            }
-            __syncthreads();
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int ss = tc + 8 * q;
-            cfma(acc, tile[tr][ss], vs[ss]);
-        }
-    }
-    red[tc][tr] = acc;
-    __syncthreads();
-    if (tid < 32) {
-        C2 s = red[0][tid];
-        for (int q = 1; q < 8; ++q) s = cadd(s, red[q][tid]);
-        int rg = r0 + tid;
-        if (rg < n) w.col[(long)b * n + rg] = s;
-    }
-}
-
-// KD: w' = tau (y - V p1 - W p2); alpha = -tau/2 (w'^H v) (last CTA).
-template <typename T>
-__global__ void __launch_bounds__(EIG_ROWS) k_tri_wupd(EigWork<T> w, int i, int j0, int ncta)
-{
-    typedef typename cplx<T>::t C2;
-    __shared__ C2 p1[EIG_NB], p2[EIG_NB];
-    __shared__ T red[EIG_ROWS / 32];
-    __shared__ unsigned ticket;
-    const int b = blockIdx.y, n = w.n, c = i - j0, tid = threadIdx.x;
-    const long ld = w.ld;
-    const C2 *V = w.V + b * w.mstride, *Wp = w.Wp + (long)b * w.wps;
-    C2 *wq = w.wq + (long)b * n;
-    const C2 *y = w.col + (long)b * n;
-    const C2 tau = w.tau[(long)b * n + i];
-    if (tid < c) {
-        p1[tid] = w.pp[b * 2 * EIG_NB + tid];
-        p2[tid] = w.pp[b * 2 * EIG_NB + EIG_NB + tid];
-    }
-    __syncthreads();
-    const int r = i + 1 + blockIdx.x * EIG_ROWS + tid;
-    T dre = T(0), dim = T(0);
-    if (r < n) {
-        C2 s = y[r];
-        for (int j = 0; j < c; ++j) {
-            s = csub(s, cmul(V[r + (long)(j0 + j) * ld], p1[j]));
-            s = csub(s, cmul(Wp[r + (long)j * n], p2[j]));
-        }
-        s = cmul(tau, s);
-        wq[r] = s;
-        C2 v = V[r + (long)i * ld];
-        dre = s.x * v.x + s.y * v.y;      // conj(w') v
-        dim = s.x * v.y - s.y * v.x;
-    }
-    if (blockIdx.x == 0)
-        for (int q = tid; q <= i; q += EIG_ROWS) wq[q] = cmk<T>(0, 0);
-    dre = block_sum(dre, red);
-    dim = block_sum(dim, red);
-    if (tid == 0) {
-        C2 p; p.x = dre; p.y = dim;
-        w.part[((long)b * ncta + blockIdx.x) * (2 * EIG_NB + 2) + 2 * EIG_NB] = p;
-        __threadfence();
-        ticket = atomicAdd(&w.counter[b], 1u);
-    }
-    __syncthreads();
-    if (ticket != (unsigned)(ncta - 1) || tid != 0) return;
-    __threadfence();
-    C2 dot = cmk<T>(0, 0);
-    for (int q = 0; q < ncta; ++q) {
-        const C2 *p = w.part + ((long)b * ncta + q) * (2 * EIG_NB + 2) + 2 * EIG_NB;
-        dot.x += __ldcg(&p->x);
-        dot.y += __ldcg(&p->y);
-    }
-    w.sc[b * 4 + 1] = cscale(cmul(tau, dot), T(-0.5));
-    w.counter[b] = 0;
-}
-
-// W[:, c] = w' + alpha v for the panel's last column.
-template <typename T>
-__global__ void k_tri_wfinal(EigWork<T> w, int i, int c)
-{
-    typedef typename cplx<T>::t C2;
-    const int b = blockIdx.y, n = w.n;
-    const C2 alpha = w.sc[b * 4 + 1];
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        C2 v = (r > i) ? w.V[b * w.mstride + r + (long)i * w.ld] : cmk<T>(0, 0);
-        C2 q = (r > i) ? w.wq[(long)b * n + r] : cmk<T>(0, 0);
-        w.Wp[(long)b * w.wps + r + (long)c * n] = cadd(q, cmul(alpha, v));
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1058,8 +790,6 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     const C2 one = cmk<T>(1, 0), mone = cmk<T>(-1, 0), zero = cmk<T>(0, 0);
     const long cnt = (long)n * n * B;
     cudaMemsetAsync(w.status, 0, sizeof(int) * B, s);
-    cudaMemsetAsync(w.counter, 0, sizeof(unsigned) * B, s);
-    cudaMemsetAsync(w.sc, 0, sizeof(C2) * 4 * B, s);
     // 0. inputs in working precision: S -> L, H -> A (A is free until step 3)
     NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, S, w.L, cnt);
     NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, H, w.A, cnt);
@@ -1104,27 +834,14 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     }
     zgemm<T>(s, n, n, n, B, one, w.Wi, ld, ms, 0, w.Y, ld, ms, 0, zero, w.A, ld, ms, 1, 0, 1, w.zs);
     if (tri_start) cudaEventRecord(tri_start, s);
-    // 4. tridiagonalisation: one cluster launch per panel (tri_panel.cuh); the
-    //    per-column launch chain below is the path for devices or sizes where
-    //    such a cluster cannot be scheduled
+    // 4. tridiagonalisation: FP32 one cluster launch per panel (tri_panel.cuh); FP64,
+    //    and where such a cluster cannot be scheduled, two launches per column
+    //    (tri_col.cuh)
     bool clusters = true;
     for (int j0 = 0; j0 < n; j0 += EIG_NB) {
         const int jb = std::min(EIG_NB, n - j0);
         if (clusters) clusters = tri_panel_launch<T>(s, w, j0, jb);
-        if (!clusters) {
-            for (int c = 0; c < jb; ++c) {
-                const int i = j0 + c;
-                const int nA = cdiv(n - i, EIG_ROWS);
-                NRLTB_LAUNCH(k_tri_colupd<T>, dim3(nA, B), EIG_ROWS, 0, s, w, i, j0, nA);
-                if (i == n - 1) break;
-                const int nB = cdiv(n - i - 1, EIG_ROWS);
-                NRLTB_LAUNCH(k_tri_vdots<T>, dim3(nB, B), EIG_ROWS, 0, s, w, i, j0, nB);
-                NRLTB_LAUNCH(k_tri_hemv<T>, dim3(cdiv(n - i - 1, 32), B), 256, 0, s, w, i);
-                NRLTB_LAUNCH(k_tri_wupd<T>, dim3(nB, B), EIG_ROWS, 0, s, w, i, j0, nB);
-            }
-            const int last = std::min(j0 + jb - 1, n - 2);
-            if (last >= j0) NRLTB_LAUNCH(k_tri_wfinal<T>, dim3(cdiv(n, 256), B), 256, 0, s, w, last, last - j0);
-        }
+        if (!clusters) tri_columns<T>(s, w, j0, jb);
         if (std::min(j0 + jb - 1, n - 2) < j0) break;
         const int t0 = j0 + jb, rem = n - t0;
         if (rem > 0) {

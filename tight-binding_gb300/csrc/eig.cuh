@@ -11,7 +11,7 @@
 //   3. A = W H W^H as two triangular GEMMs.
 //   4. A = Q T Q^H, blocked Householder tridiagonalisation (lower): per column a
 //      column update, reflector, lower-triangle Hermitian mat-vec and w update;
-//      per panel a rank-2nb trailing update as two GEMMs.
+//      per panel a rank-2nb trailing update as one GEMM.
 //   5. T (real symmetric) eigenvalues by Sturm-count bisection per unreduced
 //      block; eigenvectors by inverse iteration (dstein's factorisation and
 //      solves) in FP64, each cluster of close eigenvalues orthonormalised
@@ -28,7 +28,6 @@
 namespace nrltb {
 
 constexpr int EIG_NB = 32;          // panel width (Cholesky, inverse, tridiagonal)
-constexpr int EIG_ROWS = 128;       // rows per CTA in the column kernels
 constexpr int EIG_WY = 128;         // reflectors per block of the back-transform
 
 // Device workspace for one batch of `batch` matrices of order n.
@@ -44,12 +43,12 @@ template <typename T> struct EigWork {
     C2 *Wp;                         // panel W, n x EIG_NB per matrix (matrix stride wps)
     C2 *VW;                         // [V panel | W | V panel], n x 3 EIG_NB per matrix; Wp is its middle
     long wps;                       // matrix stride of VW and Wp
-    C2 *wq;                         // w' of the current column, n per matrix
-    C2 *col;                        // current updated column, n per matrix
+    C2 *wq;                         // w' of the current column, n per matrix (tri_panel.cuh)
+    C2 *col;                        // current updated column, n per matrix (tri_col.cuh)
     C2 *tau;                        // n per matrix
-    C2 *pp;                         // p1 | p2, 2*EIG_NB per matrix
-    C2 *part;                       // per-CTA partial sums, [batch][ncta][2*EIG_NB+2]
-    C2 *sc;                         // per-matrix scalars: [0] scale, [1] alpha
+    long npart, nyp;                // elements per matrix of part and yp
+    C2 *part;                       // per-CTA partial sums (tri_col.cuh)
+    C2 *yp;                         // y = A v, one partial per CTA of a row block (tri_col.cuh)
     C2 *Tt;                         // back-transform: G = Vb^H Vb, then the T factor of every block
     C2 *Xt;                         // EIG_NB x n per matrix
     double *d, *e;                  // tridiagonal, n per matrix
@@ -57,7 +56,6 @@ template <typename T> struct EigWork {
     double *ylu;                    // inverse-iteration scratch, 4 n per thread
     double *yvec;                   // real eigenvectors of T, n x n per matrix
     int *perm;                      // eigenvalue -> block bookkeeping, 3 n per matrix
-    unsigned *counter;              // per-matrix ticket counters (last-CTA pattern)
     int *status;                    // per-matrix status
     ZScratch zs;                    // FP64 form: digit scratch of the GEMMs (set by the caller, may be empty)
 };
