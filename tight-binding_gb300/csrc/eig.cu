@@ -237,13 +237,63 @@ __device__ void block_bounds(const double *d, const double *e, bool valid, int b
     }
 }
 
-// One thread per (matrix, row r): eigenvalue number r - b0 of r's block.
-// FP32: the matrix's d and e^2 in FP32 and the split flags of find_block are
-// staged once per CTA in shared memory (2 n floats + n bytes of dynamic shared
-// memory), so the Sturm chains read them without a conversion from FP64 per
-// step and the block search needs no FP64 work (the values are the same).
-template <typename TB>
-__global__ void k_tri_bisect(const double *dd, const double *ee, double *lamloc, int *blk, int n)
+// FP32 octasection (latency bound): seven independent Sturm chains per pass; the
+// new interval lies between the last point counting <= j eigenvalues below it and
+// the first counting more.  [a, z] shrinks to about atol.
+__device__ __forceinline__ void octasect(const float *sd, const float *se2, int b0, int b1, int j, float atol,
+                                         float pivmin, float &a, float &z)
+{
+    constexpr int NP = 7;
+    const float eps = eps_of<float>();
+    for (int it = 0; it < 64; ++it) {
+        const float h = float(1.0 / (NP + 1)) * (z - a);
+        const float tol = fmax(atol, 2.f * eps * fmax(fabs(a), fabs(z))) + pivmin;
+        float m[NP];
+        bool ok = z - a > tol;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) m[i] = a + float(i + 1) * h;
+        ok = ok && m[0] > a && m[NP - 1] < z;
+#pragma unroll
+        for (int i = 0; i + 1 < NP; ++i) ok = ok && m[i] < m[i + 1];
+        if (!ok) break;
+        float q[NP];
+        int c[NP];
+        const float d0 = sd[b0];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            q[i] = d0 - m[i];
+            if (fabs(q[i]) < pivmin) q[i] = -pivmin;
+            c[i] = q[i] < 0.f;
+        }
+        for (int k = b0 + 1; k <= b1; ++k) {
+            const float dk = sd[k], e2 = se2[k - 1];
+#pragma unroll
+            for (int i = 0; i < NP; ++i) {
+                q[i] = dk - m[i] - tri_div(e2, q[i]);
+                if (fabs(q[i]) < pivmin) q[i] = -pivmin;
+                c[i] += q[i] < 0.f;
+            }
+        }
+        float na = a, nz = z;
+        bool found = false;
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+            if (!found) {
+                if (c[i] <= j) na = m[i];
+                else { nz = m[i]; found = true; }
+            }
+        }
+        a = na;
+        z = nz;
+    }
+}
+
+// One thread per (matrix, row r): eigenvalue number r - b0 of r's block, FP32.
+// The matrix's d and e^2 in FP32 and the split flags of find_block are staged
+// once per CTA in shared memory (2 n floats + n bytes of dynamic shared memory),
+// so the Sturm chains read them without a conversion from FP64 per step and the
+// block search needs no FP64 work (the values are the same).
+__global__ void k_tri_bisect32(const double *dd, const double *ee, double *lamloc, int *blk, int n)
 {
     extern __shared__ float bis_s[];
     const int b = blockIdx.y;
@@ -251,105 +301,238 @@ __global__ void k_tri_bisect(const double *dd, const double *ee, double *lamloc,
     const double *d = dd + (long)b * n, *e = ee + (long)b * n;
     float *sd = bis_s, *se2 = bis_s + n;
     unsigned char *ssp = (unsigned char *)(bis_s + 2 * n);
-    if (sizeof(TB) == 4) {
-        for (int k = threadIdx.x; k < n; k += blockDim.x) {
-            sd[k] = d2f_rn(d[k]);
-            const float ek = d2f_rn(e[k]);
-            se2[k] = ek * ek;
-            // find_block's split test, once per row
-            ssp[k] = k < n - 1 && fabs(d[k] * d[k + 1]) * DBL_EPSILON * DBL_EPSILON + DBL_MIN >= e[k] * e[k];
-        }
-        __syncthreads();
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        sd[k] = d2f_rn(d[k]);
+        const float ek = d2f_rn(e[k]);
+        se2[k] = ek * ek;
+        // find_block's split test, once per row
+        ssp[k] = k < n - 1 && fabs(d[k] * d[k + 1]) * DBL_EPSILON * DBL_EPSILON + DBL_MIN >= e[k] * e[k];
     }
+    __syncthreads();
     const bool valid = r < n;
     int b0 = 0, b1 = -1;
-    if (valid) {
-        if (sizeof(TB) == 4) find_block_flags(ssp, n, r, b0, b1);
-        else find_block(d, e, n, r, b0, b1);
-    }
+    if (valid) find_block_flags(ssp, n, r, b0, b1);
     double tnorm = 0, lo = 1e300, hi = -1e300, emax2 = 0;
     block_bounds(d, e, valid, b0, b1, lo, hi, tnorm, emax2);
     if (!valid) return;
-    const TB eps = eps_of<TB>();
-    const TB pivmin = tiny_of<TB>() * TB(fmax(1.0, emax2));
-    const TB atol = eps * TB(tnorm);
+    const float eps = eps_of<float>();
+    const float pivmin = tiny_of<float>() * float(fmax(1.0, emax2));
+    const float atol = eps * float(tnorm);
     const int j = r - b0;
-    TB a = TB(lo) - TB(2) * atol - pivmin, z = TB(hi) + TB(2) * atol + pivmin;
-    // Sturm count: eigenvalues of the block below x (FP32: from the shared
-    // copies, the same values as converting d and e here)
-    auto count = [&](TB x) {
+    float a = float(lo) - 2.f * atol - pivmin, z = float(hi) + 2.f * atol + pivmin;
+    // Sturm count: eigenvalues of the block below x (from the shared copies, the
+    // same values as converting d and e here)
+    auto count = [&](float x) {
         int cnt = 0;
-        TB q = (sizeof(TB) == 4 ? TB(sd[b0]) : TB(d[b0])) - x;
+        float q = sd[b0] - x;
         if (fabs(q) < pivmin) q = -pivmin;
-        cnt += (q < TB(0));
+        cnt += (q < 0.f);
         for (int k = b0 + 1; k <= b1; ++k) {
-            TB e2;
-            if (sizeof(TB) == 4) {
-                e2 = TB(se2[k - 1]);
-            } else {
-                const TB ek = TB(e[k - 1]);
-                e2 = ek * ek;
-            }
-            q = (sizeof(TB) == 4 ? TB(sd[k]) : TB(d[k])) - x - e2 / q;
+            q = sd[k] - x - se2[k - 1] / q;
             if (fabs(q) < pivmin) q = -pivmin;
-            cnt += (q < TB(0));
+            cnt += (q < 0.f);
         }
         return cnt;
     };
-    if (sizeof(TB) == 4) {
-        // FP32 (latency bound): octasection, seven independent Sturm chains per
-        // pass; the new interval lies between the last point counting <= j
-        // eigenvalues below it and the first counting more
-        constexpr int NP = 7;
-        for (int it = 0; it < 64; ++it) {
-            const TB h = TB(1.0 / (NP + 1)) * (z - a);
-            const TB tol = fmax(atol, TB(2) * eps * fmax(fabs(a), fabs(z))) + pivmin;
-            TB m[NP];
-            bool ok = z - a > tol;
-#pragma unroll
-            for (int i = 0; i < NP; ++i) m[i] = a + TB(i + 1) * h;
-            ok = ok && m[0] > a && m[NP - 1] < z;
-#pragma unroll
-            for (int i = 0; i + 1 < NP; ++i) ok = ok && m[i] < m[i + 1];
-            if (!ok) break;
-            TB q[NP];
-            int c[NP];
-            const TB d0 = TB(sd[b0]);
-#pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                q[i] = d0 - m[i];
-                if (fabs(q[i]) < pivmin) q[i] = -pivmin;
-                c[i] = q[i] < TB(0);
-            }
-            for (int k = b0 + 1; k <= b1; ++k) {
-                const TB dk = TB(sd[k]), e2 = TB(se2[k - 1]);
-#pragma unroll
-                for (int i = 0; i < NP; ++i) {
-                    q[i] = dk - m[i] - tri_div(e2, q[i]);
-                    if (fabs(q[i]) < pivmin) q[i] = -pivmin;
-                    c[i] += q[i] < TB(0);
-                }
-            }
-            TB na = a, nz = z;
-            bool found = false;
-#pragma unroll
-            for (int i = 0; i < NP; ++i) {
-                if (!found) {
-                    if (c[i] <= j) na = m[i];
-                    else { nz = m[i]; found = true; }
-                }
-            }
-            a = na;
-            z = nz;
-        }
-    }
-    for (int it = 0; it < 256; ++it) {   // bisection (FP64; FP32 finishes here)
-        const TB mid = TB(0.5) * (a + z);
-        const TB tol = fmax(atol, TB(2) * eps * fmax(fabs(a), fabs(z))) + pivmin;
+    octasect(sd, se2, b0, b1, j, atol, pivmin, a, z);
+    for (int it = 0; it < 256; ++it) {
+        const float mid = 0.5f * (a + z);
+        const float tol = fmax(atol, 2.f * eps * fmax(fabs(a), fabs(z))) + pivmin;
         if (!(z - a > tol) || mid == a || mid == z) break;
         if (count(mid) <= j) a = mid; else z = mid;
     }
-    lamloc[(long)b * n + r] = (double)(TB(0.5) * (a + z));
+    lamloc[(long)b * n + r] = (double)(0.5f * (a + z));
+    blk[((long)b * n + r) * 2 + 0] = b0;
+    blk[((long)b * n + r) * 2 + 1] = b1;
+}
+
+// FP64 eigenvalues.  The FP64 pipe is 1/64 of the FP32 one and a quotient takes a
+// dozen of its operations, so (a) FP32 octasection on a scaled copy of T finds each
+// eigenvalue to ~1e-7 ||T||, (b) an FP64 bracket around that is verified by Sturm
+// counts, widening until it holds, and (c) it is closed on the zero of the
+// characteristic polynomial by false position (Illinois weights, halved where that
+// stalls or several eigenvalues share the bracket), every step kept by its count.
+// Counts and polynomial values come from one recurrence without quotients,
+//   p_k = (d_k - x) p_(k-1) - e_(k-1)^2 p_(k-2),
+// three FP64 operations a step; sign changes count the eigenvalues below x
+// (Givens), and the exponents of p_k, p_(k-1) are brought back by integer adds every
+// fourth step.  A computed p_k is the exact one of entries d_k - x and e^2 changed by a
+// few ulp, the same backward error as the quotient recurrence.  The bracket ends at
+// the width the bisection alone ended at: max(eps ||T||, 2 eps |lambda|).
+// About 9 recurrences an eigenvalue in place of 54 quotient ones:
+// N = 1152, 4 k 36.7 -> 3.0 ms; N = 288, 64 k 15.8 -> 0.8 ms.
+struct TriPoly {
+    double m;      // mantissa part and binary exponent of p_n(x)
+    int ex, cnt;   // eigenvalues of the block below x
+};
+// d, e2: the block's rows scaled so that the largest row sum is about 1
+__device__ __forceinline__ TriPoly tri_poly(const double *d, const double *e2, int b0, int b1, double x)
+{
+    double p0 = 1.0, p1 = d[b0] - x;
+    int ex = 0, cnt = 0;
+    // an exact zero counts as a sign change (the quotient form's -pivmin)
+    auto nz = [](double p, double prev) {
+        if ((__double_as_longlong(p) << 1) == 0)
+            p = __longlong_as_double((__double_as_longlong(prev) & (long long)0x8000000000000000ull) ^
+                                     (long long)0x8000000000000000ull ^ (0x200ll << 52));
+        return p;
+    };
+    auto step = [&](double dk, double ek2) {
+        const double t = (dk - x) * p1;
+        double p = fma(-ek2, p0, t);
+        p = nz(p, p1);
+        cnt += (int)((unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31);
+        p0 = p1;
+        p1 = p;
+    };
+    p1 = nz(p1, p0);
+    cnt = (int)((unsigned)__double2hiint(p1) >> 31);
+    int k = b0 + 1;
+    for (; k + 4 <= b1 + 1; k += 4) {
+        double dk[4], ek[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) { dk[u] = d[k + u]; ek[u] = e2[k + u - 1]; }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) step(dk[u], ek[u]);
+        const int e1 = (__double2hiint(p1) >> 20) & 0x7FF, e0 = (__double2hiint(p0) >> 20) & 0x7FF;
+        const int em = max(e0, e1);
+        if (em > 1023 + 300 || em < 1023 - 300) {
+            // both by 2^(1023 - em); one that would leave the normal range goes to a signed 2^-1000
+            const int sft = 1023 - em;
+            auto sc = [&](double p, int ep) {
+                const int en = ep + sft;
+                const int keep = __double2hiint(p) & (int)0x800FFFFFu;
+                return en > 20 ? __hiloint2double(keep | (en << 20), __double2loint(p))
+                               : __hiloint2double((keep & (int)0x80000000u) | (23 << 20), 0);
+            };
+            p1 = sc(p1, e1);
+            p0 = sc(p0, e0);
+            ex -= sft;
+        }
+    }
+    for (; k <= b1; ++k) step(d[k], e2[k - 1]);
+    TriPoly r;
+    const int e1 = (__double2hiint(p1) >> 20) & 0x7FF;
+    r.m = __hiloint2double((__double2hiint(p1) & (int)0x800FFFFFu) | (1023 << 20), __double2loint(p1));
+    r.ex = ex + e1 - 1023;
+    r.cnt = cnt;
+    return r;
+}
+
+// Scaled copies of d and e^2 in FP64 and FP32 and the split flags, 25 n bytes: in
+// shared memory, or in `work` (32 n bytes per matrix) where that is too little;
+// there every CTA of a matrix writes the same values and reads its own.
+__global__ void k_tri_bisect64(const double *dd, const double *ee, double *lamloc, int *blk, int n, double *work)
+{
+    extern __shared__ __align__(16) unsigned char bis64_s[];
+    __shared__ double smax[32];
+    double *d = work ? work + 4 * (long)n * blockIdx.y : (double *)bis64_s, *e2 = d + n;
+    float *sd = (float *)(e2 + n), *se2 = sd + n;
+    unsigned char *ssp = (unsigned char *)(se2 + n);
+    const int b = blockIdx.y, tid = threadIdx.x;
+    const int r = blockIdx.x * blockDim.x + tid;
+    const double *dg = dd + (long)b * n, *eg = ee + (long)b * n;
+    // scale: a power of two that brings the largest element to [1/2, 1)
+    double mx = 0;
+    for (int k = tid; k < n; k += blockDim.x) mx = fmax(mx, fmax(fabs(dg[k]), k < n - 1 ? fabs(eg[k]) : 0.0));
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if ((tid & 31) == 0) smax[tid >> 5] = mx;
+    __syncthreads();
+    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) mx = fmax(mx, smax[q]);
+    int sx = 0;
+    if (mx > 0 && mx < 1e300) frexp(mx, &sx);
+    sx = max(-900, min(900, sx));
+    const double sc = scalbn(1.0, -sx);
+    for (int k = tid; k < n; k += blockDim.x) {
+        const double dk = dg[k] * sc, ek = k < n - 1 ? eg[k] * sc : 0.0;
+        d[k] = dk;
+        e2[k] = ek * ek;
+        sd[k] = (float)dk;
+        const float ef = (float)ek;
+        se2[k] = ef * ef;
+        ssp[k] = k < n - 1 && fabs(dg[k] * dg[k + 1]) * DBL_EPSILON * DBL_EPSILON + DBL_MIN >= eg[k] * eg[k];
+    }
+    __syncthreads();
+    const bool valid = r < n;
+    int b0 = 0, b1 = -1;
+    if (valid) find_block_flags(ssp, n, r, b0, b1);
+    double tnorm = 0, lo = 1e300, hi = -1e300, emax2 = 0;
+    block_bounds(dg, eg, valid, b0, b1, lo, hi, tnorm, emax2);
+    if (!valid) return;
+    lo *= sc;
+    hi *= sc;
+    tnorm *= sc;
+    const double eps = eps_of<double>(), atol = eps * tnorm, pivmin = DBL_MIN;
+    const int j = r - b0;
+    const double glo = lo - 2.0 * atol - pivmin, ghi = hi + 2.0 * atol + pivmin;
+    double lam;
+    if (b0 == b1) {
+        lam = d[b0];
+    } else {
+        double a = glo, z = ghi;
+        if (tnorm > 1e-30) {   // FP32's range holds the block
+            float fa = (float)glo, fz = (float)ghi;
+            const float w = 4.f * eps_of<float>() * (float)tnorm;
+            fa -= w;
+            fz += w;
+            octasect(sd, se2, b0, b1, j, eps_of<float>() * (float)tnorm, tiny_of<float>(), fa, fz);
+            // the FP32 interval widened by its own error, then checked
+            const double m = 4.0 * (double)eps_of<float>() * tnorm;
+            a = fmax(glo, (double)fa - m);
+            z = fmin(ghi, (double)fz + m);
+        }
+        TriPoly pa = tri_poly(d, e2, b0, b1, a), pz = tri_poly(d, e2, b0, b1, z);
+        double h = 64.0 * (double)eps_of<float>() * tnorm;
+        for (int t = 0; t < 16 && pa.cnt > j && a > glo; ++t, h *= 64.0) {
+            z = a;
+            pz = pa;
+            a = fmax(glo, a - h);
+            pa = tri_poly(d, e2, b0, b1, a);
+        }
+        h = 64.0 * (double)eps_of<float>() * tnorm;
+        for (int t = 0; t < 16 && pz.cnt <= j && z < ghi; ++t, h *= 64.0) {
+            a = z;
+            pa = pz;
+            z = fmin(ghi, z + h);
+            pz = tri_poly(d, e2, b0, b1, z);
+        }
+        double wa = 1.0, wz = 1.0;   // Illinois weights of the two values
+        int side = 0;                // which end moved last (+1 a, -1 z), doubled when twice in a row
+        double width2 = 2.0 * (z - a);   // width two steps ago
+        for (int it = 0; it < 256; ++it) {
+            const double width = z - a, mid = a + 0.5 * width;
+            const double tol = fmax(atol, 2.0 * eps * fmax(fabs(a), fabs(z))) + pivmin;
+            if (!(width > tol) || mid <= a || mid >= z) break;
+            double x = mid;
+            const bool one = pz.cnt - pa.cnt == 1;
+            if (one && !(it & 1 && width > 0.5 * width2)) {
+                // zero of the line through the weighted values (they differ in sign)
+                const int de = max(-1000, min(1000, pz.ex - pa.ex));
+                const double fa = fabs(pa.m) * wa, fz = scalbn(fabs(pz.m) * wz, de);
+                x = a + width * (fa / (fa + fz));
+                // at least half a tolerance inside, so that the far end comes in too
+                x = fmin(fmax(x, a + 0.5 * tol), z - 0.5 * tol);
+                if (!(x > a && x < z)) x = mid;
+            }
+            if (it & 1) width2 = width;
+            const TriPoly p = tri_poly(d, e2, b0, b1, x);
+            if (p.cnt <= j) {
+                a = x;
+                pa = p;
+                wa = 1.0;
+                if (side > 0) wz *= 0.5;
+                side = 1;
+            } else {
+                z = x;
+                pz = p;
+                wz = 1.0;
+                if (side < 0) wa *= 0.5;
+                side = -1;
+            }
+        }
+        lam = a + 0.5 * (z - a);
+    }
+    lamloc[(long)b * n + r] = scalbn(lam, sx);
     blk[((long)b * n + r) * 2 + 0] = b0;
     blk[((long)b * n + r) * 2 + 1] = b1;
 }
@@ -893,10 +1076,22 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     int *blk = w.perm, *rank = w.perm + 2 * (long)n * B;
     {
         dim3 g(cdiv(n, 128), B);
-        const size_t bsm = sizeof(T) == 4 ? 2 * sizeof(float) * n + n : 0;
-        if (bsm > 48 * 1024)
-            smem_attr_at_least((const void *)k_tri_bisect<T>, (int)bsm);
-        NRLTB_LAUNCH(k_tri_bisect<T>, g, 128, bsm, s, w.d, w.e, lamloc, blk, n);
+        if (sizeof(T) == 4) {
+            const size_t bsm = 2 * sizeof(float) * n + n;
+            if (bsm > 48 * 1024) smem_attr_at_least((const void *)k_tri_bisect32, (int)bsm);
+            NRLTB_LAUNCH(k_tri_bisect32, g, 128, bsm, s, w.d, w.e, lamloc, blk, n);
+        } else {
+            // a warp per CTA while that leaves CTAs to every SM (the FP64 pipe is the SM's)
+            const int nt = (long)n * B < 64L * 152 * 8 ? 32 : 64;
+            size_t bsm = 25 * (size_t)n + 16;
+            double *work = nullptr;
+            if (bsm > 200 * 1024) {
+                work = w.ylu;   // inverse iteration's scratch, free until then
+                bsm = 0;
+            }
+            if (bsm > 48 * 1024) smem_attr_at_least((const void *)k_tri_bisect64, (int)bsm);
+            NRLTB_LAUNCH(k_tri_bisect64, dim3(cdiv(n, nt), B), nt, bsm, s, w.d, w.e, lamloc, blk, n, work);
+        }
         const size_t rsm = rank_keys_bytes(n);
         if (rsm > 48 * 1024) smem_attr_at_least((const void *)k_tri_rank, (int)rsm);
         NRLTB_LAUNCH(k_tri_rank, g, 128, rsm, s, lamloc, rank, w.lam, n, rsm > 0 ? 1 : 0);
