@@ -78,16 +78,12 @@ __global__ void k_convert_h(const double2 *__restrict__ src, C2 *__restrict__ ds
 // ---------------------------------------------------------------------------
 // v s, each part rounded on its own (never contracted into a later add)
 __device__ __forceinline__ float2 scale_rn(float2 v, float s) { return make_float2(__fmul_rn(v.x, s), __fmul_rn(v.y, s)); }
-__device__ __forceinline__ double2 scale_rn(double2 v, double s)
-{
-    return make_double2(__dmul_rn(v.x, s), __dmul_rn(v.y, s));
-}
 
-// Diagonal block: Cholesky L_jj L_jj^H = S_jj and its inverse, in shared memory.
-template <typename T>
-__global__ void __launch_bounds__(256) k_potrf_diag(EigWork<T> w, int j0, int jb)
+// Diagonal block: Cholesky L_jj L_jj^H = S_jj and its inverse, in shared memory (FP32).
+__global__ void __launch_bounds__(256) k_potrf_diag(EigWork<float> w, int j0, int jb)
 {
-    typedef typename cplx<T>::t C2;
+    typedef float T;
+    typedef float2 C2;
     __shared__ C2 a[EIG_NB][EIG_NB + 1];   // a[c][r], updated in place
     __shared__ C2 x[EIG_NB][EIG_NB + 1];   // inverse, x[c][r]
     __shared__ int bad;
@@ -669,10 +665,13 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
         TB dcur = Dk(b0) - lam, ducur = (len > 1) ? Ek(b0) : TB(0);
         TB vc = rhs(0);
         for (int kb = 0; kb < len - 1; kb += INV_BLK) {
-            TB vn[INV_BLK];
+            TB vn[INV_BLK], rgv[INV_BLK];
 #pragma unroll
             for (int u = 0; u < INV_BLK; ++u)
-                if (kb + u < len - 1) vn[u] = rhs(kb + u + 1);
+                if (kb + u < len - 1) {
+                    vn[u] = rhs(kb + u + 1);
+                    if (sizeof(TB) == 8 && it > 0) rgv[u] = RG[kb + u];
+                }
 #pragma unroll
             for (int u = 0; u < INV_BLK; ++u) {
                 const int k = kb + u;
@@ -680,15 +679,32 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
                 const TB dlk = Ek(b0 + k);
                 TB dnext = Dk(b0 + k + 1) - lam;
                 TB dunext = (k < len - 2) ? Ek(b0 + k + 1) : TB(0);
+                // FP64 takes a dozen operations of its narrow pipe for a quotient: one
+                // per step, 1 / pivot, which also gives the multiplier and which the
+                // later iterations read back
                 if (fabs(dcur) >= fabs(dlk)) {
-                    const TB f = (dcur != TB(0)) ? tri_div(dlk, dcur) : TB(0);
-                    if (it == 0) { RG[k] = tri_div(TB(1), pivot(dcur)); DU[k] = ducur; DU2[k] = TB(0); }
+                    TB f;
+                    if (sizeof(TB) == 8) {
+                        const TB rp = it == 0 ? tri_div(TB(1), pivot(dcur)) : rgv[u];
+                        f = (dcur != TB(0)) ? dlk * rp : TB(0);
+                        if (it == 0) { RG[k] = rp; DU[k] = ducur; DU2[k] = TB(0); }
+                    } else {
+                        f = (dcur != TB(0)) ? tri_div(dlk, dcur) : TB(0);
+                        if (it == 0) { RG[k] = tri_div(TB(1), pivot(dcur)); DU[k] = ducur; DU2[k] = TB(0); }
+                    }
                     dnext -= f * ducur;
                     v[k] = vc;
                     vc = vn[u] - f * vc;
                 } else {
-                    const TB f = tri_div(dcur, dlk);
-                    if (it == 0) { RG[k] = tri_div(TB(1), pivot(dlk)); DU[k] = dnext; DU2[k] = dunext; }
+                    TB f;
+                    if (sizeof(TB) == 8) {
+                        const TB rp = it == 0 ? tri_div(TB(1), pivot(dlk)) : rgv[u];
+                        f = dcur * rp;
+                        if (it == 0) { RG[k] = rp; DU[k] = dnext; DU2[k] = dunext; }
+                    } else {
+                        f = tri_div(dcur, dlk);
+                        if (it == 0) { RG[k] = tri_div(TB(1), pivot(dlk)); DU[k] = dnext; DU2[k] = dunext; }
+                    }
                     dnext = ducur - f * dnext;
                     dunext = -f * dunext;
                     v[k] = vn[u];
@@ -832,28 +848,26 @@ __global__ void k_real_to_cplx(const double *y, C2 *z, long count)
 // compact-WY T factor of a block of jb <= EIG_WY reflectors (G = Vb^H Vb and T
 // column-major nbw x nbw per matrix): column by column,
 // T[0:c, c] = -tau_c T[0:c, 0:c] G[0:c, c], T[c, c] = tau_c (LAPACK's larft,
-// forward columnwise).  One CTA of EIG_WY threads per matrix, thread = row;
-// T is built in shared memory when it fits (FP32: 128 x 129 complex = 132 KB,
-// dynamic), else in global memory.  Row r of T depends only on row r and on
-// G, so the threads need no barrier between columns: the columns of G (and
-// the taus) come in groups of LARFT_GC through shared memory, with a barrier
-// per group.  The lanes of a warp walk k together from the warp's first row,
-// so that their reads of T are consecutive and G[k, c] is one broadcast; row r
-// adds its terms k >= r in order of k (the one-row-at-a-time sums).
+// forward columnwise).  FP32: one CTA of EIG_WY threads per matrix, thread = row;
+// T is built in shared memory (128 x 129 complex = 132 KB, dynamic).  Row r of T
+// depends only on row r and on G, so the threads need no barrier between
+// columns: the columns of G (and the taus) come in groups of LARFT_GC through
+// shared memory, with a barrier per group.  The lanes of a warp walk k together
+// from the warp's first row, so that their reads of T are consecutive and G[k, c]
+// is one broadcast; row r adds its terms k >= r in order of k (the
+// one-row-at-a-time sums).
 constexpr int LARFT_GC = 8;
-template <typename T, bool SMEM>
-__global__ void __launch_bounds__(EIG_WY) k_larft_wy(const typename cplx<T>::t *G, typename cplx<T>::t *Tm,
-                                                     const typename cplx<T>::t *tau, int n, int j0, int jb, int nbw)
+__global__ void __launch_bounds__(EIG_WY) k_larft_wy(const float2 *G, float2 *Tm, const float2 *tau, int n, int j0,
+                                                     int jb, int nbw)
 {
-    typedef typename cplx<T>::t C2;
-    __shared__ C2 g[LARFT_GC][EIG_WY];
-    __shared__ C2 tg[LARFT_GC];
+    __shared__ float2 g[LARFT_GC][EIG_WY];
+    __shared__ float2 tg[LARFT_GC];
     extern __shared__ __align__(16) unsigned char larft_smem[];
     const int b = blockIdx.x, r = threadIdx.x, kw = r & ~31;
-    const C2 *Gb = G + (long)b * nbw * nbw;
-    C2 *Tb = Tm + (long)b * nbw * nbw;
-    const int lt = SMEM ? EIG_WY + 1 : nbw;   // column stride of the working T
-    C2 *Tw = SMEM ? (C2 *)larft_smem : Tb;
+    const float2 *Gb = G + (long)b * nbw * nbw;
+    float2 *Tb = Tm + (long)b * nbw * nbw;
+    constexpr int lt = EIG_WY + 1;   // column stride of the working T
+    float2 *Tw = (float2 *)larft_smem;
     for (int c0 = 0; c0 < jb; c0 += LARFT_GC) {
         const int cn = min(LARFT_GC, jb - c0);
         __syncthreads();   // every thread is done with the previous group's columns
@@ -863,12 +877,12 @@ __global__ void __launch_bounds__(EIG_WY) k_larft_wy(const typename cplx<T>::t *
         __syncthreads();
         for (int q = 0; q < cn; ++q) {
             const int c = c0 + q;
-            const C2 tc = tg[q];
+            const float2 tc = tg[q];
             if (kw < c) {   // warp-uniform
-                C2 acc = cmk<T>(0, 0);
+                float2 acc = make_float2(0.f, 0.f);
                 int k = kw;
                 for (; k + 8 <= c; k += 8) {
-                    C2 tv[8], gv[8];
+                    float2 tv[8], gv[8];
 #pragma unroll
                     for (int u = 0; u < 8; ++u) {
                         tv[u] = Tw[r + (k + u) * lt];
@@ -880,15 +894,121 @@ __global__ void __launch_bounds__(EIG_WY) k_larft_wy(const typename cplx<T>::t *
                 }
                 for (; k < c; ++k)
                     if (k >= r) cfma(acc, Tw[r + k * lt], g[q][k]);
-                if (r < c) Tw[r + (long)c * lt] = cscale(cmul(tc, acc), T(-1));
+                if (r < c) Tw[r + (long)c * lt] = cscale(cmul(tc, acc), -1.f);
             }
             if (r == c) Tw[c + (long)c * lt] = tc;
         }
     }
     __syncthreads();
-    if (SMEM)
-        for (int c = 0; c < jb; ++c)
-            if (r <= c) Tb[r + (long)c * nbw] = Tw[r + (long)c * lt];
+    for (int c = 0; c < jb; ++c)
+        if (r <= c) Tb[r + (long)c * nbw] = Tw[r + (long)c * lt];
+}
+
+// The same T factor for FP64, whose T does not fit the shared memory of one SM and
+// whose dots are bound by the FP64 pipe: row r of T depends on row r and G alone, so
+// a matrix's rows are spread over CTAs of 16, a warp holding four rows with eight
+// lanes over k each (fewer lanes a row leave a longer chain, more a longer
+// reduction); the columns of G come through shared memory eight at a time.
+// One CTA per matrix with T in global memory took 1.38 ms a block of 128 at 4 k, this
+// 0.28; at 64 k 0.95 against 0.54.
+constexpr int LARFT_RC = 8;
+__global__ void __launch_bounds__(128) k_larft_rows(const double2 *G, double2 *Tm, const double2 *tau, int n, int j0,
+                                                    int jb, int nbw)
+{
+    __shared__ double2 g[LARFT_RC][EIG_WY];
+    __shared__ double2 trow[16][EIG_WY];
+    const int b = blockIdx.y, lane = threadIdx.x & 31, kp = lane & 7, rl = threadIdx.x >> 3;
+    const int cbeg = 16 * blockIdx.x, r = cbeg + rl;   // the CTA's first row: earlier columns are zero
+    const int rw = cbeg + 4 * (threadIdx.x >> 5);      // the warp's first row
+    const double2 *Gb = G + (long)b * nbw * nbw;
+    double2 *Tb = Tm + (long)b * nbw * nbw;
+    const double2 *tb = tau + (long)b * n + j0;
+    double2 *t = trow[rl];
+    for (int c0 = cbeg / LARFT_RC * LARFT_RC; c0 < jb; c0 += LARFT_RC) {
+        const int cn = min(LARFT_RC, jb - c0);
+        __syncthreads();
+#pragma unroll 8
+        for (int q = 0; q < cn; ++q) {
+            const int k = threadIdx.x;
+            if (k < c0 + q && k >= cbeg) g[q][k] = Gb[k + (long)(c0 + q) * nbw];
+        }
+        __syncthreads();
+        for (int q = 0; q < cn; ++q) {
+            const int c = c0 + q;
+            if (c < rw) continue;   // warp-uniform
+            double2 acc = make_double2(0, 0);
+            for (int k = rw + kp; k < c; k += 8)
+                if (k >= r) cfma(acc, t[k], g[q][k]);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) {
+                acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+                acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+            }
+            if (kp == 0 && r <= c && r < jb) {
+                const double2 tc = tb[c], m = cmul(tc, acc);
+                const double2 v = c > r ? make_double2(-m.x, -m.y) : tc;
+                t[c] = v;
+                Tb[r + (long)c * nbw] = v;
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// The same for FP64, where operations of the FP64 pipe are the cost (a warp's takes 64
+// cycles of its quarter of the SM).  Factor and inverse X advance together: after
+// column k of L and row k of X, row r > k of the block takes
+//   a(r, c) -= l_rk conj(l_ck)  for columns c > k,
+//   y(r, c) += l_rk x_kc        for c <= k,  then x_r = -y_r / l_rr,
+// one FMA for all 32 lanes (lane = column, c > k of the factor, c <= k of the
+// inverse), rows dealt over the warps.  The pivot's root and reciprocal are formed by
+// one warp (tc_root).
+// 32 x 32: 187 us by the FP32 kernel's scheme in FP64 (every warp forming the root
+// and reciprocal, one warp the inverse), 53 here.
+__global__ void __launch_bounds__(256) k_potrf_diag64(EigWork<double> w, int j0, int jb)
+{
+    __shared__ double2 m[EIG_NB][EIG_NB + 1];    // m[r][c]: a (c > k) | y (c <= k)
+    __shared__ double2 lo[EIG_NB][EIG_NB + 1];   // L, lo[c][r]
+    __shared__ double2 xo[EIG_NB][EIG_NB + 1];   // X, xo[r][c]
+    __shared__ int bad;
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double2 *L = w.L + b * w.mstride + j0 + (long)j0 * w.ld;
+    double2 *Wi = w.Wi + b * w.mstride + j0 + (long)j0 * w.ld;
+    const double2 z = make_double2(0, 0);
+    for (int c = warp; c < EIG_NB; c += 8) m[lane][c] = lane < jb && c < jb ? L[lane + (long)c * w.ld] : z;
+    if (tid == 0) bad = 0;
+    __syncthreads();
+    for (int k = 0; k < jb; ++k) {
+        if (warp == (k & 7)) {
+            double piv = m[k][k].x;
+            const bool badk = !(piv > 0.0);
+            if (badk) piv = 1.0;
+            double dk, inv;
+            tc_root(piv, dk, inv);
+            const double2 y = m[k][lane], a = m[lane][k];   // row k, column k
+            xo[k][lane] = lane < k ? cscale(y, -inv) : lane == k ? make_double2(inv, 0.0) : z;
+            lo[k][lane] = lane > k ? cscale(a, inv) : lane == k ? make_double2(dk, 0.0) : z;
+            if (badk && lane == 0) bad = 1;
+        }
+        __syncthreads();
+        double2 o = xo[k][lane];
+        if (lane > k) {
+            o = lo[k][lane];
+            o.x = -o.x;   // -conj
+        }
+        for (int r = k + 1 + ((warp - (k + 1)) & 7); r < jb; r += 8) {
+            double2 t = lane == k ? z : m[r][lane];
+            cfma(t, lo[k][r], o);
+            if (lane <= r) m[r][lane] = t;
+        }
+        __syncthreads();
+    }
+    if (lane < jb)
+        for (int c = warp; c < jb; c += 8) {
+            L[lane + (long)c * w.ld] = lo[c][lane];
+            Wi[lane + (long)c * w.ld] = xo[lane][c];
+        }
+    if (tid == 0 && bad) w.status[b] = 1;
 }
 
 // Join the inverted 32 x 32 diagonal blocks of L pairwise: for the 64-block at
@@ -979,7 +1099,8 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     // 1. Cholesky S = L L^H
     for (int j0 = 0; j0 < n; j0 += EIG_NB) {
         const int jb = std::min(EIG_NB, n - j0), rem = n - j0 - jb;
-        NRLTB_LAUNCH(k_potrf_diag<T>, B, 256, 0, s, w, j0, jb);
+        if constexpr (sizeof(T) == 4) NRLTB_LAUNCH(k_potrf_diag, B, 256, 0, s, w, j0, jb);
+        else NRLTB_LAUNCH(k_potrf_diag64, B, 256, 0, s, w, j0, jb);
         if (rem > 0) {
             C2 *P = w.L + (j0 + jb) + (long)j0 * ld;
             zgemm<T>(s, rem, jb, jb, B, one, P, ld, ms, 0, w.Wi + j0 + (long)j0 * ld, ld, ms, 1, zero, P, ld, ms,
@@ -1056,10 +1177,12 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
         zgemm<T>(st, jb, jb, mb, B, one, Vb, ld, ms, 1, Vb, ld, ms, 0, zero, G, nbw, sG, 0, 0, 0, w.zs);
         if (sizeof(T) == 4) {
             const int sm = (int)(sizeof(C2) * EIG_WY * (EIG_WY + 1));
-            smem_attr_at_least((const void *)k_larft_wy<T, true>, sm);
-            NRLTB_LAUNCH((k_larft_wy<T, true>), B, EIG_WY, sm, st, G, Tf_of(j0), w.tau, n, j0, jb, nbw);
+            smem_attr_at_least((const void *)k_larft_wy, sm);
+            NRLTB_LAUNCH(k_larft_wy, B, EIG_WY, sm, st, (const float2 *)G, (float2 *)Tf_of(j0), (const float2 *)w.tau, n,
+                         j0, jb, nbw);
         } else {
-            NRLTB_LAUNCH((k_larft_wy<T, false>), B, EIG_WY, 0, st, G, Tf_of(j0), w.tau, n, j0, jb, nbw);
+            NRLTB_LAUNCH(k_larft_rows, dim3(cdiv(jb, 16), B), 128, 0, st, (const double2 *)G, (double2 *)Tf_of(j0),
+                         (const double2 *)w.tau, n, j0, jb, nbw);
         }
     };
     const int j0last = nref >= 1 ? ((nref - 1) / nbw) * nbw : -1;
