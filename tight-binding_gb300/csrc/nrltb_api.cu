@@ -1438,7 +1438,7 @@ int nrltb_fermi(nrltb_ctx *c, int nv, int nk, const double *eig, const double *w
     CK(cudaMemcpyAsync(c->d_fjob.p, &job, sizeof job, cudaMemcpyHostToDevice, s));
     {
         CallScope scope(c);
-        launch_fermi_sums(s, c->d_fjob.as<FermiJob>(), fermi_part(c));
+        launch_fermi_sums(s, c->d_fjob.as<FermiJob>(), nullptr);   // E_F alone
     }
     CKL();
     FermiOut o;

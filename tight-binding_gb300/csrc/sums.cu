@@ -1,7 +1,7 @@
 // sums.cu -- Fermi level, band energy, pressure (fermi.f, bande.f sums) and the
 // Hellmann-Feynman eigenvalue derivatives (perturb.f).
 //
-// launch_fermi_sums: k_fermi_level finds E_F in one CTA, k_band_sums and
+// launch_fermi_sums: k_fermi_level finds E_F in one cluster, k_band_sums and
 // k_band_finish form the sums over the whole GPU.  The MPI_ALLREDUCE of every
 // Newton step (fermi.f:365-376) and the final MPI_REDUCEs (bande.f:1255-1331)
 // become block and grid reductions; the iteration itself is the reference's: start at the middle of
@@ -18,6 +18,7 @@
 // what an exact summation of the rounded terms would give to within a few
 // units in the last place of the result, however much the terms cancel, and
 // the same from run to run.
+#include <cooperative_groups.h>
 #include "sums.cuh"
 
 namespace nrltb {
@@ -40,57 +41,19 @@ struct DD {
     }
 };
 
-// block-wide compensated sum; every thread gets hi + lo of the total.  `sh`
-// needs 2 * blockDim.x / 32 entries.
-__device__ double block_sum_dd(DD v, double *sh)
-{
-    for (int o = 16; o > 0; o >>= 1) {
-        const double h = __shfl_xor_sync(0xffffffffu, v.hi, o), l = __shfl_xor_sync(0xffffffffu, v.lo, o);
-        v.merge(h, l);
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    __syncthreads();
-    if (lane == 0) { sh[wid] = v.hi; sh[32 + wid] = v.lo; }
-    __syncthreads();
-    if (wid == 0) {
-        DD t;
-        if (lane < nw) { t.hi = sh[lane]; t.lo = sh[32 + lane]; }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double h = __shfl_xor_sync(0xffffffffu, t.hi, o), l = __shfl_xor_sync(0xffffffffu, t.lo, o);
-            t.merge(h, l);
-        }
-        if (lane == 0) sh[0] = t.hi + t.lo;
-    }
-    __syncthreads();
-    const double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
 __device__ inline double block_sum_d(double v, double *sh) { return block_sum<double>(v, sh); }
-__device__ inline double block_max_d(double v, double *sh)
-{
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    __syncthreads();
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    double t = (threadIdx.x < nw) ? sh[threadIdx.x] : -1e308;
-    if (wid == 0) for (int o = 16; o > 0; o >>= 1) t = fmax(t, __shfl_xor_sync(0xffffffffu, t, o));
-    if (threadIdx.x == 0) sh[0] = t;
-    __syncthreads();
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
-// number of entries of the ascending row e[0..m) below x
+// number of entries of the ascending row e[0..m) below x, by the whole warp (32
+// probes a step)
 __device__ __forceinline__ int count_below(const double *e, int m, double x)
 {
+    const int lane = threadIdx.x & 31;
     int lo = 0, hi = m;
     while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (e[mid] < x) lo = mid + 1; else hi = mid;
+        const int st = (hi - lo + 31) / 32, p = lo + lane * st;
+        const int c = __popc(__ballot_sync(0xffffffffu, p < hi && e[p] < x));
+        if (c == 0) return lo;
+        hi = min(hi, lo + c * st);
+        lo += (c - 1) * st + 1;
     }
     return lo;
 }
@@ -98,52 +61,96 @@ __device__ __forceinline__ int count_below(const double *e, int m, double x)
 // E_F (fermi.f:162-425).  When every row is ascending (the eigensolver's
 // output always is) the band edges are row ends and each Newton step's
 // occupation needs only the states inside the +-20 kT window: a row's fully
-// occupied states below it are counted by a binary search (their w_k add up
-// to count x w_k), a warp per row takes the window.  Rows that are not
-// ascending (caller eigenvalues) fall back to a scan of every state.
-__global__ void __launch_bounds__(1024) k_fermi_level(FermiJob *jobs)
+// occupied states below it are counted by a search (their w_k add up to
+// count x w_k), a warp per row takes the window.  Rows that are not ascending
+// (caller eigenvalues), and rows too short to fill a warp, take a scan of every
+// state.
+// One cluster of FERMI_CL CTAs: a Newton step is bound by the FP64 pipe (an
+// exponential and a quotient per window state, two FP64 operations a cycle per SM)
+// and then by its reduction, so the states are spread over FERMI_CL SMs and the
+// CTAs are small (every warp of the reduction costs FP64 operations too).  The
+// CTAs' compensated partials are merged in rank order by every CTA, which all take
+// the same step; one cluster barrier per step, the slots alternate.
+// One CTA of 1024 threads took 0.71 ms for 27 rows of 1152 states and 5.3 ms for 1728
+// rows of 9; this 0.10 and 0.33.
+constexpr int FERMI_CL = 8, FERMI_THREADS = 128, FERMI_ROW_MIN = 64;
+constexpr int FERMI_WARPS = FERMI_CL * FERMI_THREADS / 32;
+
+struct FermiSlot { double v[6]; };
+
+// the CTA's two sums into its slot; the cluster's totals to every thread
+__device__ __forceinline__ void fermi_totals(cooperative_groups::cluster_group &cl, DD a, DD c, FermiSlot *slot,
+                                             double (*sh)[FERMI_THREADS / 32], double &ta, double &tc)
 {
-    __shared__ double sh[64];
-    __shared__ int s_sorted;
-    FermiJob J = jobs[blockIdx.x];
-    const int nv = J.nv, nk = J.nk, tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    const int nwarps = nt >> 5;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double ah = __shfl_xor_sync(0xffffffffu, a.hi, o), al = __shfl_xor_sync(0xffffffffu, a.lo, o);
+        const double ch = __shfl_xor_sync(0xffffffffu, c.hi, o), c2 = __shfl_xor_sync(0xffffffffu, c.lo, o);
+        a.merge(ah, al);
+        c.merge(ch, c2);
+    }
+    if (lane == 0) {
+        sh[0][wid] = a.hi; sh[1][wid] = a.lo;
+        sh[2][wid] = c.hi; sh[3][wid] = c.lo;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        DD x, y;
+        for (int q = 0; q < FERMI_THREADS / 32; ++q) {
+            x.merge(sh[0][q], sh[1][q]);
+            y.merge(sh[2][q], sh[3][q]);
+        }
+        slot->v[0] = x.hi; slot->v[1] = x.lo;
+        slot->v[2] = y.hi; slot->v[3] = y.lo;
+    }
+    cl.sync();
+    DD x, y;
+    for (int q = 0; q < FERMI_CL; ++q) {
+        const FermiSlot *o = cl.map_shared_rank(slot, q);
+        x.merge(o->v[0], o->v[1]);
+        y.merge(o->v[2], o->v[3]);
+    }
+    ta = x.hi + x.lo;
+    tc = y.hi + y.lo;
+}
+
+__global__ void __cluster_dims__(FERMI_CL, 1, 1) __launch_bounds__(FERMI_THREADS) k_fermi_level(FermiJob *jobs)
+{
+    namespace cg = cooperative_groups;
+    __shared__ double sh[6][FERMI_THREADS / 32];
+    __shared__ FermiSlot slots[2], edge;
+    cg::cluster_group cl = cg::this_cluster();
+    FermiJob J = jobs[0];
+    const int nv = J.nv, nk = J.nk, tid = threadIdx.x, lane = tid & 31;
+    const int gt = (int)cl.block_rank() * FERMI_THREADS + tid, nt = FERMI_CL * FERMI_THREADS, gw = gt >> 5;
     const long tot = (long)nv * nk;
     const double el = J.el, nearz = 1e-5, tkb = J.tkb, zfill = J.zfill, tol = J.tol;
     const double beta = (tkb < nearz) ? 1.0 / nearz : 1.0 / tkb;
     const int nfill = (int)(zfill / el + nearz);
     const bool linst = fabs(zfill / el - (double)nfill) < tol;
-    if (tid == 0) s_sorted = 1;
-    __syncthreads();
-    {
-        int uns = 0;
-        for (int k = warp; k < nk; k += nwarps) {   // a warp per row
-            const double *e = J.eig + (long)k * J.ldk;
-            for (int i = lane; i + 1 < nv; i += 32)
-                if (e[i + 1] < e[i]) uns = 1;
-        }
-        if (__syncthreads_or(uns) && tid == 0) s_sorted = 0;
-        __syncthreads();
-    }
-    const bool sorted = s_sorted != 0;
     // bounds (fermi.f:197-261) from bands nfill and nfill+1; where those lie
     // outside the nv computed bands (nfill >= nv happens with one electron per
     // band) the reference reads past them: here the band indices are clamped
     // and the insulator shortcut is not taken, which moves only the start
     const int ilo = max(min(nfill, nv) - 1, 0), ihi = min(nfill, nv - 1);
     const bool inrange = nfill >= 1 && nfill < nv;
-    double stl = -1e308, sth = 1e308, mul = 1e308, muh = -1e308;
-    if (sorted) {
-        for (int k = tid; k < nk; k += nt) {
+    double stl = -1e308, sth = 1e308, mul = 1e308, muh = -1e308, uns = 0.0;
+    const bool rows = nv >= FERMI_ROW_MIN;   // a warp per row, else a thread per state
+    if (rows) {
+        for (int k = gw; k < nk; k += FERMI_WARPS) {
             const double *e = J.eig + (long)k * J.ldk;
-            stl = fmax(stl, e[ilo]);
-            sth = fmin(sth, e[ihi]);
-            muh = fmax(muh, e[nv - 1]);
-            mul = fmin(mul, e[0]);
+            for (int i = lane; i < nv; i += 32) {
+                const double v = e[i];
+                if (i + 1 < nv && e[i + 1] < v) uns = 1.0;
+                if (i == ilo) stl = fmax(stl, v);
+                if (i == ihi) sth = fmin(sth, v);
+                muh = fmax(muh, v);
+                mul = fmin(mul, v);
+            }
         }
     } else {
-        for (long q = tid; q < tot; q += nt) {
-            const int k = (int)(q / nv), i = (int)(q % nv);
+        for (long q = gt; q < tot; q += nt) {
+            const int k = (int)(q / nv), i = (int)(q - (long)k * nv);
             const double e = J.eig[(long)k * J.ldk + i];
             if (i == ilo) stl = fmax(stl, e);
             if (i == ihi) sth = fmin(sth, e);
@@ -151,46 +158,68 @@ __global__ void __launch_bounds__(1024) k_fermi_level(FermiJob *jobs)
             mul = fmin(mul, e);
         }
     }
-    double stlow = block_max_d(stl, sh), sthigh = -block_max_d(-sth, sh);
-    double muhigh = block_max_d(muh, sh), mulow = -block_max_d(-mul, sh);
-    double mu;
+    {   // over the cluster (maxima and minima: exact in any order)
+        double v[5] = {stl, -sth, muh, -mul, uns};
+#pragma unroll
+        for (int x = 0; x < 5; ++x) {
+            for (int o = 16; o > 0; o >>= 1) v[x] = fmax(v[x], __shfl_xor_sync(0xffffffffu, v[x], o));
+            if (lane == 0) sh[x][tid >> 5] = v[x];
+        }
+        __syncthreads();
+        if (tid < 5) {
+            double m = sh[tid][0];
+            for (int q = 1; q < FERMI_THREADS / 32; ++q) m = fmax(m, sh[tid][q]);
+            edge.v[tid] = m;
+        }
+        cl.sync();
+#pragma unroll
+        for (int x = 0; x < 5; ++x) {
+            double m = -1e308;
+            for (int q = 0; q < FERMI_CL; ++q) m = fmax(m, cl.map_shared_rank(&edge, q)->v[x]);
+            v[x] = m;
+        }
+        stl = v[0];
+        sth = -v[1];
+        muh = v[2];
+        mul = -v[3];
+        uns = v[4];
+    }
+    const bool sorted = rows && uns == 0.0;
+    const double stlow = stl, sthigh = sth;
+    double muhigh = muh, mulow = mul;
+    double mu = 0.5 * (stlow + sthigh);
     int it = 0;
-    if (linst && inrange && (sthigh - stlow > 20.0 * tkb)) {
-        mu = 0.5 * (stlow + sthigh);
-    } else {
-        mu = 0.5 * (stlow + sthigh);
-        for (it = 1; it <= 10000; ++it) {
+    if (!(linst && inrange && (sthigh - stlow > 20.0 * tkb))) {
+        for (it = 1; it <= 10000; ++it) {   // (the same decisions in every CTA)
             const double mum20 = mu - tkb * 20.0, mup20 = mu + tkb * 20.0, btmu = -beta * mu;
             DD ns, dns;
+            auto window = [&](double e, double wk) {
+                const double ex = exp(beta * e + btmu);
+                const double f = 1.0 / (1.0 + ex);
+                ns.add(wk * f);
+                dns.add(wk * (ex * f * f));
+            };
             if (sorted) {
-                for (int k = warp; k < nk; k += nwarps) {
+                for (int k = gw; k < nk; k += FERMI_WARPS) {
                     const double *e = J.eig + (long)k * J.ldk;
                     const double wk = J.w[k];
                     const int lo = count_below(e, nv, mum20), hi = count_below(e, nv, mup20);
                     if (lane == 0) ns.add(wk * (double)lo);
-                    for (int i = lo + lane; i < hi; i += 32) {
-                        const double ex = exp(beta * e[i] + btmu);
-                        const double f = 1.0 / (1.0 + ex);
-                        ns.add(wk * f);
-                        dns.add(wk * (ex * f * f));
-                    }
+                    for (int i = lo + lane; i < hi; i += 32) window(e[i], wk);
                 }
             } else {
-                for (long q = tid; q < tot; q += nt) {
-                    const int k = (int)(q / nv), i = (int)(q % nv);
+                for (long q = gt; q < tot; q += nt) {
+                    const int k = (int)(q / nv), i = (int)(q - (long)k * nv);
                     const double e = J.eig[(long)k * J.ldk + i];
                     const double wk = J.w[k];
                     if (e < mum20) ns.add(wk);
-                    else if (e < mup20) {
-                        const double ex = exp(beta * e + btmu);
-                        const double f = 1.0 / (1.0 + ex);
-                        ns.add(wk * f);
-                        dns.add(wk * (ex * f * f));
-                    }
+                    else if (e < mup20) window(e, wk);
                 }
             }
-            double nsum = el * block_sum_dd(ns, sh);
-            double dnsum = beta * el * block_sum_dd(dns, sh);
+            double nsum, dnsum;
+            fermi_totals(cl, ns, dns, &slots[it & 1], sh, nsum, dnsum);
+            nsum *= el;
+            dnsum *= beta * el;
             if (fabs(nsum - zfill) < tol) break;
             if (nsum < zfill) mulow = mu; else muhigh = mu;
             double mu1;
@@ -204,18 +233,28 @@ __global__ void __launch_bounds__(1024) k_fermi_level(FermiJob *jobs)
             else break;
         }
     }
-    if (tid == 0) {
+    if (gt == 0) {
         J.out->efermi = mu;
         J.out->iterations = it;
     }
+    cl.sync();   // no CTA leaves while others may read its slots
 }
 
 // The sums after E_F (bande.f:1162-1330), spread over the GPU: each CTA
 // forms compensated partial sums over a stride of the states and stores
 // them (hi, lo) in part[blockIdx.x][2 x FERMI_NSUM]; k_band_finish merges the
 // CTAs' partials in CTA order.
-constexpr int FERMI_NSUM = 11;
-__global__ void __launch_bounds__(256) k_band_sums(FermiJob *jobs, double *part)
+// A sum that the mode does not ask for is not reduced (each reduction costs every
+// warp some eighty FP64 operations), and the CTAs are small for the same reason.
+constexpr int FERMI_NSUM = 11, FERMI_SUM_THREADS = 64;
+__device__ __forceinline__ bool fermi_sum_used(const FermiJob &J, int s)
+{
+    if (s == 0) return true;                                  // E
+    if (s <= 5) return J.lpress;                              // pressure
+    if (s <= 8) return J.lentro && (s == 6 || J.lpress);      // entropy
+    return J.nks > 0;                                         // spin populations
+}
+__global__ void __launch_bounds__(FERMI_SUM_THREADS) k_band_sums(FermiJob *jobs, double *part)
 {
     __shared__ double sh[64];
     FermiJob J = jobs[0];
@@ -267,6 +306,7 @@ __global__ void __launch_bounds__(256) k_band_sums(FermiJob *jobs, double *part)
     // CTA-wide merge of each pair (fixed tree order), then one store per sum
 #pragma unroll
     for (int s = 0; s < FERMI_NSUM; ++s) {
+        if (!fermi_sum_used(J, s)) continue;   // uniform
         DD v = acc[s];
         for (int o = 16; o > 0; o >>= 1) {
             const double h = __shfl_xor_sync(0xffffffffu, v.hi, o), l = __shfl_xor_sync(0xffffffffu, v.lo, o);
@@ -285,18 +325,24 @@ __global__ void __launch_bounds__(256) k_band_sums(FermiJob *jobs, double *part)
     }
 }
 
-__global__ void k_band_finish(FermiJob *jobs, const double *part, int nblk)
+// merge of the CTAs' partials: a warp per sum, its lanes over the CTAs, then a tree
+__global__ void __launch_bounds__(32 * FERMI_NSUM) k_band_finish(FermiJob *jobs, const double *part, int nblk)
 {
     FermiJob J = jobs[0];
-    const int s = threadIdx.x;
+    const int s = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ double tot[FERMI_NSUM];
-    if (s < FERMI_NSUM) {
-        DD t;
-        for (int b = 0; b < nblk; ++b) t.merge(part[(long)b * 2 * FERMI_NSUM + 2 * s], part[(long)b * 2 * FERMI_NSUM + 2 * s + 1]);
-        tot[s] = t.hi + t.lo;
+    DD t;
+    if (fermi_sum_used(J, s)) {
+        for (int b = lane; b < nblk; b += 32)
+            t.merge(part[(long)b * 2 * FERMI_NSUM + 2 * s], part[(long)b * 2 * FERMI_NSUM + 2 * s + 1]);
+        for (int o = 16; o > 0; o >>= 1) {
+            const double h = __shfl_xor_sync(0xffffffffu, t.hi, o), l = __shfl_xor_sync(0xffffffffu, t.lo, o);
+            t.merge(h, l);
+        }
     }
+    if (lane == 0) tot[s] = t.hi + t.lo;
     __syncthreads();
-    if (s == 0) {
+    if (threadIdx.x == 0) {
         FermiOut o = *J.out;
         o.e_total = tot[0];
         o.fermi_shift = 0;
@@ -320,9 +366,10 @@ size_t fermi_part_bytes() { return sizeof(double) * 2 * FERMI_NSUM * FERMI_BLOCK
 
 void launch_fermi_sums(cudaStream_t s, FermiJob *djob, double *part)
 {
-    NRLTB_LAUNCH(k_fermi_level, 1, 1024, 0, s, djob);
-    NRLTB_LAUNCH(k_band_sums, FERMI_BLOCKS, 256, 0, s, djob, part);
-    NRLTB_LAUNCH(k_band_finish, 1, 32, 0, s, djob, part, FERMI_BLOCKS);
+    NRLTB_LAUNCH(k_fermi_level, FERMI_CL, FERMI_THREADS, 0, s, djob);
+    if (!part) return;   // E_F alone
+    NRLTB_LAUNCH(k_band_sums, FERMI_BLOCKS, FERMI_SUM_THREADS, 0, s, djob, part);
+    NRLTB_LAUNCH(k_band_finish, 1, 32 * FERMI_NSUM, 0, s, djob, part, FERMI_BLOCKS);
 }
 
 // One thread per (k, state, atom).  Z: batch column-major n2 x n2 eigenvectors

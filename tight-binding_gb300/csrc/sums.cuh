@@ -25,8 +25,8 @@ struct FermiJob {
 };
 
 // E_F, then the energy / pressure / entropy / spin sums: three launches on s
-// (one CTA for the Newton iteration, FERMI_BLOCKS CTAs for the sums, one to
-// merge them); part holds fermi_part_bytes() of device scratch.
+// (one cluster for the Newton iteration, FERMI_BLOCKS CTAs for the sums, one to
+// merge them); part holds fermi_part_bytes() of device scratch (null: E_F alone).
 constexpr int FERMI_BLOCKS = 152;
 size_t fermi_part_bytes();
 void launch_fermi_sums(cudaStream_t s, FermiJob *djob, double *part);
