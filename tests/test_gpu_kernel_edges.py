@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import oracle
-from nrltb import KMesh, synth
+from nrltb import KMesh, abi, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -127,3 +127,29 @@ def test_fp64_product_scales_and_specials(ctx, scale):
         hit = np.zeros((150, 80), bool)
         hit[140], hit[:, 11] = True, True
         assert (np.isfinite(got) == ~hit).all()
+
+
+def _pencils(n, nk, seed):
+    """nk Hermitian H and positive definite S = 1 + small, as (nk, n, n) arrays."""
+    rng = np.random.default_rng(seed)
+    H, S = _cplx(rng, (nk, n, n)), _cplx(rng, (nk, n, n)) * (0.1 / n)
+    H = H + H.conj().transpose(0, 2, 1)
+    return H, np.eye(n) + S @ S.conj().transpose(0, 2, 1)
+
+
+@pytest.mark.parametrize("n,batches", [(1, (2,)), (2, (3,)), (31, (160,)), (32, (310,)), (33, (80, 160)),
+                                       (64, (60, 330)), (65, (60, 160)), (128, (30, 40)), (129, (16, 40)),
+                                       (160, (160,)), (161, (30, 160)), (257, (12, 30)), (545, (6,)), (801, (20,))])
+def test_mixed_solve_does_not_depend_on_the_batch(ctx, n, batches):
+    """Cluster sizes 1, 2, 4 and 8 of the panel kernel, with 8 and 16 warps, one wave and more: the first two
+    matrices have the same eigenvalues and vectors, bit for bit, by themselves and ahead of others (the start of
+    the inverse iteration goes by a matrix's place); the values within the form's 1e-9 of the matrix norm."""
+    H, S = _pencils(n, 2, n)
+    first = ctx.diag(H, S, precision=abi.PREC_MIXED)
+    want = oracle.diag(H, S, vectors=False)[0]
+    assert (first[2] == 0).all() and np.abs(first[0] - want).max() <= 1e-9 * np.abs(want).max()
+    for nb in batches:
+        at = np.arange(nb) % 2
+        e, z, st = ctx.diag(H[at], S[at], precision=abi.PREC_MIXED)
+        assert (st == 0).all() and np.array_equal(e[:2], first[0]) and np.array_equal(z[:2], first[1])
+        assert np.abs(e - want[at]).max() <= 1e-9 * np.abs(want).max()

@@ -1141,10 +1141,10 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     // 4. tridiagonalisation: FP32 one cluster launch per panel (tri_panel.cuh); FP64,
     //    and where such a cluster cannot be scheduled, two launches per column
     //    (tri_col.cuh)
-    bool clusters = true;
+    bool clusters = sizeof(T) == 4;
     for (int j0 = 0; j0 < n; j0 += EIG_NB) {
         const int jb = std::min(EIG_NB, n - j0);
-        if (clusters) clusters = tri_panel_launch<T>(s, w, j0, jb);
+        if constexpr (sizeof(T) == 4) clusters = clusters && tri_panel_launch(s, w, j0, jb);
         if (!clusters) tri_columns<T>(s, w, j0, jb);
         if (std::min(j0 + jb - 1, n - 2) < j0) break;
         const int t0 = j0 + jb, rem = n - t0;
