@@ -1076,6 +1076,55 @@ __global__ void k_copy_vpanel(const C2 *V, long ld, long ms, C2 *VW, long ldw, l
     o[(long)(2 * EIG_NB + c) * ldw] = v;
 }
 
+// The FP64 form's copy.  Its product takes each row of [V W] as digits of one scale, and
+// V's entries are at most 1 while W's go as the norm of A: left as they are, a matrix of
+// norm 1e6 or 1e-6 would lose 20 bits of V or W.  So column c's pair is brought to one
+// size by powers of two, V_c 2^a and W_c 2^-a with a half the difference of their largest
+// exponents, which leaves V_c W_c^H + W_c V_c^H as it is; a pair whose V or W is zero adds
+// nothing and is cleared.  A CTA per column: a few us beside a product of 20 to 400.
+__global__ void __launch_bounds__(256) k_scale_vpanel(const double2 *V, long ld, long ms, double2 *VW, long ldw, long wps,
+                                                      int t0, int j0, int rem)
+{
+    __shared__ unsigned long long smx[2][8];
+    const int b = blockIdx.y, c = blockIdx.x, tid = threadIdx.x;
+    const double2 *v = V + b * ms + t0 + (long)(j0 + c) * ld;
+    double2 *o = VW + b * wps + t0 + (long)c * ldw, *wc = o + (long)EIG_NB * ldw, *o2 = wc + (long)EIG_NB * ldw;
+    auto part = [](double2 x) {   // as integers, so that a NaN is the largest
+        return max((unsigned long long)__double_as_longlong(fabs(x.x)), (unsigned long long)__double_as_longlong(fabs(x.y)));
+    };
+    unsigned long long mv = 0, mw = 0;
+    for (int r = tid; r < rem; r += 256) {
+        mv = max(mv, part(v[r]));
+        mw = max(mw, part(wc[r]));
+    }
+    for (int q = 16; q > 0; q >>= 1) {
+        mv = max(mv, (unsigned long long)__shfl_xor_sync(0xffffffffu, mv, q));
+        mw = max(mw, (unsigned long long)__shfl_xor_sync(0xffffffffu, mw, q));
+    }
+    if ((tid & 31) == 0) {
+        smx[0][tid >> 5] = mv;
+        smx[1][tid >> 5] = mw;
+    }
+    __syncthreads();
+    for (int q = 0; q < 8; ++q) {
+        mv = max(mv, smx[0][q]);
+        mw = max(mw, smx[1][q]);
+    }
+    const int ev = (int)(mv >> 52), ew = (int)(mw >> 52);
+    const bool keep = mv != 0 && mw != 0;
+    const int a = (ev < 2047 && ew < 2047) ? (ew - ev) >> 1 : 0;   // |a| <= 1023
+    const double up = a > -1023 ? __longlong_as_double((long long)(1023 + a) << 52) : 0x1p-1023;
+    const double dn = a < 1023 ? __longlong_as_double((long long)(1023 - a) << 52) : 0x1p-1023;
+    for (int r = tid; r < rem; r += 256) {
+        double2 x = v[r], y = wc[r];
+        x = keep ? make_double2(x.x * up, x.y * up) : make_double2(0, 0);
+        y = keep ? make_double2(y.x * dn, y.y * dn) : make_double2(0, 0);
+        o[r] = x;
+        o2[r] = x;
+        wc[r] = y;
+    }
+}
+
 __global__ void k_fill_int(int *p, int v, int count)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1153,8 +1202,11 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
             C2 *At = w.A + (long)t0 * (ld + 1);
             if (jb == EIG_NB) {
                 // A -= [Vp Wp] [Wp Vp]^H in one rank-64 update: Vp copied on both sides of W
-                NRLTB_LAUNCH(k_copy_vpanel<C2>, dim3(cdiv((long)rem * jb, 256), B), 256, 0, s, w.V, ld, ms, w.VW,
-                             (long)n, w.wps, t0, j0, jb, rem);
+                if constexpr (sizeof(T) == 4)
+                    NRLTB_LAUNCH(k_copy_vpanel<C2>, dim3(cdiv((long)rem * jb, 256), B), 256, 0, s, w.V, ld, ms, w.VW,
+                                 (long)n, w.wps, t0, j0, jb, rem);
+                else
+                    NRLTB_LAUNCH(k_scale_vpanel, dim3(jb, B), 256, 0, s, w.V, ld, ms, w.VW, (long)n, w.wps, t0, j0, rem);
                 zgemm<T>(s, rem, rem, 2 * EIG_NB, B, mone, w.VW + t0, n, w.wps, 0, w.VW + t0 + (long)n * EIG_NB, n,
                          w.wps, 1, one, At, ld, ms, 0, 0, 1, w.zs);
             } else {
