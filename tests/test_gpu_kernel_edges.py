@@ -181,3 +181,16 @@ def test_fp64_spectra(ctx, n, size):
     assert (st == 0).all() and (st2 == 0).all() and np.array_equal(e, e2)
     for name, got, w in zip(names, e, want):
         assert np.abs(got / size - w).max() <= 32 * n * 2.0 ** -53 * np.abs(w).max(), name
+
+
+@pytest.mark.parametrize("n", [2, 33, 64, 129, 200])
+@pytest.mark.parametrize("decades", [3, 30])
+def test_fp64_scaled_basis(ctx, n, decades):
+    """Basis functions scaled by powers of two: the same eigenvalues and, scaled back, the same vectors, bit for
+    bit, since every step is exact in such a scale."""
+    H, S = _pencils(n, 3, n)
+    D = 2.0 ** np.random.default_rng(n).integers(-3 * decades, 3 * decades + 1, (3, n))
+    e, z, st = ctx.diag(H, S)
+    e2, z2, st2 = ctx.diag(H * D[:, :, None] * D[:, None, :], S * D[:, :, None] * D[:, None, :])
+    assert (st == 0).all() and (st2 == 0).all()
+    assert np.array_equal(e, e2) and np.array_equal(z, z2 * D[:, :, None])

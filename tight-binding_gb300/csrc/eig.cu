@@ -58,6 +58,56 @@ template <typename T> void eig_work_carve(EigWork<T> &w, void *base, int n, int 
 }
 
 // ---------------------------------------------------------------------------
+// The FP64 form solves for D H D and D S D with D_i the power of two that brings S_ii into
+// [1, 4).  Its products are exact in digits of one scale per row and per column of an
+// operand, but not along their inner index: in L^{-1} times L or L^{-1} times H the scale
+// of the basis functions runs along it, the other way in either factor, and a basis whose
+// norms differ by 1e4 would cost eight digits.  Every step is as exact with D as without;
+// overlaps with a diagonal of ones, as tight binding has, are copied as they are.
+// S_ii that is not a positive normal number (the factorisation will fail there): D_i = 1.
+__global__ void k_unit_exp(const double2 *S, int *ex, int n, int batch)
+{
+    const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (t >= (long)n * batch) return;
+    const long b = t / n;
+    const int i = (int)(t - b * n);
+    const long long bits = __double_as_longlong(S[b * n * n + i * (n + 1L)].x);
+    const int e = (int)(bits >> 52);   // negative for negative numbers
+    ex[t] = (e >= 1 && e <= 2046) ? -((e - 1023) >> 1) : 0;
+}
+
+// L = D S D, A = D H D
+__global__ void k_to_unit(const double2 *__restrict__ S, const double2 *__restrict__ H, double2 *__restrict__ L,
+                          double2 *__restrict__ A, const int *ex, int n)
+{
+    const unsigned nn = (unsigned)n * n, b = blockIdx.y;
+    const long at = b * (long)nn;
+    ex += (long)b * n;
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < nn; t += gridDim.x * blockDim.x) {
+        const unsigned c = t / n, r = t - c * n;
+        double2 s = S[at + t], h = H[at + t];
+        const int er = ex[r], ec = ex[c];
+        if (er | ec) {
+            const double dr = __longlong_as_double((long long)(1023 + er) << 52);
+            const double dc = __longlong_as_double((long long)(1023 + ec) << 52);
+            s = make_double2(s.x * dr * dc, s.y * dr * dc);
+            h = make_double2(h.x * dr * dc, h.y * dr * dc);
+        }
+        L[at + t] = s;
+        A[at + t] = h;
+    }
+}
+
+// columns of Wi by D: X = (Wi D)^H Z then has the vectors of H and S
+__global__ void k_from_unit(double2 *Wi, const int *ex, int n)
+{
+    const int e = ex[(long)blockIdx.y * n + blockIdx.x];
+    if (e == 0) return;
+    const double d = __longlong_as_double((long long)(1023 + e) << 52);
+    double2 *w = Wi + blockIdx.y * (long)n * n + blockIdx.x * (long)n;
+    for (int r = threadIdx.x; r < n; r += blockDim.x) w[r] = make_double2(w[r].x * d, w[r].y * d);
+}
+
 template <typename C2>
 __global__ void k_convert_h(const double2 *__restrict__ src, C2 *__restrict__ dst, long count)
 {
@@ -1143,8 +1193,14 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     const long cnt = (long)n * n * B;
     cudaMemsetAsync(w.status, 0, sizeof(int) * B, s);
     // 0. inputs in working precision: S -> L, H -> A (A is free until step 3)
-    NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, S, w.L, cnt);
-    NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, H, w.A, cnt);
+    int *const ex = (int *)w.d;   // FP64: exponents of D, until step 4
+    if constexpr (sizeof(T) == 4) {
+        NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, S, w.L, cnt);
+        NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, H, w.A, cnt);
+    } else {
+        NRLTB_LAUNCH(k_unit_exp, cdiv((long)n * B, 128), 128, 0, s, S, ex, n, B);
+        NRLTB_LAUNCH(k_to_unit, dim3((unsigned)std::min(cdiv((long)n * n, 256), 512), B), 256, 0, s, S, H, w.L, w.A, ex, n);
+    }
     // 1. Cholesky S = L L^H
     for (int j0 = 0; j0 < n; j0 += EIG_NB) {
         const int jb = std::min(EIG_NB, n - j0), rem = n - j0 - jb;
@@ -1186,6 +1242,9 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
         zgemm<T>(s, n, n, n, B, one, w.A, ld, ms, 0, w.Wi, ld, ms, 1, zero, w.Y, ld, ms, 0, 1, 0, w.zs);
     }
     zgemm<T>(s, n, n, n, B, one, w.Wi, ld, ms, 0, w.Y, ld, ms, 0, zero, w.A, ld, ms, 1, 0, 1, w.zs);
+    if constexpr (sizeof(T) == 8) {
+        if (vectors) NRLTB_LAUNCH(k_from_unit, dim3(n, B), 128, 0, s, w.Wi, ex, n);
+    }
     if (tri_start) cudaEventRecord(tri_start, s);
     // 4. tridiagonalisation: FP32 one cluster launch per panel (tri_panel.cuh); FP64,
     //    and where such a cluster cannot be scheduled, two launches per column
