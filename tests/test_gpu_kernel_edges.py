@@ -194,3 +194,26 @@ def test_fp64_scaled_basis(ctx, n, decades):
     e2, z2, st2 = ctx.diag(H * D[:, :, None] * D[:, None, :], S * D[:, :, None] * D[:, None, :])
     assert (st == 0).all() and (st2 == 0).all()
     assert np.array_equal(e, e2) and np.array_equal(z, z2 * D[:, :, None])
+
+
+@pytest.mark.parametrize("n,batches", [(1, (70,)), (16, (9,)), (17, (300,)), (32, (40,)), (33, (4,)), (65, (160,)),
+                                       (112, (20,)), (113, (20, 60)), (160, (20, 80)), (161, (12, 40)), (192, (20, 80)),
+                                       (193, (20, 60)), (225, (30,)), (300, (12,))])
+def test_fp64_solve_does_not_depend_on_the_batch(ctx, n, batches):
+    """One CTA, clusters of 8, 4 and 2, and columns ahead of a cluster: the first two matrices have the same
+    eigenvalues and vectors, bit for bit, by themselves and ahead of others; values, residuals and S-orthonormality
+    as a backward stable solve leaves them, 64 n 2^-53 of the norm (S is within 2 of one)."""
+    H, S = _pencils(n, 2, n)
+    first = ctx.diag(H, S)
+    want = oracle.diag(H, S, vectors=False)[0]
+    norm, tol = np.abs(want).max(), 64 * n * 2.0 ** -53
+    assert (first[2] == 0).all() and np.abs(first[0] - want).max() <= tol * norm
+    for j in (0, 1):
+        e, z = first[0][j], first[1][j]
+        assert np.abs(H[j] @ z - (S[j] @ z) * e).max() <= tol * norm
+        assert np.abs(z.conj().T @ S[j] @ z - np.eye(n)).max() <= 1e-9   # (dstein's: eps norm / gap outside clusters)
+    for nb in batches:
+        at = np.arange(nb) % 2
+        e, z, st = ctx.diag(H[at], S[at])
+        assert (st == 0).all() and np.array_equal(e[:2], first[0]) and np.array_equal(z[:2], first[1])
+        assert np.abs(e - want[at]).max() <= tol * norm

@@ -4,6 +4,8 @@
 #include "eig.cuh"
 #include "tri_col.cuh"
 #include "tri_panel.cuh"
+#include "tri_small.cuh"
+#include "tri_cluster.cuh"
 
 namespace nrltb {
 
@@ -1246,11 +1248,22 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
         if (vectors) NRLTB_LAUNCH(k_from_unit, dim3(n, B), 128, 0, s, w.Wi, ex, n);
     }
     if (tri_start) cudaEventRecord(tri_start, s);
-    // 4. tridiagonalisation: FP32 one cluster launch per panel (tri_panel.cuh); FP64,
-    //    and where such a cluster cannot be scheduled, two launches per column
-    //    (tri_col.cuh)
+    // 4. tridiagonalisation: FP32 one cluster launch per panel (tri_panel.cuh); FP64 one
+    //    launch for a small matrix (tri_small.cuh) or for the last TK_MAX columns of a
+    //    larger one (tri_cluster.cuh).  The other columns, and all of them where a cluster
+    //    cannot be scheduled, two launches each (tri_col.cuh)
     bool clusters = sizeof(T) == 4;
-    for (int j0 = 0; j0 < n; j0 += EIG_NB) {
+    int from = 0;   // the columns that are left to the loop
+    if constexpr (sizeof(T) == 8) {
+        if (n <= TS_MAX) {
+            tri_small(s, w);
+            from = n;
+        }
+    }
+    for (int j0 = from; j0 < n; j0 += EIG_NB) {
+        if constexpr (sizeof(T) == 8) {
+            if (tri_cluster(s, w, j0)) break;
+        }
         const int jb = std::min(EIG_NB, n - j0);
         if constexpr (sizeof(T) == 4) clusters = clusters && tri_panel_launch(s, w, j0, jb);
         if (!clusters) tri_columns<T>(s, w, j0, jb);

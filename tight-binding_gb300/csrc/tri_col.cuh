@@ -1,7 +1,7 @@
 // tri_col.cuh -- one column of the blocked Householder tridiagonalisation
 // (zhetrd/zlatrd steps) in two launches over the whole GPU.  The FP64 form takes
-// this path (its mat-vec is bound by the FP64 pipe, so every SM must work on every
-// column); the FP32 form where a cluster panel (tri_panel.cuh) cannot be scheduled.
+// this path down to its last 192 columns (its mat-vec is bound by the FP64 pipe, so every
+// SM must work on every column; the rest: tri_cluster.cuh); the FP32 form where a cluster panel (tri_panel.cuh) cannot be scheduled.
 //
 //   k_tri_col  finishes W of the column before (w = w' + alpha v) and updates column
 //              i:  a_i - V W[i,:]^H - W V[i,:]^H, with per-CTA partials of |a_i|^2.
@@ -95,6 +95,51 @@ __device__ __forceinline__ void tc_root(float x, float &s, float &r)
 {
     s = sqrtf(x);
     r = 1.f / s;
+}
+
+// The reflector of (al, x), |x|^2 = xn2: H (al, x) = (beta, 0) with v = (1, scale x).
+// FP64: one chain of 13 operations from the FP32 root and reciprocal, each followed by
+// one step of third order (relative errors 2^-22 -> 2^-64, then FP64 rounding):
+//   1/sqrt(N):  y + y e (1/2 + 3/8 e),  e = 1 - N y^2;  the root N y takes the same step
+//   1/D:        r + r (e + e^2),        e = 1 - D r
+// with the exponents taken out, and back in, as integers.
+__device__ __forceinline__ void tc_reflector(double2 al, double xn2, double2 &tau, double2 &scale, double &beta)
+{
+    tau = scale = make_double2(0, 0);
+    beta = al.x;
+    if (xn2 == 0 && al.y == 0) return;
+    const double N = fma(al.y, al.y, fma(al.x, al.x, xn2));
+    int e = ((__double2hiint(N) >> 20) & 0x7FF) - 1023;
+    double g, y;   // sqrt(N), 1 / sqrt(N)
+    if (e < -1000 || e > 1000) {
+        g = sqrt(N);
+        y = 1.0 / g;
+    } else {
+        e &= ~1;
+        const double m = __hiloint2double(__double2hiint(N) - (e << 20), __double2loint(N));   // [1, 4)
+        const double y0 = f2d_exact(rsqrtf(d2f_rn(m))), g0 = m * y0, r = fma(-g0, y0, 1.0);
+        const double p = fma(0.375, r, 0.5) * r;
+        g = fma(g0, p, g0);
+        y = fma(y0, p, y0);
+        g = __hiloint2double(__double2hiint(g) + ((e / 2) << 20), __double2loint(g));
+        y = __hiloint2double(__double2hiint(y) - ((e / 2) << 20), __double2loint(y));
+    }
+    if (al.x >= 0) { g = -g; y = -y; }
+    const double2 den = make_double2(al.x - g, al.y);   // 1 / (alpha - beta)
+    const double D = fma(den.x, den.x, den.y * den.y);
+    const int f = ((__double2hiint(D) >> 20) & 0x7FF) - 1023;
+    double rd;
+    if (f < -1000 || f > 1000) {
+        rd = 1.0 / D;
+    } else {
+        const double m = __hiloint2double(__double2hiint(D) - (f << 20), __double2loint(D));   // [1, 2)
+        const double r0 = f2d_exact(__frcp_rn(d2f_rn(m))), r = fma(-m, r0, 1.0);
+        rd = fma(r0, fma(r, r, r), r0);
+        rd = __hiloint2double(__double2hiint(rd) - (f << 20), __double2loint(rd));
+    }
+    scale = make_double2(den.x * rd, -den.y * rd);
+    tau = make_double2((g - al.x) * y, -al.y * y);
+    beta = g;
 }
 
 // Programmatic dependent launch: a kernel lets its successor start once all its CTAs
