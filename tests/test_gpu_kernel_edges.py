@@ -84,6 +84,26 @@ def test_fp64_product_shapes(ctx, m, n, k, batch, opA, opB):
         _zgemm_check(_zgemm(ctx, 1, opA, opB, (0, 0, 0), alpha, beta, A, B, Cm), M, N, Cm, (0, 0, 0), alpha, beta)
 
 
+@pytest.mark.parametrize("m,n,k,batch", [(1, 1, 1, 300), (9, 9, 9, 57), (15, 15, 1, 4), (15, 15, 200, 2), (3, 15, 40, 5),
+                                         (15, 4, 0, 3), (16, 15, 20, 2)])
+@pytest.mark.parametrize("opA,opB", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("triA,triB", [(0, 0), (1, 0), (2, 0), (0, 1), (0, 2)])
+def test_fp64_small_products(ctx, m, n, k, batch, opA, opB, triA, triB):
+    """A thread per element: several matrices a CTA, a remainder of CTAs, the largest order and the next one."""
+    rng = np.random.default_rng(m + n + k)
+    A, B = _cplx(rng, (batch, m, k) if opA else (batch, k, m)), _cplx(rng, (batch, k, n) if opB else (batch, n, k))
+    Cm = _cplx(rng, (batch, n, m))
+    M = A.conj() if opA else A.transpose(0, 2, 1)
+    N = B.conj() if opB else B.transpose(0, 2, 1)
+    r, s = np.arange(m)[:, None] - np.arange(k), np.arange(k)[:, None] - np.arange(n)
+    M = M * (r >= 0 if triA == 1 else r <= 0 if triA == 2 else True)
+    N = N * (s <= 0 if triB == 1 else s >= 0 if triB == 2 else True)
+    for alpha, beta in ((1.0, 0.0), (-1.0, 1.0)):
+        got = _zgemm(ctx, 1, opA, opB, (triA, triB, 0), alpha, beta, A, B, Cm).transpose(0, 2, 1)
+        want = alpha * (M @ N) + beta * Cm.transpose(0, 2, 1)
+        assert (np.abs(got - want) <= (k + 2) * 2.0 ** -51 * (np.abs(M) @ np.abs(N) + np.abs(Cm.transpose(0, 2, 1)))).all()
+
+
 @pytest.mark.parametrize("n,batch", [(65, 1), (200, 6), (385, 5)])
 @pytest.mark.parametrize("tri", [(1, 0, 0), (2, 0, 0), (0, 1, 0), (0, 2, 0), (0, 0, 1), (0, 0, 2), (1, 0, 1), (2, 0, 2)])
 def test_fp64_product_triangles(ctx, n, batch, tri):

@@ -155,6 +155,46 @@ zgemm_kernel(GemmArgs<T> g)
     }
 }
 
+// FP64 products of at most 15 x 15: a thread per element of C, whole matrices to a CTA
+// (which therefore may be read and written by one product, as in the tiled kernel), the
+// same sums.  The FP64 pipe takes 64 clocks of an SM's quarter for a warp's operation
+// whatever its lanes hold, and a 64 x 32 tile filled with 9 x 9 elements wastes 24 of 25;
+// 1728 products of order 9: 393 -> 21 us.
+constexpr int ZGEMM_SMALL = 15, ZGEMM_SMALL_THREADS = 256;
+
+__global__ static void __launch_bounds__(ZGEMM_SMALL_THREADS) zgemm_small_kernel(GemmArgs<double> g)
+{
+    const int mn = g.m * g.n, per = ZGEMM_SMALL_THREADS / mn, t = threadIdx.x;
+    const long b = (long)blockIdx.x * per + t / mn;
+    const int e = t % mn, j = e / g.m, i = e - j * g.m;
+    const bool on = t < per * mn && b < g.batch;
+    double2 *c = nullptr;
+    double2 v = make_double2(0, 0);
+    if (on) {
+        const double2 *A = g.A + b * g.sA + (g.opA ? i * g.lda : (long)i);
+        const double2 *B = g.B + b * g.sB + (g.opB ? (long)j : j * g.ldb);
+        const long ia = g.opA ? 1 : g.lda, ib = g.opB ? g.ldb : 1;
+        int k = 0, kend = g.k;
+        if (g.triA == 1) kend = min(kend, i + 1);
+        if (g.triA == 2) k = max(k, i);
+        if (g.triB == 1) kend = min(kend, j + 1);
+        if (g.triB == 2) k = max(k, j);
+        double2 acc = make_double2(0, 0);
+#pragma unroll 4
+        for (; k < kend; ++k) {
+            double2 a = A[k * ia], x = B[k * ib];
+            if (g.opA) a.y = -a.y;
+            if (g.opB) x.y = -x.y;
+            cfma(acc, a, x);
+        }
+        c = g.C + b * g.sC + i + j * g.ldc;
+        v = cmul(g.alpha, acc);
+        if (g.beta.x != 0 || g.beta.y != 0) v = cadd(v, cmul(g.beta, *c));
+    }
+    __syncthreads();
+    if (on) *c = v;
+}
+
 // FP32 on the tensor cores: tcgen05 with tensor-memory accumulators for
 // op(A) = A (gemm_umma.cu), mma.sync otherwise (gemm_tc.cu)
 void zgemm_tc_launch(cudaStream_t s, const GemmArgs<float> &g);
@@ -263,6 +303,13 @@ void zgemm_simt(cudaStream_t s, int m, int n, int k, int batch, typename cplx<T>
     constexpr int BM = 64, BN = 64, TM = 4, TN = 4;
     dim3 grid(cdiv(m, BM), cdiv(n, BN), batch);
     cudaEvent_t ev = kt_begin(s);
+    if constexpr (sizeof(T) == 8) {
+        if (m <= ZGEMM_SMALL && n <= ZGEMM_SMALL) {
+            NRLTB_LAUNCH(zgemm_small_kernel, cdiv(batch, ZGEMM_SMALL_THREADS / (m * n)), ZGEMM_SMALL_THREADS, 0, s, g);
+            if (ev) kt_end(ev, s, KC_GEMM_SIMT, 8.0 * gemm_useful_macs(m, n, k, triA, triB, triC) * batch);
+            return;
+        }
+    }
     // short k (the rank-32 panel updates): the whole k range in one or two
     // shared-memory stages instead of four to eight; n <= 32 (the Cholesky
     // panel solves) on 64 x 32 tiles.  Every element's k loop is the same in
