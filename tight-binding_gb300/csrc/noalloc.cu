@@ -142,11 +142,9 @@ extern "C" int nrltb_search2_noalloc(int device, void *stream, int natoms, const
         nrltb_internal_set_error(msg);
         return NRLTB_E_ARG;
     }
-    k_search_eval<<<std::min(cdiv(ncand, 256), 152 * 16), 256, 0, s>>>(S, P, ncand, code, misc, dmin);
-    if (cudaMemcpyAsync(host_misc, misc, sizeof host_misc, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess)
-        return NRLTB_E_CUDA;
-    k_search_ties<<<1, 1, 0, s>>>(code, ncand, kneigh_in, misc + 2, host_misc[0] > 0);
+    const int G = search_groups(natoms, box);
+    k_search_eval<<<cdiv(G * box, 256), 256, 0, s>>>(S, P, (int)box, G, code, misc, dmin);
+    k_search_ties<<<1, 1, 0, s>>>(code, ncand, kneigh_in, misc, misc + 2);
     k_search_count<<<nblk, SEARCH_BLOCK, 0, s>>>(code, ncand, blk);
     k_scan_small<<<1, 1024, 0, s>>>(blk, nblk, misc + 1);
     if (cudaMemcpyAsync(host_misc, misc, sizeof host_misc, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -156,8 +154,10 @@ extern "C" int nrltb_search2_noalloc(int device, void *stream, int natoms, const
     DevPairs out;
     out.tt = d_tt; out.dlv = d_dlv; out.dist = d_dist; out.screen = d_screen; out.dscrn = d_dscrn;
     out.jkind = d_jkind; out.jatm = d_jatm;
-    if (capacity > 0)
-        k_search_scatter<<<nblk, SEARCH_BLOCK, 0, s>>>(S, P, code, ncand, blk, out, capacity);
+    if (const int count = std::min(total, capacity)) {
+        k_search_scatter<<<nblk, SEARCH_BLOCK, 0, s>>>(code, ncand, blk, out, count);
+        k_search_pairs<<<cdiv(count, 64), 64, 0, s>>>(S, P, out, count);
+    }
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return NRLTB_E_CUDA;
     *npairs = total;
     if (kneigh_out) *kneigh_out = host_misc[2];

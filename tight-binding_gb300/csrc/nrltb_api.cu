@@ -411,17 +411,14 @@ static int run_search2(nrltb_ctx *c, int kneigh_in)
     CK(cudaMemcpyAsync(dmin, &inf, 8, cudaMemcpyHostToDevice, s));
     DevStructure DS = dev_structure(c);
     DevParams DP = dev_params(c);
-    NRLTB_LAUNCH(k_search_eval, std::min(cdiv(ncand, 256), 152 * 16), 256, 0, s, DS, DP, ncand,
-                 c->d_code.as<unsigned char>(), misc, dmin);
-    CKL();
-    int host_misc[6];
-    CK(cudaMemcpyAsync(host_misc, misc, sizeof host_misc, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    const int ties = host_misc[0];
-    NRLTB_LAUNCH(k_search_ties, 1, 1, 0, s, c->d_code.as<unsigned char>(), ncand, kneigh_in, misc + 2, ties > 0);
+    const int G = search_groups(S.natoms, box);
+    NRLTB_LAUNCH(k_search_eval, cdiv(G * box, 256), 256, 0, s, DS, DP, (int)box, G, c->d_code.as<unsigned char>(), misc,
+                 dmin);
+    NRLTB_LAUNCH(k_search_ties, 1, 1, 0, s, c->d_code.as<unsigned char>(), ncand, kneigh_in, misc, misc + 2);
     NRLTB_LAUNCH(k_search_count, nblk, SEARCH_BLOCK, 0, s, c->d_code.as<unsigned char>(), ncand, c->d_blk.as<int>());
     NRLTB_LAUNCH(k_scan_small, 1, 1024, 0, s, c->d_blk.as<int>(), nblk, misc + 1);
     CKL();
+    int host_misc[6];
     CK(cudaMemcpyAsync(host_misc, misc, sizeof host_misc, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     const int total = host_misc[1];
@@ -434,8 +431,11 @@ static int run_search2(nrltb_ctx *c, int kneigh_in)
     c->npairs = total;
     RET(c->d_pairs.ensure(pairs_bytes(std::max(total, 1))));
     DevPairs P = pairs_view(c, std::max(total, 1));
-    NRLTB_LAUNCH(k_search_scatter, nblk, SEARCH_BLOCK, 0, s, DS, DP, c->d_code.as<unsigned char>(), ncand,
-                 c->d_blk.as<int>(), P, total);
+    if (total > 0) {
+        NRLTB_LAUNCH(k_search_scatter, nblk, SEARCH_BLOCK, 0, s, c->d_code.as<unsigned char>(), ncand, c->d_blk.as<int>(), P,
+                     total);
+        NRLTB_LAUNCH(k_search_pairs, cdiv(total, 64), 64, 0, s, DS, DP, P, total);
+    }
     CKL();
     return NRLTB_OK;
 }

@@ -1,6 +1,7 @@
 // setup.cuh -- device views of the structure, parameters, pair list and the
 // k-independent Slater-Koster tables, and the kernels of setup.cu.
 #pragma once
+#include <algorithm>
 #include "common.cuh"
 
 #define NRLTB_MAX_KINDS 8
@@ -45,13 +46,19 @@ struct DevSK {
     double *E;                          // [4][P][81] SK blocks: H, S, dH, dS
 };
 
-__global__ void k_search_eval(DevStructure S, DevParams P, long ncand, unsigned char *code, int *tie_count,
+__global__ void k_search_eval(DevStructure S, DevParams P, int box, int G, unsigned char *code, int *tie_count,
                               unsigned long long *dismin_bits);
-__global__ void k_search_ties(unsigned char *code, long ncand, int kneigh_in, int *kneigh_out, int resolve);
+// its groups of atom pairs: as many as fill the device with a thread per image and group twice over
+inline int search_groups(int natoms, long box)
+{
+    return (int)std::min<long>((long)natoms * natoms, std::max(1L, 152L * 4096 / box));
+}
+__global__ void k_search_ties(unsigned char *code, long ncand, int kneigh_in, const int *tie_count, int *kneigh_out);
 __global__ void k_search_count(const unsigned char *code, long ncand, int *blockcnt);
 __global__ void k_scan_small(int *cnt, int nblk, int *total);
-__global__ void k_search_scatter(DevStructure S, DevParams P, const unsigned char *code, long ncand,
-                                 const int *blockoff, DevPairs out, int capacity);
+__global__ void k_search_scatter(const unsigned char *code, long ncand, const int *blockoff, DevPairs out,
+                                 int capacity);
+__global__ void k_search_pairs(DevStructure S, DevParams P, DevPairs out, int count);
 __global__ void k_setpar_pairs(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, int deriv);
 __global__ void k_setpar_atoms(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, int deriv);
 __global__ void k_sk_blocks(DevPairs pr, int npairs, DevSK sk, int nwhich);
