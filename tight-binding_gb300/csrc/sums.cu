@@ -72,7 +72,7 @@ __device__ __forceinline__ int count_below(const double *e, int m, double x)
 // CTAs' compensated partials are merged in rank order by every CTA, which all take
 // the same step; one cluster barrier per step, the slots alternate.
 // One CTA of 1024 threads took 0.71 ms for 27 rows of 1152 states and 5.3 ms for 1728
-// rows of 9; this 0.10 and 0.33.
+// rows of 9; this 0.10 and 0.22 (0.33 before the short rows' window states were gathered).
 constexpr int FERMI_CL = 8, FERMI_THREADS = 128, FERMI_ROW_MIN = 64;
 constexpr int FERMI_WARPS = FERMI_CL * FERMI_THREADS / 32;
 
@@ -119,6 +119,7 @@ __global__ void __cluster_dims__(FERMI_CL, 1, 1) __launch_bounds__(FERMI_THREADS
     namespace cg = cooperative_groups;
     __shared__ double sh[6][FERMI_THREADS / 32];
     __shared__ FermiSlot slots[2], edge;
+    __shared__ double2 wait[FERMI_THREADS / 32][64];
     cg::cluster_group cl = cg::this_cluster();
     FermiJob J = jobs[0];
     const int nv = J.nv, nk = J.nk, tid = threadIdx.x, lane = tid & 31;
@@ -208,13 +209,33 @@ __global__ void __cluster_dims__(FERMI_CL, 1, 1) __launch_bounds__(FERMI_THREADS
                     for (int i = lo + lane; i < hi; i += 32) window(e[i], wk);
                 }
             } else {
-                for (long q = gt; q < tot; q += nt) {
-                    const int k = (int)(q / nv), i = (int)(q - (long)k * nv);
-                    const double e = J.eig[(long)k * J.ldk + i];
-                    const double wk = J.w[k];
-                    if (e < mum20) ns.add(wk);
-                    else if (e < mup20) window(e, wk);
+                // the window's states wait until they fill a warp: its exponential and
+                // quotient are some 60 FP64 operations whatever the lanes hold
+                double2 *const pend = wait[tid >> 5];
+                int np = 0;
+                for (long q0 = gt - lane; q0 < tot; q0 += nt) {
+                    const long q = q0 + lane;
+                    double e = 0, wk = 0;
+                    bool in = false;
+                    if (q < tot) {
+                        const int k = (int)(q / nv), i = (int)(q - (long)k * nv);
+                        e = J.eig[(long)k * J.ldk + i];
+                        wk = J.w[k];
+                        if (e < mum20) ns.add(wk);
+                        else in = e < mup20;
+                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, in);
+                    if (in) pend[np + __popc(m & ((1u << lane) - 1))] = make_double2(e, wk);
+                    np += __popc(m);
+                    __syncwarp();
+                    if (np >= 32) {
+                        np -= 32;
+                        window(pend[np + lane].x, pend[np + lane].y);
+                        __syncwarp();
+                    }
                 }
+                if (lane < np) window(pend[lane].x, pend[lane].y);
+                __syncwarp();
             }
             double nsum, dnsum;
             fermi_totals(cl, ns, dns, &slots[it & 1], sh, nsum, dnsum);
