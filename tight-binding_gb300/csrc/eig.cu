@@ -964,6 +964,11 @@ __global__ void __launch_bounds__(EIG_WY) k_larft_wy(const float2 *G, float2 *Tm
 // One CTA per matrix with T in global memory took 1.38 ms a block of 128 at 4 k, this
 // 0.28; at 64 k 0.95 against 0.54.
 constexpr int LARFT_RC = 8;
+// T = [T1, -T1 G12 T2; 0, T2] for the reflectors before and from LARFT_HALF on: only T1
+// and T2 are formed here, which is a quarter of the operations and half of the chain, the
+// corner by two digit products (wy_block): a block of 128 with these products, n = 144 218 ->
+// 150 us (charges of 16 atoms), n = 288, 64 matrices 543 -> 310.
+constexpr int LARFT_HALF = 64;
 __global__ void __launch_bounds__(128) k_larft_rows(const double2 *G, double2 *Tm, const double2 *tau, int n, int j0,
                                                     int jb, int nbw)
 {
@@ -976,6 +981,7 @@ __global__ void __launch_bounds__(128) k_larft_rows(const double2 *G, double2 *T
     double2 *Tb = Tm + (long)b * nbw * nbw;
     const double2 *tb = tau + (long)b * n + j0;
     double2 *t = trow[rl];
+    if (cbeg < LARFT_HALF) jb = min(jb, LARFT_HALF);   // a multiple of the CTA's rows
     for (int c0 = cbeg / LARFT_RC * LARFT_RC; c0 < jb; c0 += LARFT_RC) {
         const int cn = min(LARFT_RC, jb - c0);
         __syncthreads();
@@ -1305,8 +1311,16 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
             NRLTB_LAUNCH(k_larft_wy, B, EIG_WY, sm, st, (const float2 *)G, (float2 *)Tf_of(j0), (const float2 *)w.tau, n,
                          j0, jb, nbw);
         } else {
-            NRLTB_LAUNCH(k_larft_rows, dim3(cdiv(jb, 16), B), 128, 0, st, (const double2 *)G, (double2 *)Tf_of(j0),
+            C2 *const Tf = Tf_of(j0);
+            NRLTB_LAUNCH(k_larft_rows, dim3(cdiv(jb, 16), B), 128, 0, st, (const double2 *)G, (double2 *)Tf,
                          (const double2 *)w.tau, n, j0, jb, nbw);
+            if (jb > LARFT_HALF) {   // T1 G12, then that times T2, in T's corner
+                const int h = LARFT_HALF, j2 = jb - h;
+                C2 *const T12 = Tf + (long)h * nbw;
+                zgemm<T>(st, h, j2, h, B, one, Tf, nbw, sG, 0, G + (long)h * nbw, nbw, sG, 0, zero, T12, nbw, sG, 2, 0, 0,
+                         w.zs);
+                zgemm<T>(st, h, j2, j2, B, mone, T12, nbw, sG, 0, T12 + h, nbw, sG, 0, zero, T12, nbw, sG, 0, 1, 0, w.zs);
+            }
         }
     };
     const int j0last = nref >= 1 ? ((nref - 1) / nbw) * nbw : -1;
