@@ -579,7 +579,9 @@ template <int CL, int NW> inline bool tp_try(cudaStream_t s, const EigWork<float
 //   n = 1404, 8 matrices  (CL 8)        37.0 -> 31.3 ms
 // and whole calls whose matrices don't fit (two waves and more): n = 72, 600 matrices:
 // 11.4 ms with 16 warps, 9.4 with CL 2, 7.9 as here; n = 144, 400 matrices: 19.1, 16.1, 14.5.
-// Clusters of 16 gained nothing (n = 1800, one matrix: 38.0 against 38.2 ms).
+// Clusters of 16 gained nothing (n = 1300, one matrix: panels 26.5 against 26.7 ms), though
+// each SM then has half of the mat-vec: what the SMs of a cluster, which are neighbours,
+// can read from L2 together seems to set the pace.
 inline bool tri_panel_launch(cudaStream_t s, const EigWork<float> &w, int j0, int jb)
 {
     const int tiles = cdiv(w.n, 32), left = cdiv(w.n - j0, 32);

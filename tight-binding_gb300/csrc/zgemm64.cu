@@ -65,6 +65,11 @@ struct ZOperand {
     int tile_rows;        // rows of a tile: 128 (A), 64 (X)
 };
 
+// Longest rows whose exponents the digit kernel forms: each of their up to four chunks reads the
+// whole row again.  Against a launch for them, a preparation of K = 64 or 128: N = 288, 64
+// matrices 56 -> 36 us, N = 144, 15 matrices 28 -> 16; rows up to 192 lost (charges of 16
+// atoms, K = 144: 11.30 -> 11.45 ms a call).
+constexpr int Z_FUSE = 128;
 enum ZOrder { Z_BY_MATRIX, Z_ROWS_UP, Z_ROWS_DOWN, Z_COLS_UP, Z_COLS_DOWN, Z_LOWER };
 constexpr int Z_GROUP = 4;   // matrices whose tiles are dealt together (see z_tile)
 
@@ -92,6 +97,24 @@ __device__ __forceinline__ int z_exp_above(unsigned long long bits)
 
 __device__ __forceinline__ bool z_in(int tri, int r, int k) { return tri == 0 || (tri == 1 ? k <= r : k >= r); }
 
+__device__ __forceinline__ void z_stat(double2 v, unsigned long long &mx, double &sum)
+{
+    const double ar = fabs(v.x), ai = fabs(v.y);
+    mx = max(mx, max((unsigned long long)__double_as_longlong(ar), (unsigned long long)__double_as_longlong(ai)));
+    sum += ar + ai;
+}
+// the exponents ex, la of a row's largest magnitude and sum
+__device__ __forceinline__ int2 z_row_exps(unsigned long long mx, double sum)
+{
+    const bool bad = mx >= (0x7FFull << 52);
+    const int e = bad ? Z_BAD : z_exp_above(mx);
+    // the sum's own rounding (K 2^-53 relative) widens it by 2^-30
+    const double s = sum * (1.0 + 0x1p-30);
+    int l = (mx && !bad && s < 0x1p1000) ? z_exp_above((unsigned long long)__double_as_longlong(s)) : e;
+    if (!bad && s >= 0x1p1000) l = e + 19;   // more than the 2^17 elements of a row can add
+    return make_int2(e, bad ? Z_BAD : max(l, e));
+}
+
 // Largest magnitude and sum of magnitudes of every row.  One CTA per 32 rows, a
 // warp's lanes over rows (BYROW: rows are contiguous) or over k.
 template <bool BYROW>
@@ -114,18 +137,10 @@ __device__ __forceinline__ void z_stats_rows(const ZOperand &o, int block, int b
                 if (z_in(o.tri, r, k + 32 * u)) v[u] = P[r * o.sr + (k + 32 * u) * o.sk];
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const double ar = fabs(v[u].x), ai = fabs(v[u].y);
-                mx = max(mx, max((unsigned long long)__double_as_longlong(ar), (unsigned long long)__double_as_longlong(ai)));
-                sum += ar + ai;
-            }
+            for (int u = 0; u < 4; ++u) z_stat(v[u], mx, sum);
         }
         for (; k < o.K; k += 32) {
-            if (!z_in(o.tri, r, k)) continue;
-            const double2 v = P[r * o.sr + k * o.sk];
-            const double ar = fabs(v.x), ai = fabs(v.y);
-            mx = max(mx, max((unsigned long long)__double_as_longlong(ar), (unsigned long long)__double_as_longlong(ai)));
-            sum += ar + ai;
+            if (z_in(o.tri, r, k)) z_stat(P[r * o.sr + k * o.sk], mx, sum);
         }
     }
     if (BYROW) {   // warps hold parts of the same 32 rows: transpose, then a warp per row
@@ -141,14 +156,9 @@ __device__ __forceinline__ void z_stats_rows(const ZOperand &o, int block, int b
     }
     if (lane == 0 && r0 + warp < o.rp) {
         const long at = (long)b * o.rp + r0 + warp;
-        const bool bad = mx >= (0x7FFull << 52);
-        const int e = bad ? Z_BAD : z_exp_above(mx);
-        o.ex[at] = e;
-        // the sum's own rounding (K 2^-53 relative) widens it by 2^-30
-        const double s = sum * (1.0 + 0x1p-30);
-        int l = (mx && !bad && s < 0x1p1000) ? z_exp_above((unsigned long long)__double_as_longlong(s)) : e;
-        if (!bad && s >= 0x1p1000) l = e + 19;   // more than the 2^17 elements of a row can add
-        o.la[at] = bad ? Z_BAD : max(l, e);
+        const int2 x = z_row_exps(mx, sum);
+        o.ex[at] = x.x;
+        o.la[at] = x.y;
     }
 }
 
@@ -173,16 +183,59 @@ __global__ void __launch_bounds__(1024) k_z_stats(ZOperand a, ZOperand x)
 // Digit planes.  One CTA per 64 rows and chunk; thread = row and 8 consecutive k
 // (four threads hold a row's chunk, so that they write 64 contiguous bytes).
 // XOP: the tile rows [re | -im] and [im | re] of op(B); else [re | im] of op(A).
-template <bool XOP> __device__ __forceinline__ void z_digits_rows(const ZOperand &o, int block, int kc, int b)
+// STATS: the rows' exponents are formed here, by every chunk's CTA from the whole row
+// (Z_FUSE: short rows, which then are read again from L2 by their few chunks), instead of
+// by a launch before.
+template <bool XOP, bool STATS> __device__ __forceinline__ void z_digits_rows(const ZOperand &o, int block, int kc, int b)
 {
     const int g = threadIdx.x & 3, r = block * 64 + (threadIdx.x >> 2), k0 = kc * Z_BK + 8 * g;
     if (r >= o.rp) return;
     const int t0 = r / o.tile_rows * o.tile_rows;   // first row of the tile
+    const double2 *P = o.P + b * o.sb;
+    int2 x;
+    if (STATS) {
+        // the sum in integers, 2^-30 of the largest magnitude and rounded up (the FP64 pipe would
+        // take 128 clocks an element and warp)
+        unsigned long long mx = 0, sum = 0;
+        auto each = [&](auto use) {
+            if (r < o.R)
+                for (int k = g; k < o.K; k += 16) {
+                    double2 v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        v[u] = make_double2(0, 0);
+                        if (k + 4 * u < o.K && z_in(o.tri, r, k + 4 * u)) v[u] = P[r * o.sr + (k + 4 * u) * o.sk];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        use((unsigned long long)__double_as_longlong(v[u].x) & ~(1ull << 63));
+                        use((unsigned long long)__double_as_longlong(v[u].y) & ~(1ull << 63));
+                    }
+                }
+        };
+        each([&](unsigned long long a) { mx = max(mx, a); });
+#pragma unroll
+        for (int q = 1; q < 4; q <<= 1)   // the row's four threads (o.rp is a multiple of the block's rows)
+            mx = max(mx, (unsigned long long)__shfl_xor_sync(0xffffffffu, (long long)mx, q));
+        const bool bad = mx >= (0x7FFull << 52);
+        x.x = bad ? Z_BAD : z_exp_above(mx);
+        each([&](unsigned long long a) {
+            const int E = max((int)(a >> 52), 1), sh = 23 + x.x + 1022 - E;
+            const unsigned long long m = (a & 0xFFFFFFFFFFFFFull) | ((a >> 52) ? 1ull << 52 : 0);
+            if (m) sum += (sh < 64 ? m >> sh : 0) + 1;
+        });
+#pragma unroll
+        for (int q = 1; q < 4; q <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, q);
+        x.y = bad ? Z_BAD : max(x.x, sum ? x.x - 30 + 64 - __clzll((long long)sum) : x.x);
+        if (kc == 0 && g == 0) {
+            o.ex[(long)b * o.rp + r] = x.x;
+            o.la[(long)b * o.rp + r] = x.y;
+        }
+    }
     // chunks that a triangular operand's tile never reads
     if (o.tri == 1 && kc * Z_BK >= t0 + o.tile_rows) return;
     if (o.tri == 2 && (kc + 1) * Z_BK <= t0 / Z_BK * Z_BK) return;
-    const double2 *P = o.P + b * o.sb;
-    const int e = o.ex[(long)b * o.rp + r];
+    const int e = STATS ? x.x : o.ex[(long)b * o.rp + r];
     const int p = 8 * ZD - 1 - e;
     const bool use = r < o.R && e != Z_BAD;
     uint32_t wr[ZD][4], wi[ZD][4];
@@ -232,11 +285,11 @@ template <bool XOP> __device__ __forceinline__ void z_digits_rows(const ZOperand
     }
 }
 
-__global__ void __launch_bounds__(256) k_z_digits(ZOperand a, ZOperand x)
+template <bool STATS> __global__ void __launch_bounds__(256) k_z_digits(ZOperand a, ZOperand x)
 {
     const int na = a.rp / 64, q = blockIdx.x;
-    if (q < na) z_digits_rows<false>(a, q, blockIdx.y, blockIdx.z);
-    else z_digits_rows<true>(x, q - na, blockIdx.y, blockIdx.z);
+    if (q < na) z_digits_rows<false, STATS>(a, q, blockIdx.y, blockIdx.z);
+    else z_digits_rows<true, STATS>(x, q - na, blockIdx.y, blockIdx.z);
 }
 
 // the results that leave the normal range (a call, so that its FP64-pipe
@@ -646,8 +699,13 @@ bool zgemm64_launch(cudaStream_t s, const GemmArgs<double> &g, const ZScratch &z
         x.ex = exX;
         x.la = laX;
         x.tile_rows = Z_BN;
-        NRLTB_LAUNCH(k_z_stats, dim3((a.rp + x.rp) / 32, bn), 1024, 0, s, a, x);
-        NRLTB_LAUNCH(k_z_digits, dim3((a.rp + x.rp) / 64, kc, bn), 256, 0, s, a, x);
+        const dim3 gd((a.rp + x.rp) / 64, kc, bn);
+        if (g.k <= Z_FUSE) {
+            NRLTB_LAUNCH(k_z_digits<true>, gd, 256, 0, s, a, x);
+        } else {
+            NRLTB_LAUNCH(k_z_stats, dim3((a.rp + x.rp) / 32, bn), 1024, 0, s, a, x);
+            NRLTB_LAUNCH(k_z_digits<false>, gd, 256, 0, s, a, x);
+        }
         ZProduct p = {};
         p.DA = DA;
         p.DX = DX;
