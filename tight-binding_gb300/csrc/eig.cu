@@ -731,32 +731,30 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
                 const TB dlk = Ek(b0 + k);
                 TB dnext = Dk(b0 + k + 1) - lam;
                 TB dunext = (k < len - 2) ? Ek(b0 + k + 1) : TB(0);
-                // FP64 takes a dozen operations of its narrow pipe for a quotient: one
-                // per step, 1 / pivot, which also gives the multiplier and which the
-                // later iterations read back
-                if (fabs(dcur) >= fabs(dlk)) {
-                    TB f;
-                    if (sizeof(TB) == 8) {
-                        const TB rp = it == 0 ? tri_div(TB(1), pivot(dcur)) : rgv[u];
-                        f = (dcur != TB(0)) ? dlk * rp : TB(0);
-                        if (it == 0) { RG[k] = rp; DU[k] = ducur; DU2[k] = TB(0); }
-                    } else {
-                        f = (dcur != TB(0)) ? tri_div(dlk, dcur) : TB(0);
-                        if (it == 0) { RG[k] = tri_div(TB(1), pivot(dcur)); DU[k] = ducur; DU2[k] = TB(0); }
-                    }
+                if (sizeof(TB) == 8) {
+                    // FP64 takes a dozen operations of its narrow pipe for a quotient: one
+                    // per step, 1 / pivot, which also gives the multiplier and which the
+                    // later iterations read back.  The rows are exchanged by selection, so
+                    // that a warp whose threads differ pays for one form (N = 1152, 4
+                    // matrices 3.72 -> 3.46 ms, N = 144, 15 matrices 0.43 -> 0.34)
+                    const bool sw = fabs(dcur) < fabs(dlk);
+                    const TB p = sw ? dlk : dcur, q = sw ? dcur : dlk, g1 = sw ? dnext : ducur, g2 = sw ? ducur : dnext;
+                    const TB rp = it == 0 ? tri_div(TB(1), pivot(p)) : rgv[u];
+                    const TB f = q * rp, vk = sw ? vn[u] : vc, vo = sw ? vc : vn[u];
+                    if (it == 0) { RG[k] = rp; DU[k] = g1; DU2[k] = sw ? dunext : TB(0); }
+                    dnext = g2 - f * g1;
+                    if (sw) dunext = -f * dunext;
+                    v[k] = vk;
+                    vc = vo - f * vk;
+                } else if (fabs(dcur) >= fabs(dlk)) {
+                    const TB f = (dcur != TB(0)) ? tri_div(dlk, dcur) : TB(0);
+                    if (it == 0) { RG[k] = tri_div(TB(1), pivot(dcur)); DU[k] = ducur; DU2[k] = TB(0); }
                     dnext -= f * ducur;
                     v[k] = vc;
                     vc = vn[u] - f * vc;
                 } else {
-                    TB f;
-                    if (sizeof(TB) == 8) {
-                        const TB rp = it == 0 ? tri_div(TB(1), pivot(dlk)) : rgv[u];
-                        f = dcur * rp;
-                        if (it == 0) { RG[k] = rp; DU[k] = dnext; DU2[k] = dunext; }
-                    } else {
-                        f = tri_div(dcur, dlk);
-                        if (it == 0) { RG[k] = tri_div(TB(1), pivot(dlk)); DU[k] = dnext; DU2[k] = dunext; }
-                    }
+                    const TB f = tri_div(dcur, dlk);
+                    if (it == 0) { RG[k] = tri_div(TB(1), pivot(dlk)); DU[k] = dnext; DU2[k] = dunext; }
                     dnext = ducur - f * dnext;
                     dunext = -f * dunext;
                     v[k] = vn[u];
