@@ -222,7 +222,7 @@ template <bool XOP, bool STATS> __device__ __forceinline__ void z_digits_rows(co
         each([&](unsigned long long a) {
             const int E = max((int)(a >> 52), 1), sh = 23 + x.x + 1022 - E;
             const unsigned long long m = (a & 0xFFFFFFFFFFFFFull) | ((a >> 52) ? 1ull << 52 : 0);
-            if (m) sum += (sh < 64 ? m >> sh : 0) + 1;
+            if (m) sum += ((unsigned)sh < 64u ? m >> sh : 0) + 1;
         });
 #pragma unroll
         for (int q = 1; q < 4; q <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, q);
