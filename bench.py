@@ -208,10 +208,10 @@ def run_reference(args):
 KCLASSES = [  # (class id, name, bound, unit of work, kernel name prefix in ncu)
     (0, "zgemm_umma_kernel / zgemm_tc_kernel: FP32 complex GEMM on the tensor cores (3xTF32; tcgen05 with "
         "tensor-memory accumulators for op(A) = A, mma.sync for op(A) = A^H)", "tensor", "flop", "zgemm_umma"),
-    (1, "zgemm_kernel: complex GEMM on the FMA pipe (FP64 form; FP32 shapes below the tensor-core thresholds)",
+    (1, "zgemm_kernel: complex GEMM on the FMA pipe (shapes below the tensor-core thresholds)",
      "fma", "flop", "zgemm_kernel"),
     (2, "k_oz_gemm: bf16 digit products on tcgen05 (refinement H X, S X to FP64 accuracy; Hellmann-Feynman "
-        "dH Z, dS Z from 3-digit dH, dS)", "tensor", "flop", "k_oz_gemm"),
+        "dH Z, dS Z from 3-digit dH, dS; k_z_gemm, the FP64 solves' products)", "tensor", "flop", "k_oz_gemm"),
     (3, "k_tri_panel: tridiagonalisation panel (cluster per matrix, Hermitian mat-vec)", "hbm", "byte",
      "k_tri_panel"),
 ]

@@ -63,7 +63,7 @@ int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, int k, int b
 /* Fault flags of the tcgen05 kernels: bit 0 the FP32 GEMM, bit 1 the
  * refinement's digit product, bit 2 the FP64 GEMM's; a bit is set once a bounded barrier wait inside
  * that kernel ran out (the kernel then leaves its output untouched).
- * clear = 1 resets both. */
+ * clear = 1 resets them. */
 int nrltb_bench_umma_fault(int clear);
 
 /* Raise the context's own bounded-wait expiry word, as a tcgen05 kernel of
@@ -75,12 +75,13 @@ int nrltb_bench_raise_fault_word(nrltb_ctx *ctx);
 
 /* Kernel-class timing of the context's own calls: with on = 1 every later
  * launch of a timed class (0 = FP32 tensor-core GEMM, 1 = SIMT GEMM, 2 = the
- * refinement's tensor-core digit product, 3 = the tridiagonalisation panel
- * kernel) is bracketed by CUDA events on the launching stream and tagged with
- * its algorithmic work (flops: 8 per complex multiply-add a GEMM needs, zeros
- * of triangular operands and a skipped triangle of C excluded; bytes: the
- * trailing lower triangles a panel reads).  Turning it on clears
- * the records; stats synchronizes the stream and sums one class. */
+ * tensor-core digit products, the refinement's and the FP64 GEMMs' with the
+ * making of their digits, 3 = the FP32 tridiagonalisation panel kernel) is
+ * bracketed by CUDA events on the launching stream and tagged with its
+ * algorithmic work (flops: 8 per complex multiply-add a GEMM needs, zeros of
+ * triangular operands and a skipped triangle of C excluded; bytes: the trailing
+ * lower triangles a panel reads).  Turning it on clears the records; stats
+ * synchronizes the stream and sums one class. */
 int nrltb_bench_kernel_timing(nrltb_ctx *ctx, int on);
 int nrltb_bench_kernel_stats(nrltb_ctx *ctx, int cls, double *ms, double *work, int *launches);
 
