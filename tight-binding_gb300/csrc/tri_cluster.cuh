@@ -25,9 +25,9 @@
 // of about 7 us a column (n = 128, eight CTAs: 9 us in all): two cluster barriers, and sums
 // and scalars whose operations take 64 cycles of an SM's quarter each.
 // Against two launches a column (tri_col.cuh), whole tridiagonalisations: n = 144 2.8 -> 1.5 ms
-// (4 matrices), 3.6 -> 2.2 (36), 7.1 -> 5.3 (150); by columns n = 180 takes 3.6, 5.1 and 10.8 ms,
-// here n = 192 2.3, 3.2 and 8.2; n = 288, the last 192 columns here: 6.4 -> 4.8 ms (4), 14.7 ->
-// 11.4 (64).
+// (4 matrices), 3.6 -> 1.9 (36), 7.1 -> 5.2 (150); by columns n = 180 takes 3.6, 5.1 and 10.8 ms,
+// here n = 192 2.3, 2.9 and 8.0; n = 288, the last 192 columns here: 6.4 -> 4.7 ms (4), 14.7 ->
+// 11.2 (64).
 #pragma once
 #include <cooperative_groups.h>
 #include "eig.cuh"
@@ -35,17 +35,21 @@
 
 namespace nrltb {
 
-constexpr int TK_THREADS = 256, TK_WARPS = TK_THREADS / 32;
+// 16 warps cover each other's latencies better than 8: n = 144 1.53 -> 1.46 ms with 15 matrices,
+// 2.16 -> 1.87 with 36, 2.9 -> 2.6 with 64
+constexpr int TK_THREADS = 512, TK_WARPS = TK_THREADS / 32;
 constexpr int TK_RANKS = 8;     // y is summed as by eight CTAs, whatever the cluster size
 constexpr int TK_MAX = 192;     // the largest order whose triangle two CTAs hold
 
 struct TkSizes {
     int T, ntiles, slots, np;
     __host__ __device__ TkSizes(int m, int cl) : T((m + 31) / 32), ntiles(T * (T + 1) / 2), slots((ntiles + cl - 1) / cl), np(32 * T) {}
+    // elements for the shares of y of one rank: what two CTAs' memory leaves beside the tiles
+    __host__ __device__ int part_size() const { return T <= 5 ? 640 : 256; }
     // tiles | v of two columns | w | y of each rank | shares of y | sums per warp, scalars, counters | tile numbers
     __host__ __device__ int bytes(int cl) const
     {
-        return 16 * (1024 * slots + (3 + TK_RANKS) * np + 256 * (TK_RANKS / cl)) + 8 * (TK_WARPS + 8) + 16 + 4 * slots;
+        return 16 * (1024 * slots + (3 + TK_RANKS) * np + part_size() * (TK_RANKS / cl)) + 8 * (TK_WARPS + 8) + 16 + 4 * slots;
     }
 };
 
@@ -63,7 +67,7 @@ __global__ void __launch_bounds__(TK_THREADS, 1) k_tri_cluster(EigWork<double> w
     double2 *const tiles = (double2 *)tk_raw, *const vb = tiles + 1024 * z.slots, *const wv = vb + 2 * np;
     constexpr int NR = TK_RANKS / CL;   // ranks of this CTA: rank + CL j
     double2 *const ybuf = wv + np, *const part = ybuf + TK_RANKS * np;
-    double *const red = (double *)(part + 256 * NR), *const sc = red + TK_WARPS;   // sc[4 p ..]: tau and scale of parity p
+    double *const red = (double *)(part + z.part_size() * NR), *const sc = red + TK_WARPS;   // sc[4 p ..]: tau and scale of parity p
     int *const ctr = (int *)(sc + 8);
     short2 *const tab = (short2 *)(ctr + 4);   // row and column block of each own tile
     const double2 *A = w.A + b * w.mstride + j0 * (ld + 1);
@@ -186,8 +190,8 @@ __global__ void __launch_bounds__(TK_THREADS, 1) k_tri_cluster(EigWork<double> w
         if (apply) {
             // ---- A ----
             if (tid == 0) ctr[1] = 0;
-            // (shares of a row block's columns: K rows <= 256)
-            const int nb = T - tb, rows = 32 * nb, K = nb <= 2 ? 4 : nb <= 4 ? 2 : 1, W = 32 / K;
+            // (shares of a row block's columns: K rows <= part_size)
+            const int nb = T - tb, rows = 32 * nb, K = T <= 5 ? (nb <= 2 ? 8 : 4) : nb <= 2 ? 4 : nb <= 4 ? 2 : 1, W = 32 / K;
             for (int un = grab(ctr); un < nb * K * NR; un = grab(ctr)) {
                 const int j = un % NR, k = un / NR % K, R = T - 1 - un / (NR * K), k0 = k * W, rk = rank + CL * j;
                 double2 acc = zero;
@@ -322,12 +326,12 @@ template <int CL> inline bool tk_try(cudaStream_t s, const EigWork<double> &w, i
 
 // The columns from j0 on in one launch; false if they don't fit or no cluster can be scheduled.
 // The cluster is the largest whose matrices all fit the device at once (the chain is the same,
-// the shares of the FP64 work shorter): n = 144: 1.54 ms with eight CTAs, up to 4 to 15
-// matrices, 2.15 with four, up to 36, 2.9 with two, up to 72.  Larger triangles need four CTAs
-// and more, and are faster here only while they fit in one wave (n = 288: 36 matrices 7.2 ms
-// against 10.9 by columns, 64 matrices 14.3 against 14.7); taking the last 192 columns alone
-// is as fast in the first case (8.7) and better in the second (11.4), and goes by the order
-// alone, so that a matrix has the same result in every batch.
+// the shares of the FP64 work shorter): n = 144: 1.46 ms with eight CTAs (15 matrices), 1.87 with
+// four (36), 2.6 with two (64).  Larger triangles need four CTAs and more, and were faster here
+// only while they fit in one wave (n = 288, 8 warps: 36 matrices 7.2 ms against 10.9 by columns,
+// 64 matrices 14.3 against 14.7); taking the last 192 columns alone is as fast in the first
+// case (8.3) and better in the second (11.2), and goes by the order alone, so that a matrix
+// has the same result in every batch.
 inline bool tri_cluster(cudaStream_t s, const EigWork<double> &w, int j0)
 {
     if (w.n - j0 > TK_MAX) return false;

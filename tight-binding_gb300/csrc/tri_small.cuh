@@ -17,7 +17,7 @@
 //    warps update the rest of the triangle.
 // Against two launches a column (tri_col.cuh), whole tridiagonalisations: n = 9 108 -> 43 us
 // (4 matrices), 920 -> 77 us (1728); n = 36 736 -> 186 us, n = 64 1311 -> 532 us, n = 108
-// 2586 -> 1617 us (36 matrices each), of which the FP64 pipe needs 820.
+// 2586 -> 1395 us (36 matrices each), of which the FP64 pipe needs 820.
 #pragma once
 #include "eig.cuh"
 #include "tri_col.cuh"
@@ -25,12 +25,12 @@
 namespace nrltb {
 
 // Above, a cluster (tri_cluster.cuh) is faster unless there are hundreds of matrices: n = 128
-// 2.5 ms here, 1.15 to 1.9 ms there for 1 to 64 matrices, 3.5 for 150; below, n = 108, 1.6 ms
-// against 1.1 to 1.8 and 2.3.  The rule goes by the order alone, so that a matrix has the same
+// 2.1 ms here, 1.13 to 1.7 ms there for 1 to 64 matrices, 3.4 for 150; below, n = 108, 1.4 ms
+// against 1.1 to 1.6 and 2.3.  The rule goes by the order alone, so that a matrix has the same
 // result in every batch.
 constexpr int TS_MAX = 112;
 
-inline int ts_threads(int n) { return n <= 16 ? 32 : n <= 32 ? 64 : n <= 64 ? 128 : 256; }
+inline int ts_threads(int n) { return n <= 16 ? 32 : n <= 32 ? 64 : n <= 64 ? 128 : n <= 96 ? 256 : 512; }
 // triangle | v, two columns' | w | partial y | sums per warp | scalars of two columns, counter | shares per order
 inline size_t ts_smem(int n, int nt)
 {
@@ -38,10 +38,13 @@ inline size_t ts_smem(int n, int nt)
            sizeof(int) * 2 + (size_t)n;
 }
 
-// shares of the columns for a mat-vec of order m on nt threads: the rounds of warps over
-// the four quarters times the columns of a share, and the addition of the shares
+// shares of the columns for a mat-vec of order m on nt threads: where an SM holds one matrix
+// (n > 96), as many as there are threads, for warps to cover each other's latencies (n = 108:
+// 1.61 -> 1.39 ms with 16 warps); else, with other matrices to do that, the rounds of warps
+// over the four quarters times the columns of a share, and the addition of the shares
 __device__ inline int ts_share_count(int m, int nt)
 {
+    if (nt > 256) return min(nt / m, m);
     int best = 1, cost = 1 << 30;
     for (int k = 1; k * m <= nt && k <= m; ++k) {
         const int c = 8 * ((((m * k + 31) / 32) + 3) / 4) * ((m + k - 1) / k) + 4 * k * ((m + 127) / 128);
@@ -53,7 +56,7 @@ __device__ inline int ts_share_count(int m, int nt)
     return best;
 }
 
-__global__ void __launch_bounds__(256) k_tri_small(EigWork<double> w)
+__global__ void __launch_bounds__(512) k_tri_small(EigWork<double> w)
 {
     extern __shared__ __align__(16) unsigned char ts_raw[];
     const int b = blockIdx.x, n = w.n, nt = blockDim.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
