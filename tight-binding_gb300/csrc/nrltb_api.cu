@@ -562,7 +562,7 @@ static int run_bloch_on(nrltb_ctx *c, cudaStream_t s, DBuf &phb, int k0, int nk,
                      c->d_kq.as<double>() + 3 * (long)k0, nk, phb.as<double2>());
     const long tiles = cdiv(nv, 32);
     if (nv <= 32)   // one tile
-        NRLTB_LAUNCH(k_bloch_small, cdiv((long)nv * (nv + 1) / 2 * cdiv(nk, BLOCH_K), 64), 64, 0, s, DS, DP, pr, c->npairs,
+        NRLTB_LAUNCH(k_bloch_small, cdiv((long)nv * (nv + 1) / 2 * nk, 64), 64, 0, s, DS, DP, pr, c->npairs,
                      sk, c->d_seg.as<int2>(), c->d_orb.as<int>(), c->d_ksk.as<int>(), phb.as<double2>(), nk, nv, which0, M1,
                      M2, S.jsover);
     else

@@ -689,62 +689,52 @@ k_bloch_build(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, co
 }
 
 // The same for matrices of one tile (nv <= 32): a thread per element on or above the
-// diagonal and group of BLOCH_K k, dealt over all groups without gaps; the tile kernel
-// would fill 9 lanes of 32 at nv = 9 and form every element of its diagonal tile.  The
-// same sums.  Bound: the FP64 pipe (one atom, 1728 k: about 100 us).  Small CTAs, since a warp or
-// two per quarter of an SM have to keep it busy.  One atom, 1728 k: 923 -> 172 us a call;
-// 8 sp3 atoms (nv = 32), 125 k: 174 -> 33.
+// diagonal and k, dealt over all k without gaps; the tile kernel would fill 9 lanes of 32
+// at nv = 9 and form every element of its diagonal tile.  The same sums.  Bound: the FP64
+// pipe (one atom, 1728 k: about 110 us), which needs many warps: with four k to a thread,
+// as in the tile kernel, 172 us, with two 133.  Against the tile kernel: one atom, 1728 k
+// 923 -> 121 us a call; 8 sp3 atoms (nv = 32), 125 k 174 -> 30.
 __global__ void __launch_bounds__(64)
 k_bloch_small(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, const int2 *seg,
               const int *orb_atom, const int *ksk, const double2 *ph, int nk, int nv, int which0,
               double2 *M1, double2 *M2, int jsover)
 {
-    const int ne = nv * (nv + 1) / 2, groups = (nk + BLOCH_K - 1) / BLOCH_K;
+    const int ne = nv * (nv + 1) / 2;
     const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const int kg = (int)(t / ne), e = (int)(t - (long)kg * ne);
-    if (kg >= groups) return;
+    const int kk = (int)(t / ne), e = (int)(t - (long)kk * ne);
+    if (kk >= nk) return;
     int c = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);   // e = c (c + 1) / 2 + r, r <= c
     while ((c + 1) * (c + 2) / 2 <= e) ++c;
     while (c * (c + 1) / 2 > e) --c;
-    const int r = e - c * (c + 1) / 2, kk0 = kg * BLOCH_K, kn = min(BLOCH_K, nk - kk0);
+    const int r = e - c * (c + 1) / 2;
     int a1, a2, oi, oj;
     bool conjg;   // false: r <= c
     int2 sg;
     double on1, on2;
     bloch_elem(S, sk, npairs, seg, orb_atom, ksk, r, c, which0, a1, a2, oi, oj, conjg, sg, on1, on2);
     const double *E1 = sk.E + (long)which0 * npairs * 81 + oi * 9 + oj, *E2 = E1 + (long)npairs * 81;
-    const double2 *phk = ph + kk0;
-    double2 h[BLOCH_K], s[BLOCH_K];
-#pragma unroll
-    for (int kk = 0; kk < BLOCH_K; ++kk) h[kk] = s[kk] = make_double2(0, 0);
-#pragma unroll 2
+    double2 h = make_double2(0, 0), s = h;
+#pragma unroll 4
     for (int p = sg.x; p < sg.y; ++p) {
         const double e1 = E1[(long)p * 81], e2 = jsover ? E2[(long)p * 81] : 0.0;
-#pragma unroll
-        for (int kk = 0; kk < BLOCH_K; ++kk) {
-            const double2 z = phk[(long)p * nk + (kk < kn ? kk : 0)];
-            h[kk].x += e1 * z.x;
-            h[kk].y += e1 * z.y;
-            if (jsover) {
-                s[kk].x += e2 * z.x;
-                s[kk].y += e2 * z.y;
-            }
+        const double2 z = ph[(long)p * nk + kk];
+        h.x += e1 * z.x;
+        h.y += e1 * z.y;
+        if (jsover) {
+            s.x += e2 * z.x;
+            s.y += e2 * z.y;
         }
     }
     const long nn = (long)nv * nv;
-#pragma unroll
-    for (int kk = 0; kk < BLOCH_K; ++kk) {
-        if (kk >= kn) break;
-        double2 *m1 = M1 + (kk0 + kk) * nn, *m2 = M2 + (kk0 + kk) * nn;
-        h[kk].x += on1;
-        if (jsover) s[kk].x += on2;
-        else s[kk].x = (r == c && which0 == 0) ? 1.0 : 0.0;
-        m1[r + c * nv] = h[kk];
-        m2[r + c * nv] = s[kk];
-        if (r != c) {
-            m1[c + r * nv] = make_double2(h[kk].x, -h[kk].y);
-            m2[c + r * nv] = make_double2(s[kk].x, -s[kk].y);
-        }
+    double2 *m1 = M1 + kk * nn, *m2 = M2 + kk * nn;
+    h.x += on1;
+    if (jsover) s.x += on2;
+    else s.x = (r == c && which0 == 0) ? 1.0 : 0.0;
+    m1[r + c * nv] = h;
+    m2[r + c * nv] = s;
+    if (r != c) {
+        m1[c + r * nv] = make_double2(h.x, -h.y);
+        m2[c + r * nv] = make_double2(s.x, -s.y);
     }
 }
 

@@ -79,7 +79,7 @@ __global__ void k_bloch_build(DevStructure S, DevParams P, DevPairs pr, int npai
 __global__ void k_bloch_small(DevStructure S, DevParams P, DevPairs pr, int npairs, DevSK sk, const int2 *seg,
                               const int *orb_atom, const int *ksk, const double2 *ph, int nk, int nv, int which0,
                               double2 *M1, double2 *M2, int jsover);
-constexpr int BLOCH_K = 4;   // k points per CTA of k_bloch_build (grid = tile pairs x cdiv(nk, BLOCH_K)), per thread of k_bloch_small
+constexpr int BLOCH_K = 4;   // k points per CTA of k_bloch_build: grid = tile pairs x cdiv(nk, BLOCH_K)
 
 constexpr int SEARCH_BLOCK = 1024;
 
