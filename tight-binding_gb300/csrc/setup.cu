@@ -351,30 +351,47 @@ __global__ void k_setpar_atoms(DevStructure S, DevParams P, DevPairs pr, int npa
     const int a = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (a >= S.natoms) return;   // warp-uniform
     const int kinds = P.kinds;
-    double den[NRLTB_MAX_KINDS], vden[NRLTB_MAX_KINDS];
-    for (int k = 0; k < kinds; ++k) { den[k] = 0; vden[k] = 0; }
+    // lane 2 (k - 1) sums kind k's terms of the density, the next lane those of its derivative,
+    // both in pair order: one FP64 addition a pair, whose latency is the bound (a one-atom
+    // cell's 226 pairs: 46 us with every lane adding both, 25 here)
+    __shared__ double2 term[8][32];
+    __shared__ int kind[8][32];
+    const int wb = threadIdx.x >> 5;
+    double acc = 0;
     for (int p0 = 0; p0 < npairs; p0 += 32) {
         const int p = p0 + lane;
-        int iat = -1, jat = -1, kk = 0;
-        double d1 = 0, v1 = 0;
-        bool m1 = false, m2 = false;
+        int kk = 0;
+        double2 t = make_double2(0, 0);
+        bool hit = false;
         if (p < npairs) {
-            iat = pr.jatm[2 * p] - 1;
-            jat = pr.jatm[2 * p + 1] - 1;
-            m1 = iat == a;
-            m2 = jat == a && iat != a;
-            if (m1) { kk = pr.jkind[2 * p + 1]; d1 = sk.dent[2 * (long)p]; v1 = sk.vdent[2 * (long)p]; }
-            else if (m2) { kk = pr.jkind[2 * p]; d1 = sk.dent[2 * (long)p + 1]; v1 = sk.vdent[2 * (long)p + 1]; }
+            const int iat = pr.jatm[2 * p] - 1, jat = pr.jatm[2 * p + 1] - 1;
+            const int end = iat == a ? 0 : 1;
+            hit = iat == a || jat == a;
+            if (hit) {
+                kk = pr.jkind[2 * p + 1 - end];
+                t = make_double2(sk.dent[2 * (long)p + end], sk.vdent[2 * (long)p + end]);
+            }
         }
-        unsigned hits = __ballot_sync(0xffffffffu, m1 || m2);
-        while (hits) {   // in pair order
-            const int l = __ffs(hits) - 1;
-            hits &= hits - 1;
-            const int k = __shfl_sync(0xffffffffu, kk, l);
-            const double d = __shfl_sync(0xffffffffu, d1, l), v = __shfl_sync(0xffffffffu, v1, l);
-            den[k - 1] += d;
-            vden[k - 1] += v;
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        if (hits == 0) continue;
+        if (hit) {
+            const int at = __popc(hits & ((1u << lane) - 1));
+            term[wb][at] = t;
+            kind[wb][at] = kk;
         }
+        __syncwarp();
+        const int n = __popc(hits);
+#pragma unroll 4
+        for (int l = 0; l < n; ++l) {
+            const double2 x = term[wb][l];
+            if (kind[wb][l] - 1 == lane >> 1) acc += lane & 1 ? x.y : x.x;
+        }
+        __syncwarp();
+    }
+    double den[NRLTB_MAX_KINDS], vden[NRLTB_MAX_KINDS];
+    for (int k = 0; k < kinds; ++k) {
+        den[k] = __shfl_sync(0xffffffffu, acc, 2 * k);
+        vden[k] = __shfl_sync(0xffffffffu, acc, 2 * k + 1);
     }
     if (lane != 0) return;
     const double *Pm = atom_params(S, P, a);   // on-site terms from the atom's own spin set
