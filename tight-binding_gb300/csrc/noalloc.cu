@@ -144,7 +144,7 @@ extern "C" int nrltb_search2_noalloc(int device, void *stream, int natoms, const
     }
     const int G = search_groups(natoms, box);
     k_search_eval<<<cdiv(G * box, 256), 256, 0, s>>>(S, P, (int)box, G, code, misc, dmin);
-    k_search_ties<<<1, 1, 0, s>>>(code, ncand, kneigh_in, misc, misc + 2);
+    k_search_ties<<<1, 32, 0, s>>>(code, ncand, kneigh_in, misc, misc + 2);
     k_search_count<<<nblk, SEARCH_BLOCK, 0, s>>>(code, ncand, blk);
     k_scan_small<<<1, 1024, 0, s>>>(blk, nblk, misc + 1);
     if (cudaMemcpyAsync(host_misc, misc, sizeof host_misc, cudaMemcpyDeviceToHost, s) != cudaSuccess ||

@@ -414,7 +414,7 @@ static int run_search2(nrltb_ctx *c, int kneigh_in)
     const int G = search_groups(S.natoms, box);
     NRLTB_LAUNCH(k_search_eval, cdiv(G * box, 256), 256, 0, s, DS, DP, (int)box, G, c->d_code.as<unsigned char>(), misc,
                  dmin);
-    NRLTB_LAUNCH(k_search_ties, 1, 1, 0, s, c->d_code.as<unsigned char>(), ncand, kneigh_in, misc, misc + 2);
+    NRLTB_LAUNCH(k_search_ties, 1, 32, 0, s, c->d_code.as<unsigned char>(), ncand, kneigh_in, misc, misc + 2);
     NRLTB_LAUNCH(k_search_count, nblk, SEARCH_BLOCK, 0, s, c->d_code.as<unsigned char>(), ncand, c->d_blk.as<int>());
     NRLTB_LAUNCH(k_scan_small, 1, 1024, 0, s, c->d_blk.as<int>(), nblk, misc + 1);
     CKL();

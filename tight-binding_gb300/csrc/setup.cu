@@ -132,12 +132,15 @@ k_search_eval(DevStructure S, DevParams P, int box, int G, unsigned char *code, 
 
 // Ties (dd == dnnsq exactly) take search2's carried kneigh flag: resolved in
 // candidate order by one thread, only when any tie exists.  Also returns the
-// final flag.
+// final flag, that of the last candidate that sets it: one warp looks for it from
+// the end, 128 candidates at a time (a thread by itself: 21 us for a one-atom cell,
+// whose last images are all out of reach).
 __global__ void k_search_ties(unsigned char *code, long ncand, int kneigh_in, const int *tie_count, int *kneigh_out)
 {
-    if (threadIdx.x || blockIdx.x) return;
+    const int lane = threadIdx.x;
     int kn = kneigh_in;
     if (*tie_count > 0) {
+        if (lane) return;
         for (long c = 0; c < ncand; ++c) {
             unsigned char cd = code[c];
             if (cd == 0) kn = 0;
@@ -145,12 +148,26 @@ __global__ void k_search_ties(unsigned char *code, long ncand, int kneigh_in, co
             else if (cd == 3) code[c] = kn ? 1 : 2;
         }
     } else {
-        for (long c = ncand - 1; c >= 0; --c) {
-            unsigned char cd = code[c];
-            if (cd == 0 || cd == 1) { kn = cd; break; }
+        for (long end = ncand; end > 0; end -= 128) {
+            unsigned char cd[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {   // candidates end - 1 - lane - 32 u
+                const long c = end - 1 - lane - 32 * u;
+                cd[u] = c >= 0 ? code[c] : 2;
+            }
+            bool found = false;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned m = __ballot_sync(0xffffffffu, cd[u] < 2);
+                if (m && !found) {
+                    kn = __shfl_sync(0xffffffffu, (int)cd[u], __ffs(m) - 1);
+                    found = true;
+                }
+            }
+            if (found) break;
         }
     }
-    *kneigh_out = kn;
+    if (lane == 0) *kneigh_out = kn;
 }
 
 // Order-preserving compaction: per-block counts, scan, scatter.
