@@ -72,46 +72,63 @@ __device__ __forceinline__ int count_below(const double *e, int m, double x)
 // CTAs' compensated partials are merged in rank order by every CTA, which all take
 // the same step; one cluster barrier per step, the slots alternate.
 // One CTA of 1024 threads took 0.71 ms for 27 rows of 1152 states and 5.3 ms for 1728
-// rows of 9; this 0.10 and 0.22 (0.33 before the short rows' window states were gathered).
+// rows of 9; this 0.09 and 0.16.
 constexpr int FERMI_CL = 8, FERMI_THREADS = 128, FERMI_ROW_MIN = 64;
 constexpr int FERMI_WARPS = FERMI_CL * FERMI_THREADS / 32;
 
 struct FermiSlot { double v[6]; };
 
-// the CTA's two sums into its slot; the cluster's totals to every thread
+// The CTA's two sums into its slot; the cluster's totals to every thread.  A merge is eight
+// dependent FP64 operations, so the two sums are merged side by side, one by each half of a
+// warp, in trees over lanes, warps and CTAs: 8 merges one after another where both sums in
+// every lane and lists over warps and CTAs took 34 (1728 rows of 9 states 0.22 -> 0.16 ms,
+// 12 atoms on a band path 0.10 -> 0.08; 27 rows of 1152 a call 0.206 -> 0.187).
 __device__ __forceinline__ void fermi_totals(cooperative_groups::cluster_group &cl, DD a, DD c, FermiSlot *slot,
                                              double (*sh)[FERMI_THREADS / 32], double &ta, double &tc)
 {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) {
-        const double ah = __shfl_xor_sync(0xffffffffu, a.hi, o), al = __shfl_xor_sync(0xffffffffu, a.lo, o);
-        const double ch = __shfl_xor_sync(0xffffffffu, c.hi, o), c2 = __shfl_xor_sync(0xffffffffu, c.lo, o);
-        a.merge(ah, al);
-        c.merge(ch, c2);
+    constexpr int W = FERMI_THREADS / 32;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, l = lane & 15, at = lane & 16 ? 2 : 0;
+    DD t = at ? c : a;   // lanes below 16: a, the others c
+    auto tree = [&](int from) {
+        for (int o = from; o > 0; o >>= 1) {
+            const double h = __shfl_xor_sync(0xffffffffu, t.hi, o), b = __shfl_xor_sync(0xffffffffu, t.lo, o);
+            t.merge(h, b);
+        }
+    };
+    {
+        const DD other = at ? a : c;
+        const double h = __shfl_xor_sync(0xffffffffu, other.hi, 16), b = __shfl_xor_sync(0xffffffffu, other.lo, 16);
+        t.merge(h, b);
     }
-    if (lane == 0) {
-        sh[0][wid] = a.hi; sh[1][wid] = a.lo;
-        sh[2][wid] = c.hi; sh[3][wid] = c.lo;
+    tree(8);
+    if (l == 0) {
+        sh[at][wid] = t.hi;
+        sh[at + 1][wid] = t.lo;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        DD x, y;
-        for (int q = 0; q < FERMI_THREADS / 32; ++q) {
-            x.merge(sh[0][q], sh[1][q]);
-            y.merge(sh[2][q], sh[3][q]);
+    if (wid == 0) {
+        t = DD();
+        if (l < W) {
+            t.hi = sh[at][l];
+            t.lo = sh[at + 1][l];
         }
-        slot->v[0] = x.hi; slot->v[1] = x.lo;
-        slot->v[2] = y.hi; slot->v[3] = y.lo;
+        tree(W / 2);
+        if (l == 0) {
+            slot->v[at] = t.hi;
+            slot->v[at + 1] = t.lo;
+        }
     }
     cl.sync();
-    DD x, y;
-    for (int q = 0; q < FERMI_CL; ++q) {
-        const FermiSlot *o = cl.map_shared_rank(slot, q);
-        x.merge(o->v[0], o->v[1]);
-        y.merge(o->v[2], o->v[3]);
+    t = DD();
+    if (l < FERMI_CL) {
+        const FermiSlot *o = cl.map_shared_rank(slot, l);
+        t.hi = o->v[at];
+        t.lo = o->v[at + 1];
     }
-    ta = x.hi + x.lo;
-    tc = y.hi + y.lo;
+    tree(FERMI_CL / 2);
+    const double total = t.hi + t.lo;
+    ta = __shfl_sync(0xffffffffu, total, 0);
+    tc = __shfl_sync(0xffffffffu, total, 16);
 }
 
 __global__ void __cluster_dims__(FERMI_CL, 1, 1) __launch_bounds__(FERMI_THREADS) k_fermi_level(FermiJob *jobs)
