@@ -72,7 +72,7 @@ __device__ __forceinline__ int count_below(const double *e, int m, double x)
 // CTAs' compensated partials are merged in rank order by every CTA, which all take
 // the same step; one cluster barrier per step, the slots alternate.
 // One CTA of 1024 threads took 0.71 ms for 27 rows of 1152 states and 5.3 ms for 1728
-// rows of 9; this 0.09 and 0.16.
+// rows of 9; this 0.13 and 0.16.
 constexpr int FERMI_CL = 8, FERMI_THREADS = 128, FERMI_ROW_MIN = 64;
 constexpr int FERMI_WARPS = FERMI_CL * FERMI_THREADS / 32;
 
@@ -80,7 +80,7 @@ struct FermiSlot { double v[6]; };
 
 // The CTA's two sums into its slot; the cluster's totals to every thread.  A merge is eight
 // dependent FP64 operations, so the two sums are merged side by side, one by each half of a
-// warp, in trees over lanes, warps and CTAs: 8 merges one after another where both sums in
+// warp, in trees over lanes, warps and CTAs: 10 merges one after another where both sums in
 // every lane and lists over warps and CTAs took 34 (1728 rows of 9 states 0.22 -> 0.16 ms,
 // 12 atoms on a band path 0.10 -> 0.08; 27 rows of 1152 a call 0.206 -> 0.187).
 __device__ __forceinline__ void fermi_totals(cooperative_groups::cluster_group &cl, DD a, DD c, FermiSlot *slot,
