@@ -545,8 +545,9 @@ static int run_skblocks(nrltb_ctx *c, int nwhich)
     return NRLTB_OK;
 }
 
-// dense matrices of k points [k0, k0+nk) into H, S (which0 0: H/S, 2: dH/dS)
-static int run_bloch_on(nrltb_ctx *c, cudaStream_t s, DBuf &phb, int k0, int nk, int which0, double2 *M1,
+// dense matrices of k points [k0, k0+nk) into H, S (which0 0: H/S, 2: dH/dS).  phased: the
+// phases of these k are in phb already, from the H/S sums of the same chunk on this stream
+static int run_bloch_on(nrltb_ctx *c, cudaStream_t s, DBuf &phb, bool phased, int k0, int nk, int which0, double2 *M1,
                         double2 *M2)
 {
     NvtxRange nv_(which0 ? "Bloch sums dH dS" : "Bloch sums H S");
@@ -557,7 +558,7 @@ static int run_bloch_on(nrltb_ctx *c, cudaStream_t s, DBuf &phb, int k0, int nk,
     DevPairs pr = pairs_view(c, P);
     DevStructure DS = dev_structure(c);
     DevParams DP = dev_params(c);
-    if (c->npairs > 0)
+    if (c->npairs > 0 && !phased)
         NRLTB_LAUNCH(k_phases, cdiv((long)c->npairs * nk, 256), 256, 0, s, DS, pr, c->npairs,
                      c->d_kq.as<double>() + 3 * (long)k0, nk, phb.as<double2>());
     const long tiles = cdiv(nv, 32);
@@ -573,9 +574,9 @@ static int run_bloch_on(nrltb_ctx *c, cudaStream_t s, DBuf &phb, int k0, int nk,
     return NRLTB_OK;
 }
 
-static int run_bloch(nrltb_ctx *c, int k0, int nk, int which0, double2 *M1, double2 *M2)
+static int run_bloch(nrltb_ctx *c, int k0, int nk, int which0, double2 *M1, double2 *M2, bool phased = false)
 {
-    return run_bloch_on(c, c->stream, c->d_ph, k0, nk, which0, M1, M2);
+    return run_bloch_on(c, c->stream, c->d_ph, phased, k0, nk, which0, M1, M2);
 }
 
 // The FP64 eigenvectors sit after the FP32 staging area of d_X, at a 256-byte
@@ -863,7 +864,7 @@ static int run_all(nrltb_ctx *c)
                     pre[0] = ozaki_prepare_a(sd, c->d_H.as<double2>(), nv, nkc, 6, oa);
                     pre[1] = ozaki_prepare_a(sd, c->d_S.as<double2>(), nv, nkc, 6, oa + oa6);
                     if (lpress) {
-                        RET(run_bloch_on(c, sd, c->d_ph2, k0, nkc, 2, c->d_dH.as<double2>(), c->d_dS.as<double2>()));
+                        RET(run_bloch_on(c, sd, c->d_ph2, false, k0, nkc, 2, c->d_dH.as<double2>(), c->d_dS.as<double2>()));
                         pre[2] = ozaki_prepare_a(sd, c->d_dH.as<double2>(), nv, nkc, 3, oa + 2 * oa6);
                         pre[3] = ozaki_prepare_a(sd, c->d_dS.as<double2>(), nv, nkc, 3, oa + 2 * oa6 + oa3);
                     }
@@ -905,10 +906,10 @@ static int run_all(nrltb_ctx *c)
                 if (lpress) {
                     NvtxRange nv_("Hellmann-Feynman");
                     if (S.noncol) {
-                        if ((rc = run_bloch(c, k0, nkc, 2, Hn, Sn))) break;
+                        if ((rc = run_bloch(c, k0, nkc, 2, Hn, Sn, true))) break;
                         if ((rc = run_noncol_expand(c, nkc, Hn, Sn, true))) break;
                     } else if (!overlap &&
-                               (rc = run_bloch(c, k0, nkc, 2, c->d_H.as<double2>(), c->d_S.as<double2>()))) {
+                               (rc = run_bloch(c, k0, nkc, 2, c->d_H.as<double2>(), c->d_S.as<double2>(), true))) {
                         break;
                     }
                     if ((rc = c->d_hf.ensure(hf_scratch_bytes(nv, nkc)))) break;
