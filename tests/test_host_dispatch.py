@@ -1,0 +1,86 @@
+"""The library's host code against a stand-in for the CUDA runtime (fake_cudart.c): refused launches, limits and
+allocations, a second device.  Each case runs in a process of its own, since limits and capacities are kept
+for the process."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import REPO
+
+# (kernels go by a part of their mangled names)
+PRELUDE = """
+import ctypes as C, sys
+import numpy as np
+from nrltb import abi
+lib = abi._bind(sys.argv[1], abi.GPU_SYMBOLS)
+for f in ("fake_runs", "fake_refused"):
+    getattr(lib, f).argtypes = [C.c_char_p, C.c_int]
+for f in ("fake_refuse_launch", "fake_refuse_limit", "fake_refuse_cluster"):
+    getattr(lib, f).argtypes = [C.c_char_p]
+for f in ("fake_free_bytes", "fake_alloc_limit"):
+    getattr(lib, f).argtypes = [C.c_size_t]
+lib.fake_largest_alloc.restype = C.c_size_t
+
+def context(device=0):
+    h = C.c_void_p()
+    assert lib.nrltb_ctx_create(C.byref(h), device) == 0
+    return h
+
+def diag(h, n, nk, vectors, precision=abi.PREC_FP64):
+    H = np.tile(np.eye(n, dtype=complex), (nk, 1, 1))
+    e, z = np.zeros((nk, n)), np.zeros((nk, n, n), complex)
+    p = lambda a: a.ctypes.data_as(abi._dp)
+    return lib.nrltb_diag(h, n, nk, p(H), p(H), precision, p(e), p(z) if vectors else None, None)
+"""
+
+
+@pytest.fixture(scope="session")
+def fake_lib(tmp_path_factory):
+    """The library's objects linked against the stand-in."""
+    from nrltb import build
+    build.build_all()
+    cuda = os.path.dirname(os.path.dirname(build._nvcc()))
+    out = tmp_path_factory.mktemp("fake")
+    subprocess.run(["gcc", "-O1", "-fPIC", "-Wall", "-I", os.path.join(cuda, "include"), "-c",
+                    os.path.join(REPO, "tests", "fake_cudart.c"), "-o", str(out / "fake.o")], check=True)
+    objs = [os.path.join(build.OBJ, f[:-3] + ".o") for f in build.CU_SOURCES]
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", str(out / "lib.so"), str(out / "fake.o")] + objs +
+                   ["-lpthread", "-ldl"], check=True)
+    return str(out / "lib.so")
+
+
+def _run(lib, code):
+    env = dict(os.environ, PYTHONPATH=os.path.join(REPO, "tight-binding_gb300"))
+    r = subprocess.run([sys.executable, "-c", PRELUDE + code, lib], env=env, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("n", [160, 300])
+@pytest.mark.parametrize("kernel", ["k_to_unit", "k_potrf_diag64", "k_z_gemm"])
+@pytest.mark.parametrize("clusters", [1000, 3])
+def test_refused_launch_before_the_clusters_is_reported(fake_lib, n, kernel, clusters):
+    """FP64 eigenvalues alone: a launch refused in the reduction is an error of the call, whether or not the choice of
+    a cluster size, which follows it, finds room for the batch (1000 clusters, 3)."""
+    _run(fake_lib, f"""
+h = context()
+lib.fake_clusters({clusters})
+lib.fake_refuse_launch(b"{kernel}")
+assert diag(h, {n}, 20, False) == abi.NRLTB_E_CUDA
+assert lib.fake_refused(b"{kernel}", 0) > 0
+lib.fake_refuse_launch(b"")
+assert diag(h, {n}, 20, False) == 0
+""")
+
+
+@pytest.mark.parametrize("how", ["fake_refuse_limit", "fake_refuse_cluster", "fake_refuse_launch"])
+def test_refused_clusters_leave_the_columns(fake_lib, how):
+    """Where no cluster can be had the columns take over, and the refusals are no error of the call."""
+    _run(fake_lib, f"""
+h = context()
+lib.{how}(b"13k_tri_cluster")
+assert diag(h, 160, 20, True) == 0
+assert lib.fake_runs(b"13k_tri_cluster", 0) == (1 if {how!r} == "fake_refuse_cluster" else 0)
+assert lib.fake_runs(b"k_tri_mv", 0) == (0 if {how!r} == "fake_refuse_cluster" else 159)
+""")

@@ -215,6 +215,14 @@ inline cudaError_t smem_attr_at_least(const void *func, int bytes)
     return e;
 }
 
+// Runtime calls that may be refused because another route follows.  clear() takes back
+// the error that such a refusal left, unless one of an earlier call was pending when
+// this was made: that one stays for the check at the end of the library's call.
+struct Refusable {
+    const bool pending = cudaPeekAtLastError() != cudaSuccess;
+    void clear() const { if (!pending) cudaGetLastError(); }
+};
+
 struct KTimer {
     bool on = false;
     struct Rec { int cls; cudaEvent_t a, b; double work; };

@@ -293,8 +293,9 @@ template <int CL> inline bool tk_try(cudaStream_t s, const EigWork<double> &w, i
     const TkSizes z(w.n - j0, CL);
     const int smem = z.bytes(CL);
     const void *f = (const void *)k_tri_cluster<CL>;
+    const Refusable r;   // another size, or the column kernels, take over
     if (smem_attr_at_least(f, smem) != cudaSuccess) {
-        cudaGetLastError();   // not sticky, here and below: another size, or the column kernels, take over
+        r.clear();
         return false;
     }
     cudaLaunchConfig_t cfg = {};
@@ -311,13 +312,14 @@ template <int CL> inline bool tk_try(cudaStream_t s, const EigWork<double> &w, i
     cfg.numAttrs = 1;
     if (must_fit) {
         int count = 0;
-        if (cudaOccupancyMaxActiveClusters(&count, k_tri_cluster<CL>, &cfg) != cudaSuccess || count < w.batch) {
-            cudaGetLastError();
+        if (cudaOccupancyMaxActiveClusters(&count, k_tri_cluster<CL>, &cfg) != cudaSuccess) {
+            r.clear();
             return false;
         }
+        if (count < w.batch) return false;
     }
     if (cudaLaunchKernelEx(&cfg, k_tri_cluster<CL>, w, j0) != cudaSuccess) {
-        cudaGetLastError();
+        r.clear();
         return false;
     }
     if (g_launch_counter) ++*g_launch_counter;
