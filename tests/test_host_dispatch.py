@@ -84,3 +84,26 @@ assert diag(h, 160, 20, True) == 0
 assert lib.fake_runs(b"13k_tri_cluster", 0) == (1 if {how!r} == "fake_refuse_cluster" else 0)
 assert lib.fake_runs(b"k_tri_mv", 0) == (0 if {how!r} == "fake_refuse_cluster" else 159)
 """)
+
+
+@pytest.mark.parametrize("kernel", ["k_convert_h", "12k_potrf_diag"])
+@pytest.mark.parametrize("clusters", [1000, 3, 0])
+def test_refused_launch_before_the_panels_is_reported(fake_lib, kernel, clusters):
+    """The same for the mixed form, whose first panel asks the device for its cluster capacities."""
+    _run(fake_lib, f"""
+h = context()
+lib.fake_clusters({clusters})
+lib.fake_refuse_launch(b"{kernel}")
+assert diag(h, 160, 20, True, abi.PREC_MIXED) == abi.NRLTB_E_CUDA
+assert lib.fake_refused(b"{kernel}", 0) > 0
+""")
+
+
+@pytest.mark.parametrize("how", ["fake_refuse_limit", "fake_refuse_cluster", "fake_refuse_launch"])
+def test_refused_panels_leave_the_columns(fake_lib, how):
+    _run(fake_lib, f"""
+h = context()
+lib.{how}(b"11k_tri_panel")
+assert diag(h, 160, 20, True, abi.PREC_MIXED) == 0
+assert lib.fake_runs(b"11k_tri_panel", 0) == 0 and lib.fake_runs(b"8k_tri_mv", 0) == 159
+""")

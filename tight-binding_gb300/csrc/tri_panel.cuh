@@ -533,13 +533,14 @@ template <int CL, int NW> inline int tp_capacity(size_t smem)
     if (it != known.end()) return it->second;
     int count = 0;
     const void *f = (const void *)k_tri_panel<float, CL, NW>;
+    const Refusable r;   // another size, or the column kernels, take over
     bool ok = smem_attr_at_least(f, (int)smem) == cudaSuccess;
     if (ok) {
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = tp_config<CL, NW>(&attr, 1, smem);
         ok = cudaOccupancyMaxActiveClusters(&count, k_tri_panel<float, CL, NW>, &cfg) == cudaSuccess;
     }
-    cudaGetLastError();   // not sticky: another size, or the column kernels, take over
+    if (!ok) r.clear();
     return known[std::make_pair(dev, smem)] = ok ? count : 0;
 }
 
@@ -551,8 +552,9 @@ template <int CL, int NW> inline bool tp_try(cudaStream_t s, const EigWork<float
     cudaLaunchConfig_t cfg = tp_config<CL, NW>(&attr, w.batch, smem);
     cfg.stream = s;
     cudaEvent_t ev = kt_begin(s);
+    const Refusable r;
     if (cudaLaunchKernelEx(&cfg, k_tri_panel<float, CL, NW>, w, j0, jb) != cudaSuccess) {
-        cudaGetLastError();
+        r.clear();
         return false;
     }
     if (g_launch_counter) ++*g_launch_counter;
