@@ -107,3 +107,26 @@ lib.{how}(b"11k_tri_panel")
 assert diag(h, 160, 20, True, abi.PREC_MIXED) == 0
 assert lib.fake_runs(b"11k_tri_panel", 0) == 0 and lib.fake_runs(b"8k_tri_mv", 0) == 159
 """)
+
+
+@pytest.mark.parametrize("n", [20, 160])
+def test_fp64_products_on_a_second_device(fake_lib, n):
+    """A kernel's shared-memory limit belongs to one device: contexts on two devices of a process launch alike."""
+    _run(fake_lib, f"""
+runs = []
+for dev in (0, 1):
+    h = context(dev)
+    assert diag(h, {n}, 3, True) == 0
+    runs.append([lib.fake_runs(b"8k_z_gemm", dev), lib.fake_runs(b"k_", dev)])
+    assert runs[-1][0] > 0 and lib.fake_refused(b"k_", dev) == 0
+assert runs[0] == runs[1]
+""")
+
+
+def test_fp64_products_without_their_limit_take_the_fma_pipe(fake_lib):
+    _run(fake_lib, """
+h = context()
+lib.fake_refuse_limit(b"8k_z_gemm")
+assert diag(h, 160, 3, True) == 0
+assert lib.fake_runs(b"8k_z_gemm", 0) == 0 and lib.fake_runs(b"zgemm_kernel", 0) > 0
+""")

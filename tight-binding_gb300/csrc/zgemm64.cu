@@ -656,11 +656,11 @@ bool zgemm64_launch(cudaStream_t s, const GemmArgs<double> &g, const ZScratch &z
     const size_t per = z_bytes_per_matrix(g.m, g.n, g.k);
     if (!zs.p || zs.bytes < per + 4 * 256) return false;
     const int nb = (int)std::min<size_t>(g.batch, (zs.bytes - 4 * 256) / per);
-    static const bool attr = [] {
-        cudaFuncSetAttribute(k_z_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, Z_SMEM);
-        return true;
-    }();
-    (void)attr;
+    const Refusable r;   // the FMA-pipe kernel takes over
+    if (smem_attr_at_least((const void *)k_z_gemm, Z_SMEM) != cudaSuccess) {
+        r.clear();
+        return false;
+    }
     const int mt = cdiv(g.m, Z_BM), nt = cdiv(g.n, Z_BN), kc = cdiv(g.k, Z_BK);
     unsigned char *base = (unsigned char *)zs.p;
     unsigned char *DA = base, *DX = DA + (size_t)nb * mt * kc * ZD * Z_TILE;
