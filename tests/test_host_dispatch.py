@@ -130,3 +130,15 @@ lib.fake_refuse_limit(b"8k_z_gemm")
 assert diag(h, 160, 3, True) == 0
 assert lib.fake_runs(b"8k_z_gemm", 0) == 0 and lib.fake_runs(b"zgemm_kernel", 0) > 0
 """)
+
+
+def test_mixed_form_on_a_second_device(fake_lib):
+    _run(fake_lib, """
+runs = []
+for dev in (0, 1):
+    h = context(dev)
+    assert diag(h, 160, 3, True, abi.PREC_MIXED) == 0
+    runs.append([lib.fake_runs(k, dev) for k in (b"k_oz_gemm", b"zgemm_umma_kernel", b"k_ref_band", b"k_")])
+    assert min(runs[-1]) > 0 and lib.fake_refused(b"k_", dev) + lib.fake_refused(b"zgemm", dev) == 0
+assert runs[0] == runs[1]
+""")

@@ -388,12 +388,7 @@ bool zgemm_umma_supported(const GemmArgs<float> &g)
 
 void zgemm_umma_launch(cudaStream_t s, const GemmArgs<float> &g)
 {
-    static const bool attr = [] {
-        cudaFuncSetAttribute(zgemm_umma_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM);
-        cudaFuncSetAttribute(zgemm_umma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM);
-        return true;
-    }();
-    (void)attr;
+    smem_attr_at_least(g.opB ? (const void *)zgemm_umma_kernel<1> : (const void *)zgemm_umma_kernel<0>, UM_SMEM);
     dim3 grid(cdiv(g.m, UM_BM), cdiv(g.n, UM_BN), g.batch);
     // 16-byte loads need every element address of an even row (A) or even k (B)
     // 16-byte aligned: an aligned base, even leading dimension and batch stride

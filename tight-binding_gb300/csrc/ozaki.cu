@@ -526,11 +526,7 @@ template <int SA> static void ozaki_product(cudaStream_t s, const OzakiX &ox, co
                                             double2 *Y)
 {
     const int n = ox.n, np = ox.np, batch = ox.batch;
-    static const bool attr = [] {
-        cudaFuncSetAttribute(k_oz_gemm<SA>, cudaFuncAttributeMaxDynamicSharedMemorySize, OZ_SMEM);
-        return true;
-    }();
-    (void)attr;
+    smem_attr_at_least((const void *)k_oz_gemm<SA>, OZ_SMEM);
     // one CTA per SM (its shared and tensor memory allow no second), each
     // looping over tiles
     const long ntiles = (long)(np / OZ_NX) * (np / OZ_MA) * batch;

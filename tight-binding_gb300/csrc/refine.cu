@@ -687,11 +687,7 @@ void refine_eigen(cudaStream_t s, RefineWork &w, const double2 *H, const double2
     //    diagonal over all i, its off-diagonal on the band of near neighbours
     conj_transpose<float>(s, w.G, T2, n, B);
     NRLTB_LAUNCH(k_ref_update, cdiv(nb * 32, 256), 256, 0, s, w, T2);
-    static const bool band_attr = [] {
-        cudaFuncSetAttribute(k_ref_band, cudaFuncAttributeMaxDynamicSharedMemorySize, REF_BAND_SMEM);
-        return true;
-    }();
-    (void)band_attr;
+    smem_attr_at_least((const void *)k_ref_band, REF_BAND_SMEM);
     NRLTB_LAUNCH(k_ref_band, dim3(cdiv(n, REF_BT), B), 256, REF_BAND_SMEM, s, w, w.Fb);
     NRLTB_LAUNCH(k_ref_band_apply, cdiv(nb * (2 * REF_BAND + 1), 256), 256, 0, s, w, w.Fb);
     // 5. Z = X' + X' E, reordered
