@@ -142,3 +142,15 @@ for dev in (0, 1):
     assert min(runs[-1]) > 0 and lib.fake_refused(b"k_", dev) + lib.fake_refused(b"zgemm", dev) == 0
 assert runs[0] == runs[1]
 """)
+
+
+@pytest.mark.parametrize("n,digits", [(9, False), (15, False), (16, True)])
+def test_digit_scratch_goes_to_orders_that_can_use_it(fake_lib, n, digits):
+    """No product of an order below 16 is a digit product; their scratch for 600 matrices would be 138 MB, everything
+    else a solve of these orders needs less than 16 MB a buffer."""
+    _run(fake_lib, f"""
+h = context()
+assert diag(h, {n}, 600, True) == 0
+assert (lib.fake_runs(b"8k_z_gemm", 0) > 0) == {digits}
+assert (lib.fake_largest_alloc() > 100e6) == {digits}
+""")

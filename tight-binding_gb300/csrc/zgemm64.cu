@@ -613,11 +613,12 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
 // takes 15 000 cycles a chunk (tensor pipe 60 % busy, 8 700 cycles of MMAs), the
 // rest waiting on the folds, whose conversions and 64-bit adds come to 6 000 issue
 // slots a chunk; a tile's entry and write-back add about 20 000 cycles.
+constexpr int Z_MIN = 16;
 bool zgemm64_supported(const GemmArgs<double> &g)
 {
     const bool al = g.alpha.y == 0.0 && (g.alpha.x == 1.0 || g.alpha.x == -1.0);
     const bool be = g.beta.y == 0.0 && (g.beta.x == 0.0 || g.beta.x == 1.0);
-    return al && be && g.m >= 16 && g.n >= 16 && g.k >= 16 && g.k <= 131072;
+    return al && be && g.m >= Z_MIN && g.n >= Z_MIN && g.k >= Z_MIN && g.k <= 131072;
 }
 
 static inline size_t z_al(size_t x) { return (x + 255) & ~size_t(255); }
@@ -644,8 +645,10 @@ static size_t z_bytes_per_matrix(int m, int n, int k)
 
 size_t zgemm64_scratch_bytes(int n, int batch)
 {
-    // enough for every matrix of a batch at once, or as many as Z_SCRATCH_MAX holds:
-    // a larger batch goes in parts, and one matrix above it takes the FMA pipe
+    // enough for every matrix of a batch at once, or as many as ZGEMM64_SCRATCH_MAX holds:
+    // a larger batch goes in parts, and one matrix above it takes the FMA pipe, as
+    // every product of an order below Z_MIN does
+    if (n < Z_MIN) return 0;
     const size_t per = z_bytes_per_matrix(n, n, n);
     if (per > ZGEMM64_SCRATCH_MAX) return 0;
     return std::min<size_t>(per * batch, ZGEMM64_SCRATCH_MAX) + 4 * 256;
