@@ -14,7 +14,7 @@ enum { MAXF = 512, MAXD = 8, MAXA = 4096 };
 static struct { const void *host; const char *name; int limit[MAXD]; int runs[MAXD]; int refused[MAXD]; } fn[MAXF];
 static struct { void *p; size_t bytes; } mem[MAXA];
 static int nfn, clusters = 1000;
-static size_t free_bytes = (size_t)256 << 30, alloc_limit = (size_t)256 << 30, largest;
+static size_t free_bytes = (size_t)256 << 30, capacity = (size_t)256 << 30, used, largest;
 static char no_launch[128], no_limit[128], no_cluster[128];
 static __thread int device;
 static __thread cudaError_t last;
@@ -30,7 +30,8 @@ static int named(int f, const char *part) { return part[0] && strstr(fn[f].name,
 /* what the tests set and read */
 void fake_clusters(int n) { clusters = n; }
 void fake_free_bytes(size_t n) { free_bytes = n; }
-void fake_alloc_limit(size_t n) { alloc_limit = n; }
+void fake_capacity(size_t n) { capacity = n; }
+size_t fake_used(void) { return used; }
 void fake_refuse_launch(const char *part) { snprintf(no_launch, sizeof no_launch, "%s", part); }
 void fake_refuse_limit(const char *part) { snprintf(no_limit, sizeof no_limit, "%s", part); }
 void fake_refuse_cluster(const char *part) { snprintf(no_cluster, sizeof no_cluster, "%s", part); }
@@ -140,12 +141,13 @@ const char *cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no er
 cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { *f = free_bytes; *t = (size_t)256 << 30; return cudaSuccess; }
 cudaError_t cudaMalloc(void **p, size_t n)
 {
-    if (n > alloc_limit) return ret(cudaErrorMemoryAllocation);
+    if (used + n > capacity) return ret(cudaErrorMemoryAllocation);
     if (n > largest) largest = n;
     for (int i = 0; i < MAXA; ++i)
         if (!mem[i].p) {
             *p = mem[i].p = calloc(1, n);
             mem[i].bytes = n;
+            used += n;
             return *p ? cudaSuccess : ret(cudaErrorMemoryAllocation);
         }
     abort();
@@ -153,7 +155,7 @@ cudaError_t cudaMalloc(void **p, size_t n)
 cudaError_t cudaFree(void *p)
 {
     for (int i = 0; p && i < MAXA; ++i)
-        if (mem[i].p == p) { free(p); mem[i].p = NULL; return cudaSuccess; }
+        if (mem[i].p == p) { free(p); mem[i].p = NULL; used -= mem[i].bytes; return cudaSuccess; }
     return p ? ret(cudaErrorInvalidValue) : cudaSuccess;
 }
 cudaError_t cudaMemset(void *p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }

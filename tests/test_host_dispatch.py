@@ -19,9 +19,9 @@ for f in ("fake_runs", "fake_refused"):
     getattr(lib, f).argtypes = [C.c_char_p, C.c_int]
 for f in ("fake_refuse_launch", "fake_refuse_limit", "fake_refuse_cluster"):
     getattr(lib, f).argtypes = [C.c_char_p]
-for f in ("fake_free_bytes", "fake_alloc_limit"):
+for f in ("fake_free_bytes", "fake_capacity"):
     getattr(lib, f).argtypes = [C.c_size_t]
-lib.fake_largest_alloc.restype = C.c_size_t
+lib.fake_largest_alloc.restype = lib.fake_used.restype = C.c_size_t
 
 def context(device=0):
     h = C.c_void_p()
@@ -153,4 +153,21 @@ h = context()
 assert diag(h, {n}, 600, True) == 0
 assert (lib.fake_runs(b"8k_z_gemm", 0) > 0) == {digits}
 assert (lib.fake_largest_alloc() > 100e6) == {digits}
+""")
+
+
+@pytest.mark.parametrize("room,digits", [(1.0, True), (0.7, True), (0.21, True), (0.1, False)])
+def test_digit_scratch_that_does_not_fit(fake_lib, room, digits):
+    """5 matrices of order 288 on a device that has room for a part of their 41.4 MB of digits, which are asked for
+    last: the products go in parts, and on the FMA pipe where not even one matrix's digits fit."""
+    _run(fake_lib, f"""
+h = context()
+assert diag(h, 288, 5, True) == 0
+used, whole = lib.fake_used(), lib.fake_runs(b"8k_z_gemm", 0)
+assert lib.nrltb_ctx_destroy(h) == 0 and lib.fake_used() == 0
+lib.fake_capacity(used - int({1 - room} * 41.4e6))
+h = context()
+assert diag(h, 288, 5, True) == 0 and diag(h, 288, 5, False) == 0
+runs = lib.fake_runs(b"8k_z_gemm", 0) - whole
+assert runs > whole if {digits} else runs == 0
 """)

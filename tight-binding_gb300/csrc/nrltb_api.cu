@@ -583,14 +583,20 @@ static int run_bloch(nrltb_ctx *c, int k0, int nk, int which0, double2 *M1, doub
 // aligned offset (double2 accesses need 16-byte alignment).
 static size_t zoff(size_t nn, int nk) { return (sizeof(float2) * nn * nk + 255) & ~size_t(255); }
 
-// digit scratch of the FP64 products of nk matrices of order nv
-static int z_scratch(nrltb_ctx *c, int nv, int nk, ZScratch &zs)
+// digit scratch of the FP64 products of nk matrices of order nv: as much of it as the
+// device has (the products go in smaller parts, or on the FMA pipe, with less), half of it
+// at a time down to one matrix
+static void z_scratch(nrltb_ctx *c, int nv, int nk, ZScratch &zs)
 {
-    const size_t bytes = zgemm64_scratch_bytes(nv, nk);
-    RET(c->d_zs.ensure(bytes));
+    size_t bytes = zgemm64_scratch_bytes(nv, nk);
+    const size_t one = zgemm64_scratch_bytes(nv, 1);
+    const Refusable r;
+    while (c->d_zs.ensure(bytes) != NRLTB_OK) {
+        r.clear();
+        bytes = bytes == one ? 0 : std::max(one, bytes / 2);
+    }
     zs.p = c->d_zs.p;
     zs.bytes = bytes;
-    return NRLTB_OK;
 }
 
 static size_t per_k_bytes(int nv, int prec)
@@ -635,7 +641,7 @@ static int run_solve(nrltb_ctx *c, int nv, int nkc, int prec, const double2 *H, 
         RET(c->d_work.ensure(eig_work_bytes<double>(nv, nkc)));
         EigWork<double> w;
         eig_work_carve<double>(w, c->d_work.p, nv, nkc);
-        RET(z_scratch(c, nv, nkc, w.zs));
+        z_scratch(c, nv, nkc, w.zs);
         // one stream: the WY factors and the tridiagonal solve both load the
         // FP64 pipe, and overlapping them measured slower
         eig_solve<double>(s, w, H, S, eig, Zout, vectors);
@@ -727,7 +733,7 @@ static int run_lowdin(nrltb_ctx *c, int nv, int nkc, const double2 *S, const dou
         RET(c->d_work.ensure(eig_work_bytes<double>(nv, nkc)));
         EigWork<double> w;
         eig_work_carve<double>(w, c->d_work.p, nv, nkc);
-        RET(z_scratch(c, nv, nkc, w.zs));
+        z_scratch(c, nv, nkc, w.zs);
         eig_solve<double>(s, w, A, B, o, V, true);
         CKL();
         const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
@@ -761,7 +767,7 @@ static int fix_nonpd(nrltb_ctx *c, int nv, const std::vector<int> &bad, const do
     RET(c->d_work.ensure(eig_work_bytes<double>(nv, nb)));
     EigWork<double> w;
     eig_work_carve<double>(w, c->d_work.p, nv, nb);
-    RET(z_scratch(c, nv, nb, w.zs));
+    z_scratch(c, nv, nb, w.zs);
     eig_solve<double>(s, w, Hp, Sp, ep, nullptr, false);
     CKL();
     for (int j = 0; j < nb; ++j)
@@ -916,7 +922,7 @@ static int run_all(nrltb_ctx *c)
                     const double2 *dH = overlap ? c->d_dH.as<double2>() : c->d_H.as<double2>();
                     const double2 *dS = overlap ? c->d_dS.as<double2>() : c->d_S.as<double2>();
                     ZScratch zs;
-                    if (o.precision == NRLTB_PREC_FP64 && (rc = z_scratch(c, nv, nkc, zs))) break;
+                    if (o.precision == NRLTB_PREC_FP64) z_scratch(c, nv, nkc, zs);
                     if ((rc = run_hf(s, nv, nkc, o.precision, dH, dS, Z, eig, c->d_deig.as<double>() + (size_t)r0 * nv,
                                      c->d_hf.p, overlap ? pre + 2 : nullptr, zs)))
                         { set_err("hf failed"); break; }
