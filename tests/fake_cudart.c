@@ -5,16 +5,18 @@
  *     and a launch above it (48 KB where it was never raised) is refused;
  *   - the last error of a thread, which cudaGetLastError clears;
  *   - chosen kernels, limits and allocations being refused (the fake_* calls). */
+#define _GNU_SOURCE
 #include <cuda_runtime_api.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <sys/mman.h>
 
 enum { MAXF = 512, MAXD = 8, MAXA = 4096 };
 static struct { const void *host; const char *name; int limit[MAXD]; int runs[MAXD]; int refused[MAXD]; } fn[MAXF];
 static struct { void *p; size_t bytes; } mem[MAXA];
 static int nfn, clusters = 1000;
-static size_t free_bytes = (size_t)256 << 30, capacity = (size_t)256 << 30, used, largest;
+static size_t capacity = (size_t)256 << 30, used, largest;
 static char no_launch[128], no_limit[128], no_cluster[128];
 static __thread int device;
 static __thread cudaError_t last;
@@ -29,7 +31,6 @@ static int named(int f, const char *part) { return part[0] && strstr(fn[f].name,
 
 /* what the tests set and read */
 void fake_clusters(int n) { clusters = n; }
-void fake_free_bytes(size_t n) { free_bytes = n; }
 void fake_capacity(size_t n) { capacity = n; }
 size_t fake_used(void) { return used; }
 void fake_refuse_launch(const char *part) { snprintf(no_launch, sizeof no_launch, "%s", part); }
@@ -138,24 +139,26 @@ cudaError_t cudaPeekAtLastError(void) { return last; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no error" : "refused by the test"; }
 
 /* memory */
-cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { *f = free_bytes; *t = (size_t)256 << 30; return cudaSuccess; }
+cudaError_t cudaMemGetInfo(size_t *f, size_t *t) { *f = capacity - used; *t = capacity; return cudaSuccess; }
 cudaError_t cudaMalloc(void **p, size_t n)
 {
     if (used + n > capacity) return ret(cudaErrorMemoryAllocation);
     if (n > largest) largest = n;
     for (int i = 0; i < MAXA; ++i)
         if (!mem[i].p) {
-            *p = mem[i].p = calloc(1, n);
+            *p = mmap(NULL, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+            if (*p == MAP_FAILED) abort();
+            mem[i].p = *p;
             mem[i].bytes = n;
             used += n;
-            return *p ? cudaSuccess : ret(cudaErrorMemoryAllocation);
+            return cudaSuccess;
         }
     abort();
 }
 cudaError_t cudaFree(void *p)
 {
     for (int i = 0; p && i < MAXA; ++i)
-        if (mem[i].p == p) { free(p); mem[i].p = NULL; used -= mem[i].bytes; return cudaSuccess; }
+        if (mem[i].p == p) { munmap(p, mem[i].bytes); mem[i].p = NULL; used -= mem[i].bytes; return cudaSuccess; }
     return p ? ret(cudaErrorInvalidValue) : cudaSuccess;
 }
 cudaError_t cudaMemset(void *p, int v, size_t n) { memset(p, v, n); return cudaSuccess; }

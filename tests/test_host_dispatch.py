@@ -19,8 +19,7 @@ for f in ("fake_runs", "fake_refused"):
     getattr(lib, f).argtypes = [C.c_char_p, C.c_int]
 for f in ("fake_refuse_launch", "fake_refuse_limit", "fake_refuse_cluster"):
     getattr(lib, f).argtypes = [C.c_char_p]
-for f in ("fake_free_bytes", "fake_capacity"):
-    getattr(lib, f).argtypes = [C.c_size_t]
+lib.fake_capacity.argtypes = [C.c_size_t]
 lib.fake_largest_alloc.restype = lib.fake_used.restype = C.c_size_t
 
 def context(device=0):
@@ -170,4 +169,24 @@ h = context()
 assert diag(h, 288, 5, True) == 0 and diag(h, 288, 5, False) == 0
 runs = lib.fake_runs(b"8k_z_gemm", 0) - whole
 assert runs > whole if {digits} else runs == 0
+""")
+
+
+@pytest.mark.parametrize("precision,mode,gigabytes", [("PREC_FP64", 4, 6), ("PREC_FP64", 4, 96), ("PREC_FP64", 6, 96),
+                                                      ("PREC_MIXED", 6, 6), ("PREC_MIXED", 6, 40), ("PREC_MIXED", 4, 6)])
+def test_chunks_of_k_fill_half_of_the_memory(fake_lib, precision, mode, gigabytes):
+    """The chunk is chosen for half of the free memory: with the digits of the FP64 products, which a large chunk
+    has 6 GB of, it comes to that (less what modes without derivatives don't use), the pair tables and results of
+    all k points aside (3 per cent, and 8 N^2 bytes a k point of charges)."""
+    _run(fake_lib, f"""
+from nrltb import Context, KMesh, Opts, synth
+abi._cache[abi.GPU_LIB] = lib
+lib.fake_capacity({gigabytes} << 30)
+st, par, _, _ = synth.bcc32()
+nk = 6000
+km = KMesh(np.zeros((nk, 3)), np.full(nk, 1.0 / nk))
+ctx = Context(0)
+ctx.bande(st, par, km, Opts(mode={mode}, precision=abi.{precision}))
+share = (lib.fake_used() - (8 * 288 * 288 * nk if {mode} == 6 else 0)) / ({gigabytes} << 29)
+assert lib.fake_runs(b"k_bloch_build", 0) > 2 and {0.95 if mode == 4 else 0.7} < share < 1.03, share
 """)

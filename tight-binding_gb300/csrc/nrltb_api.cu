@@ -599,25 +599,29 @@ static void z_scratch(nrltb_ctx *c, int nv, int nk, ZScratch &zs)
     zs.bytes = bytes;
 }
 
-static size_t per_k_bytes(int nv, int prec)
+// charges: the overlap's FP64 eigenproblem follows the solve in its work space
+static size_t per_k_bytes(int nv, int prec, bool charges)
 {
     size_t nn = (size_t)nv * nv;
     size_t w = (prec == NRLTB_PREC_FP64) ? eig_work_bytes<double>(nv, 1) : eig_work_bytes<float>(nv, 1);
     size_t x = (prec == NRLTB_PREC_FP64) ? 16 * nn : 8 * nn;
     size_t ref = (prec == NRLTB_PREC_FP64) ? 0 : refine_work_bytes(nv, 1);
-    if (prec == NRLTB_PREC_FP64) w += zgemm64_scratch_bytes(nv, 1);
+    if (charges) w = std::max(w, eig_work_bytes<double>(nv, 1));
     return 32 * nn + w + x + ref + hf_scratch_bytes(nv, 1) + 64 * (size_t)nv;
 }
 
-static int choose_chunk(int nv, int nk, int prec, size_t extra_per_k = 0)
+// k points of a chunk: as many as half of the free memory holds, with the digits of the FP64
+// products, which a large batch takes in parts (ZGEMM64_SCRATCH_MAX)
+static int choose_chunk(int nv, int nk, int prec, bool charges, size_t extra_per_k = 0)
 {
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    size_t budget = std::min<size_t>(free_b / 2, (size_t)48 << 30);
-    size_t per = per_k_bytes(nv, prec) + extra_per_k;
-    long c = (long)(budget / std::max<size_t>(per, 1));
-    c = std::max(1L, std::min<long>(c, nk));
-    return (int)c;
+    const size_t budget = std::min<size_t>(free_b / 2, (size_t)48 << 30);
+    const size_t per = std::max<size_t>(per_k_bytes(nv, prec, charges) + extra_per_k, 1);
+    const size_t digits = (prec == NRLTB_PREC_FP64 || charges) ? zgemm64_scratch_bytes(nv, 1) : 0;
+    size_t c = budget / (per + digits);
+    if (digits * c > ZGEMM64_SCRATCH_MAX) c = (budget - ZGEMM64_SCRATCH_MAX) / per;
+    return (int)std::max<size_t>(1, std::min<size_t>(c, nk));
 }
 
 // eigensolve of nkc matrices in H, S; eigenvalues into eig (ld nv), vectors into Z (FP64, optional)
@@ -816,7 +820,7 @@ static int run_all(nrltb_ctx *c)
         const size_t side_per_k = overlap ? 2 * ozaki_a_bytes(nv, 1, 6) +
                                                 (lpress ? 2 * ozaki_a_bytes(nv, 1, 3) + 32 * (size_t)nv * nv : 0)
                                           : 0;
-        const int chunk = choose_chunk(nv, nk, o.precision,
+        const int chunk = choose_chunk(nv, nk, o.precision, lqlmt && S.jsover,
                                        (lqlmt ? lowdin_bytes_per_k(nv) : 0) + (S.noncol ? 32 * nnb : 0) +
                                            side_per_k);
         const size_t nn = (size_t)nv * nv;
