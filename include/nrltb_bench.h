@@ -5,6 +5,7 @@
  */
 #ifndef NRLTB_BENCH_H
 #define NRLTB_BENCH_H
+#include <stddef.h>
 #include "nrltb.h"
 #ifdef __cplusplus
 extern "C" {
@@ -59,6 +60,18 @@ int nrltb_bench_cgemm_run(nrltb_ctx *ctx, int method, int m, int n, int k, int o
 int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, int k, int batch, int opA, int opB, int triA,
                           int triB, int triC, double alpha, double beta, const double *A, int lda, const double *B,
                           int ldb, double *C, int ldc);
+
+/* The same with `scratch` bytes for the operands' digits: less than those of the batch
+ * take it in parts, less than one matrix's the FMA pipe. */
+int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int n, int k, int batch, int opA, int opB, int triA,
+                              int triB, int triC, double alpha, double beta, const double *A, int lda, const double *B,
+                              int ldb, double *C, int ldc, size_t scratch);
+
+/* One digit product (1 the refinement's, 2 the FP64 GEMM's) of order n >= 128 on zeros,
+ * one of whose barrier waits is sure to run out, after a millisecond: returns
+ * NRLTB_E_TIMEOUT if the kernel raised its own fault flag and no other (and clears it),
+ * NRLTB_OK if it did not. */
+int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int batch);
 
 /* Fault flags of the tcgen05 kernels: bit 0 the FP32 GEMM, bit 1 the
  * refinement's digit product, bit 2 the FP64 GEMM's; a bit is set once a bounded barrier wait inside

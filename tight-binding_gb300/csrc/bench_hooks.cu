@@ -324,6 +324,14 @@ extern "C" int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, i
                                      int triA, int triB, int triC, double alpha, double beta, const double *A,
                                      int lda, const double *B, int ldb, double *C, int ldc)
 {
+    return nrltb_bench_zgemm_scratch(ctx, method, m, n, k, batch, opA, opB, triA, triB, triC, alpha, beta, A, lda, B, ldb,
+                                     C, ldc, zgemm64_scratch_bytes(std::max(m, std::max(n, k)), std::max(batch, 1)));
+}
+
+extern "C" int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int n, int k, int batch, int opA, int opB,
+                                         int triA, int triB, int triC, double alpha, double beta, const double *A,
+                                         int lda, const double *B, int ldb, double *C, int ldc, size_t scratch)
+{
     if (!ctx || m < 1 || n < 1 || k < 1 || batch < 1 || !A || !B || !C || method < 1 || method > 2) return NRLTB_E_ARG;
     const long ra = opA ? k : m, ca = opA ? m : k, rb = opB ? n : k, cb = opB ? k : n;
     if (lda < ra || ldb < rb || ldc < m) return NRLTB_E_ARG;
@@ -331,7 +339,7 @@ extern "C" int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, i
     cudaStream_t s = nrltb_ctx_stream_internal(ctx);
     DevBufs d;
     ZScratch zs;
-    zs.bytes = zgemm64_scratch_bytes(std::max(m, std::max(n, k)), batch);
+    zs.bytes = scratch;
     void *z = nullptr;
     if (cudaMalloc(&d.p[0], sizeof(double2) * na * batch) != cudaSuccess ||
         cudaMalloc(&d.p[1], sizeof(double2) * nb * batch) != cudaSuccess ||
@@ -352,6 +360,41 @@ extern "C" int nrltb_bench_zgemm_run(nrltb_ctx *ctx, int method, int m, int n, i
     }
     cudaFree(z);
     return ok && cudaGetLastError() == cudaSuccess ? NRLTB_OK : NRLTB_E_CUDA;
+}
+
+// one product on zeros whose wait for an emptied accumulator runs out
+extern "C" int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int batch)
+{
+    if (!ctx || (kernel != 1 && kernel != 2) || n < 128 || batch < 1) return NRLTB_E_ARG;
+    cudaStream_t s = nrltb_ctx_stream_internal(ctx);
+    const size_t nn = (size_t)n * n * batch;
+    const size_t scratch = kernel == 1 ? ozaki_work_bytes(n, batch) : zgemm64_scratch_bytes(n, batch);
+    TcWait wait;
+    wait.ns = 1000000;
+    wait.hold = 1;
+    DevBufs d;
+    for (int q = 0; q < 3; ++q)
+        if (cudaMalloc(&d.p[q], sizeof(double2) * nn) != cudaSuccess) return NRLTB_E_NOMEM;
+    if (cudaMalloc(&d.p[3], scratch) != cudaSuccess) return NRLTB_E_NOMEM;
+    bool ok = cudaMemsetAsync(d.p[0], 0, sizeof(double2) * nn, s) == cudaSuccess &&
+              cudaMemsetAsync(d.p[1], 0, sizeof(double2) * nn, s) == cudaSuccess;
+    const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
+    const double2 *A = (const double2 *)d.p[0], *B = (const double2 *)d.p[1];
+    if (kernel == 1) {
+        OzakiX ox = ozaki_prepare_x(s, (float2 *)d.p[1], n, batch, d.p[3]);
+        ox.wait = wait;
+        ozaki_gemm(s, ox, A, (double2 *)d.p[2]);
+    } else {
+        ZScratch zs;
+        zs.p = d.p[3];
+        zs.bytes = scratch;
+        zs.wait = wait;
+        zgemm<double>(s, n, n, n, batch, one, A, n, (long)n * n, 0, B, n, (long)n * n, 0, zero, (double2 *)d.p[2], n,
+                      (long)n * n, 0, 0, 0, zs);
+    }
+    ok = ok && cudaGetLastError() == cudaSuccess && cudaStreamSynchronize(s) == cudaSuccess;
+    const int raised = ok ? nrltb_bench_umma_fault(1) : 0;
+    return !ok ? NRLTB_E_CUDA : raised == 1 << kernel ? NRLTB_E_TIMEOUT : NRLTB_OK;
 }
 
 extern "C" int nrltb_bench_umma_fault(int clear)

@@ -63,8 +63,8 @@ constexpr int OZ_APF = 4;                 // A blocks ahead of the one being cop
 constexpr int OZ_NBUF = 4;                // tensor-memory level buffers, 128 columns each
 constexpr int OZ_FOLD_WARPS = 16;         // 4 per 32-lane quarter, 16 columns each
 constexpr int OZ_THREADS = 32 * (OZ_FOLD_WARPS + 2);   // + producer warp + MMA warp
-constexpr int OZ_NBAR = 2 * OZ_NXS + 2 * OZ_NAS + 2 * OZ_NBUF;
-constexpr int OZ_SMEM = OZ_NXS * OZ_XSTAGE + OZ_NAS * OZ_ABLK + 1024 + 8 * OZ_NBAR + 16;
+constexpr int OZ_NBAR = 2 * OZ_NXS + 2 * OZ_NAS + 2 * OZ_NBUF;   // and one for the MMAs at the end
+constexpr int OZ_SMEM = OZ_NXS * OZ_XSTAGE + OZ_NAS * OZ_ABLK + 1024 + 8 * (OZ_NBAR + 1) + 16;
 constexpr uint32_t OZ_TMEM_COLS = 512;
 
 static inline size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -252,7 +252,7 @@ __device__ __forceinline__ void df_add(float &hi, float &lo, float v)
 template <int SA>
 __global__ void __maxnreg__(96)
 k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, const int *exX, double2 *Y, int n,
-          int np, int batch, unsigned *fault)
+          int np, int batch, unsigned *fault, TcWait wait)
 {
     extern __shared__ __align__(16) unsigned char oz_raw[];
     const int KC = np / OZ_BK, NJ = np / OZ_NX, NI = np / OZ_MA;
@@ -262,7 +262,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
     unsigned char *sX = base;                                   // OZ_NXS x 72 KB
     unsigned char *sA = base + OZ_NXS * OZ_XSTAGE;              // OZ_NAS x 32 KB
     uint64_t *bars = (uint64_t *)(sA + OZ_NAS * OZ_ABLK);
-    uint32_t *tslot = (uint32_t *)(bars + OZ_NBAR);
+    uint32_t *tslot = (uint32_t *)(bars + OZ_NBAR + 1);
     volatile int *abort = (volatile int *)(tslot + 1);
     const uint32_t bar0 = oz_saddr(bars);
     // barrier addresses: X full/empty, A full/empty, level full/empty
@@ -289,10 +289,11 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int q = 0; q < OZ_NBAR; ++q) {
-            const bool fold = q >= 2 * OZ_NXS + 2 * OZ_NAS + OZ_NBUF;   // level-empty: one arrive per fold warp
+        for (int q = 0; q <= OZ_NBAR; ++q) {
+            // level-empty: one arrive per fold warp
+            const bool fold = q >= 2 * OZ_NXS + 2 * OZ_NAS + OZ_NBUF && q < OZ_NBAR;
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar0 + 8u * q),
-                         "r"(fold ? OZ_FOLD_WARPS : 1) : "memory");
+                         "r"(fold ? OZ_FOLD_WARPS + wait.hold : 1) : "memory");
         }
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -315,14 +316,15 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
             if (blockIdx.x < ntiles)
                 for (int qa = OZ_NAS; qa < min(OZ_APF, QA); ++qa)
                     oz_prefetch_l2(tile_a(blockIdx.x) + (long)qa * OZ_ABLK, OZ_ABLK);
-            int ti = 0;
+            int ti = 0, nx = 0, na = 0;   // tiles; X chunks and A planes sent
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++ti) {
                 const int tn = t + gridDim.x;   // the next tile, if any
                 const unsigned char *gX = tile_x(t), *gA = tile_a(t);
                 for (int kc = 0; kc < KC && ok; ++kc) {
                     const int g = ti * KC + kc, jx = g % OZ_NXS, ux = g / OZ_NXS;
-                    if (ux > 0 && !(ok = oz_wait(empty_x(jx), (ux - 1) & 1, abort))) break;
+                    if (ux > 0 && !(ok = oz_wait(empty_x(jx), (ux - 1) & 1, abort, wait.ns))) break;
                     oz_expect(full_x(jx), OZ_XSTAGE);
+                    nx = g + 1;
                     for (int q = 0; q < OZ_SB; ++q)
                         oz_bulk(oz_saddr(sX + jx * OZ_XSTAGE + q * OZ_XBLK), gX + ((long)kc * OZ_SB + q) * OZ_XBLK,
                                 OZ_XBLK, full_x(jx));
@@ -335,13 +337,17 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
                         if (qa + OZ_APF < QA) oz_prefetch_l2(gA + (long)(qa + OZ_APF) * OZ_ABLK, OZ_ABLK);
                         else if (tn < ntiles && qa + OZ_APF - QA < QA)
                             oz_prefetch_l2(tile_a(tn) + (long)(qa + OZ_APF - QA) * OZ_ABLK, OZ_ABLK);
-                        if (ua > 0 && !(ok = oz_wait(empty_a(ia), (ua - 1) & 1, abort))) break;
+                        if (ua > 0 && !(ok = oz_wait(empty_a(ia), (ua - 1) & 1, abort, wait.ns))) break;
                         oz_expect(full_a(ia), OZ_ABLK);
+                        na = qg + 1;
                         oz_bulk(oz_saddr(sA + ia * OZ_ABLK), gA + (long)qa * OZ_ABLK, OZ_ABLK, full_a(ia));
                     }
                 }
             }
             if (!ok) { *abort = 1; atomicOr(fault ? fault : &g_oz_fault, 1u); }
+            // the last copy into every stage has landed
+            for (int q = max(nx - OZ_NXS, 0); q < nx; ++q) oz_drain(full_x(q % OZ_NXS), (q / OZ_NXS) & 1);
+            for (int q = max(na - OZ_NAS, 0); q < na; ++q) oz_drain(full_a(q % OZ_NAS), (q / OZ_NAS) & 1);
         }
     } else if (warp == OZ_FOLD_WARPS + 1) {
         // ---- MMA issue: plane s takes the digit pairs (s, 0), (s, 1), (s, 2) ----
@@ -352,10 +358,10 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 for (int kc = 0; kc < KC && ok; ++kc, ++g) {
                     const int jx = g % OZ_NXS, ux = g / OZ_NXS;
-                    if (!(ok = oz_wait(full_x(jx), ux & 1, abort))) break;
+                    if (!(ok = oz_wait(full_x(jx), ux & 1, abort, wait.ns))) break;
                     for (int sdig = 0; sdig < SA; ++sdig) {
                         const int qg = g * SA + sdig, ia = qg % OZ_NAS, ua = qg / OZ_NAS;
-                        if (!(ok = oz_wait(full_a(ia), ua & 1, abort))) break;
+                        if (!(ok = oz_wait(full_a(ia), ua & 1, abort, wait.ns))) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t ar = sa0 + ia * OZ_ABLK, ai = ar + OZ_MA * 128;
                         for (int tdig = 0; tdig < OZ_SB; ++tdig) {
@@ -365,7 +371,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
                             const bool first = sdig == (L > 2 ? L - 2 : 0);
                             if (first && ql >= OZ_NBUF) {
                                 // the fold of level ql - OZ_NBUF has emptied this buffer
-                                if (!(ok = oz_wait(tempty(buf), ((ql - OZ_NBUF) / OZ_NBUF) & 1, abort))) break;
+                                if (!(ok = oz_wait(tempty(buf), ((ql - OZ_NBUF) / OZ_NBUF) & 1, abort, wait.ns))) break;
                                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             }
                             // X block rows: [-Xi | Xr | Xi]; w1 = [Xr | Xi], w2 = [-Xi | Xr]
@@ -395,9 +401,15 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
             if (ok && g > 0) {
                 // the last commit has landed: every MMA of the CTA has finished
                 const int jx = (g - 1) % OZ_NXS, ux = (g - 1) / OZ_NXS;
-                ok = oz_wait(empty_x(jx), ux & 1, abort);
+                ok = oz_wait(empty_x(jx), ux & 1, abort, wait.ns);
             }
-            if (!ok) { *abort = 1; atomicOr(fault ? fault : &g_oz_fault, 1u); }
+            if (!ok) {
+                *abort = 1;
+                atomicOr(fault ? fault : &g_oz_fault, 1u);
+                const uint32_t last = bar0 + 8u * OZ_NBAR;
+                oz_commit(last);
+                oz_drain(last, 0);
+            }
         }
     } else {
         // ---- fold warps: level sums -> double-float accumulators -> Y ----
@@ -413,7 +425,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
 #pragma unroll 1
                 for (int L = 0; L < NL; ++L) {
                     const int ql = g * NL + L, buf = ql % OZ_NBUF;
-                    ok = __all_sync(0xffffffffu, oz_wait(tfull(buf), (ql / OZ_NBUF) & 1, abort));
+                    ok = __all_sync(0xffffffffu, oz_wait(tfull(buf), (ql / OZ_NBUF) & 1, abort, wait.ns));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const float w = ldexpf(1.0f, -8 * (L + 2));
@@ -534,7 +546,7 @@ template <int SA> static void ozaki_product(cudaStream_t s, const OzakiX &ox, co
     const int grid = (int)std::min<long>(ntiles, oz_device_sms());
     cudaEvent_t ev = kt_begin(s);
     NRLTB_LAUNCH(k_oz_gemm<SA>, grid, OZ_THREADS, OZ_SMEM, s, DA, (const unsigned char *)ox.DX, exA, ox.exX, Y, n,
-                 np, batch, g_fault_word);
+                 np, batch, g_fault_word, ox.wait);
     kt_end(ev, s, KC_DIGIT_GEMM, 8.0 * n * (double)n * n * batch);
 }
 

@@ -49,7 +49,7 @@ constexpr int Z_TILE = 128 * 128;           // one plane tile, bytes
 constexpr int Z_SLOT = 2 * Z_TILE;          // planes A_p and X_p
 constexpr int Z_FOLD = 16;                  // fold warps: 4 per 32-lane quarter, 16 columns each
 constexpr int Z_THREADS = 32 * (Z_FOLD + 2);   // + producer warp + MMA warp
-constexpr int Z_NBAR = 2 * ZD + 8;          // slot full / empty, level full / empty
+constexpr int Z_NBAR = 2 * ZD + 9;          // slot full / empty, level full / empty, MMAs at the end
 constexpr int Z_SMEM = ZD * Z_SLOT + 1024 + 8 * Z_NBAR + 16;
 constexpr int Z_BAD = INT_MAX;              // exponent of a row or column with an infinity or a NaN
 static_assert(Z_SMEM <= 227 * 1024, "planes of a chunk fit the shared memory of an SM");
@@ -81,6 +81,7 @@ struct ZProduct {
     int order, per, gb;   // tile order, tiles of one matrix, matrices of a group
     double2 *C;
     long ldc, sC;
+    TcWait wait;
 };
 }  // namespace
 
@@ -386,6 +387,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
     auto empty = [&](int p) { return bar0 + 8u * (ZD + p); };
     auto tfull = [&](int q) { return bar0 + 8u * (2 * ZD + q); };
     auto tempty = [&](int q) { return bar0 + 8u * (2 * ZD + 4 + q); };
+    const uint32_t last = bar0 + 8u * (2 * ZD + 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -395,7 +397,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
     if (tid == 0) {
         for (int q = 0; q < Z_NBAR; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar0 + 8u * q),
-                         "r"(q >= 2 * ZD + 4 ? Z_FOLD : 1) : "memory");
+                         "r"(q >= 2 * ZD + 4 && q < 2 * ZD + 8 ? Z_FOLD + g.wait.hold : 1) : "memory");
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -409,7 +411,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
         // ---- producer: slots 6, 5, .. 0 of every chunk ----
         if (lane == 0) {
             bool ok = true;
-            int c = 0;   // chunks of this CTA so far
+            int c = 0, stop = 0;   // chunks of this CTA so far; slot at which it gave up
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 int b, it, jt;
                 z_tile(g, t, b, it, jt);
@@ -420,7 +422,10 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                 const unsigned char *px = g.DX + (((long)b * g.nt + jt) * g.kc) * ZD * Z_TILE;
                 for (int kc = c0; kc < c1 && ok; ++kc, ++c)
                     for (int p = ZD - 1; p >= 0; --p) {
-                        if (c > 0 && !(ok = oz_wait(empty(p), (c - 1) & 1, abort))) break;
+                        if (c > 0 && !(ok = oz_wait(empty(p), (c - 1) & 1, abort, g.wait.ns))) {
+                            stop = p + 1;
+                            break;
+                        }
                         const uint32_t dst = oz_saddr(base + p * Z_SLOT);
                         const long off = ((long)kc * ZD + p) * Z_TILE;
                         oz_expect(full(p), Z_SLOT);
@@ -433,6 +438,11 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                     }
             }
             if (!ok) { *abort = 1; atomicOr(fault ? fault : &g_z64_fault, 1u); }
+            // every copy has landed (c counts the chunk it gave up in: slots stop .. 6 were sent)
+            for (int p = 0; p < ZD; ++p) {
+                const int sent = p < stop ? c - 1 : c;
+                if (sent > 0) oz_drain(full(p), (sent - 1) & 1);
+            }
         }
     } else if (warp == Z_FOLD + 1) {
         // ---- MMA issue ----
@@ -453,7 +463,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                     for (int L = ZL - 1; L >= 0; --L) {
                         if (!ok) break;
                         const int q = 7 - L, buf = q & 3, use = 2 * c + (q >> 2);
-                        if (use > 0) ok = oz_wait(tempty(buf), (use - 1) & 1, abort);
+                        if (use > 0) ok = oz_wait(tempty(buf), (use - 1) & 1, abort, g.wait.ns);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t tl = tmem + 128u * buf;
                         // pairs (sd, L - sd) from the middle outwards: the slots that the
@@ -465,7 +475,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                             const int sd = (u & 1) ? mid - (u + 1) / 2 : mid + u / 2, td = L - sd;
                             if (L == ZL - 1 || (L == ZL - 2 && (sd == 0 || td == 0))) {
                                 // first reads of this chunk's slots
-                                if (ok) ok = oz_wait(full(sd), c & 1, abort) && oz_wait(full(td), c & 1, abort);
+                                if (ok) ok = oz_wait(full(sd), c & 1, abort, g.wait.ns) && oz_wait(full(td), c & 1, abort, g.wait.ns);
                                 if (!ok) break;
                                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             }
@@ -481,8 +491,13 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                     }
                 }
             }
-            if (ok && c > 0) ok = oz_wait(empty(0), (c - 1) & 1, abort);   // every MMA has finished
-            if (!ok) { *abort = 1; atomicOr(fault ? fault : &g_z64_fault, 1u); }
+            if (ok && c > 0) ok = oz_wait(empty(0), (c - 1) & 1, abort, g.wait.ns);   // every MMA has finished
+            if (!ok) {
+                *abort = 1;
+                atomicOr(fault ? fault : &g_z64_fault, 1u);
+                oz_commit(last);
+                oz_drain(last, 0);
+            }
         }
     } else if (warp < Z_FOLD) {
         // ---- fold warps ----
@@ -527,7 +542,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
 #pragma unroll
                 for (int lp = 0; lp < 4; ++lp) {
                     const int buf = (2 * lp) & 3, use = 2 * c + (lp >> 1);
-                    if (ok) ok = oz_wait(tfull(buf), use & 1, abort) && oz_wait(tfull(buf + 1), use & 1, abort);
+                    if (ok) ok = oz_wait(tfull(buf), use & 1, abort, g.wait.ns) && oz_wait(tfull(buf + 1), use & 1, abort, g.wait.ns);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -731,6 +746,7 @@ bool zgemm64_launch(cudaStream_t s, const GemmArgs<double> &g, const ZScratch &z
         p.C = g.C + b0 * g.sC;
         p.ldc = g.ldc;
         p.sC = g.sC;
+        p.wait = zs.wait;
         p.order = g.triC == 1   ? Z_LOWER
                   : g.triA == 1 ? Z_ROWS_DOWN
                   : g.triA == 2 ? Z_ROWS_UP
