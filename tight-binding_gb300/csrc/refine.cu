@@ -33,6 +33,7 @@
 // far below 1e-9 Ry; the remaining error is third order in the FP32 error.
 #include <cfloat>
 #include "refine.cuh"
+#include "refine_cut.h"
 #include "gemm.cuh"
 #include "ozaki.cuh"
 #include "sums.cuh"
@@ -183,26 +184,7 @@ __global__ void __launch_bounds__(1024) k_ref_clusters(RefineWork w, int *status
         int forced = 0, p0 = 0;
         for (int p = 1; p <= n; ++p) {
             if (p < n && srt[p] - srt[p - 1] < delta) continue;
-            int stk[64][2], sp = 0;
-            stk[sp][0] = p0; stk[sp][1] = p; ++sp;
-            while (sp > 0) {
-                --sp;
-                const int a = stk[sp][0], e = stk[sp][1];
-                if (e - a <= REF_CMAX || sp >= 62) {
-                    for (int q = a; q < e; ++q) { pos0[ord[q]] = a; csz[ord[q]] = e - a; }
-                    if (e - a > REF_CMAX) forced = 1;
-                    continue;
-                }
-                int cut = a + 1;
-                double best = -1.0;
-                for (int q = a + 1; q < e; ++q) {
-                    const double g = srt[q] - srt[q - 1];
-                    if (g > best) { best = g; cut = q; }
-                }
-                if (best < 1e-7 * span) forced = 1;
-                stk[sp][0] = a; stk[sp][1] = cut; ++sp;
-                stk[sp][0] = cut; stk[sp][1] = e; ++sp;
-            }
+            forced |= ref_cut(srt, p0, p, REF_CMAX, 1e-7 * span, ord, pos0, csz);
             p0 = p;
         }
         if (forced) status[b] = NRLTB_K_NOT_CONVERGED;
