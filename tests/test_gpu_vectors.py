@@ -1,0 +1,55 @@
+"""Eigenvectors of matrices whose tridiagonal form falls into blocks, some of them zero or far from one in size."""
+import numpy as np
+import pytest
+
+from nrltb import abi
+
+pytestmark = pytest.mark.gpu
+
+
+def _hermitian(n, rng):
+    G = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+    return (G + G.conj().T) / 2
+
+
+def _two_blocks(n, size, seed):
+    """Half of the orbitals coupled among themselves, the others too, `size` times as strongly; and the same shuffled."""
+    rng, h = np.random.default_rng(seed), n // 2
+    G = _hermitian(n, rng)
+    G[:h, h:] = G[h:, :h] = 0
+    G[h:, h:] *= size
+    at = rng.permutation(n)
+    return [G, G[np.ix_(at, at)]]
+
+
+def _check(ctx, H, precision, norm=None):
+    """Residuals within 64 n units of the norm, as for any matrix (the mixed form's 1e-9), and orthonormal vectors
+    (within 1e-9: dstein's bound goes by the gaps)."""
+    n = len(H[0])
+    e, z, st = ctx.diag(np.array(H), np.tile(np.eye(n) + 0j, (len(H), 1, 1)), precision=precision)
+    assert (st == 0).all() and np.isfinite(e).all() and np.isfinite(z).all()
+    tol = 64 * n * 2.0 ** -53 if precision == abi.PREC_FP64 else 1e-9
+    for h, ej, zj in zip(H, e, z):
+        assert np.abs(h @ zj - zj * ej).max() <= tol * np.abs(np.linalg.eigvalsh(h)).max()
+        assert np.abs(zj.conj().T @ zj - np.eye(n)).max() <= 1e-9
+    return e
+
+
+# (the mixed form refines clusters of up to 16 vectors)
+@pytest.mark.parametrize("precision,n", [(abi.PREC_FP64, n) for n in (1, 2, 9, 20, 64, 128, 200)] +
+                         [(abi.PREC_MIXED, n) for n in (1, 2, 9, 16)])
+def test_zero_blocks(ctx, precision, n):
+    u = np.random.default_rng(n).normal(size=n) + 1j
+    H = [np.zeros((n, n), complex), np.outer(u, u.conj())]
+    if n > 1:
+        H += _two_blocks(n, 0.0, n) + _two_blocks(n, 1e-15, n)
+    _check(ctx, H, precision)
+
+
+@pytest.mark.parametrize("n", [9, 20, 64, 128, 200])
+def test_graded(ctx, n):
+    """Rows and columns falling by 2^-80: the reduction leaves zero blocks of the smallest."""
+    D = 2.0 ** -(np.arange(n) * 80.0 / n)
+    G = _hermitian(n, np.random.default_rng(n)) * D[:, None] * D
+    at = np.random.default_rng(n).permutation(n)
+    _check(ctx, [G, G[::-1, ::-1], G[np.ix_(at, at)]], abi.PREC_FP64)

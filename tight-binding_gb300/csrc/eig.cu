@@ -699,7 +699,15 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
     Strided<TB> S(scratch + ((long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, NT);
     // 1 / pivots, first and second super-diagonals of U, iterate
     Strided<TB> RG = S, DU = S + n, DU2 = S + 2 * n, v = S + 3 * n;
-    const TB tiny = eps_of<TB>() * TB(2) * TB(fmax(tnorm, (double)tiny_of<TB>()));
+    // A solve multiplies its right-hand side by up to 1 / tiny, and the norm squares that.  A block
+    // whose norm is so far from one that this leaves the range (one of zeros, above all) takes
+    // right-hand sides of the size of `tiny`; the factor is a power of two and goes with the norm.
+    constexpr int range = sizeof(TB) == 8 ? 400 : 40;
+    const double tn = fmax(tnorm, sizeof(TB) == 8 ? 0x1p-900 : 0x1p-80);
+    const TB tiny = eps_of<TB>() * TB(2) * TB(tn);
+    const int ex = (__double2hiint(tn) >> 20) - 1023;
+    const bool far = ex < -range || ex > range;
+    const TB size = far ? TB(__hiloint2double((1023 + ex - (sizeof(TB) == 8 ? 51 : 22)) << 20, 0)) : TB(1);
     const TB lam = TB(L[r]);
     auto pivot = [&](TB g) { return (fabs(g) < tiny) ? ((g < TB(0)) ? -tiny : tiny) : g; };
     const unsigned seed = (unsigned)(b * 7919 + r);
@@ -713,7 +721,12 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
         // forward: factor (dgttrf) and apply P, L; element k + 1 of the
         // right-hand side is the previous iterate scaled by inv (the random
         // start in the first iteration)
-        auto rhs = [&](int k) { return it == 0 ? hash_unit<TB>(seed, (unsigned)k) : v[k] * inv; };
+        auto rhs = [&](int k) {
+            if (it > 0) return v[k] * inv;
+            TB h = hash_unit<TB>(seed, (unsigned)k);
+            if (far) h *= size;
+            return h;
+        };
         TB dcur = Dk(b0) - lam, ducur = (len > 1) ? Ek(b0) : TB(0);
         TB vc = rhs(0);
         for (int kb = 0; kb < len - 1; kb += INV_BLK) {
@@ -793,6 +806,7 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
         }
         nrm = sqrt(nrm);
         inv = (nrm > TB(0)) ? TB(1) / nrm : TB(0);
+        if (far && it < iters - 1) inv *= size;
     }
     // sign convention: largest component positive
     (void)kmax;
