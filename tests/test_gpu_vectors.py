@@ -53,3 +53,16 @@ def test_graded(ctx, n):
     G = _hermitian(n, np.random.default_rng(n)) * D[:, None] * D
     at = np.random.default_rng(n).permutation(n)
     _check(ctx, [G, G[::-1, ::-1], G[np.ix_(at, at)]], abi.PREC_FP64)
+
+
+@pytest.mark.parametrize("n", [4, 9, 20, 64, 128, 200])
+@pytest.mark.parametrize("size", [1e-15, 1e-40, 1e-70, 1e-100, 1e-150])
+def test_small_blocks_have_their_own_scale(ctx, n, size):
+    """A decoupled block's eigenvalues are good to 32 n units of the block's norm, however small it is beside the
+    other's (e^2 stays a normal number), and its vectors orthonormal; shuffled, the reduction mixes the blocks and
+    the matrix's norm counts."""
+    H = _two_blocks(n, size, n)
+    e = _check(ctx, H, abi.PREC_FP64)
+    w = np.linalg.eigvalsh(H[0][n // 2:, n // 2:] / size)
+    got = np.sort(e[0][np.argsort(np.abs(e[0]))[:n - n // 2]]) / size
+    assert np.abs(got - w).max() <= 32 * n * 2.0 ** -53 * np.abs(w).max()

@@ -413,10 +413,12 @@ struct TriPoly {
     double m;      // mantissa part and binary exponent of p_n(x)
     int ex, cnt;   // eigenvalues of the block below x
 };
-// d, e2: the block's rows scaled so that the largest row sum is about 1
-__device__ __forceinline__ TriPoly tri_poly(const double *d, const double *e2, int b0, int b1, double x)
+// d(k), e2(k): the block's rows, scaled so that its norm is about 1 (2^-100 at least: four
+// steps between two looks at the exponents must not leave the range)
+template <typename D, typename E>
+__device__ __forceinline__ TriPoly tri_poly(D d, E e2, int b0, int b1, double x)
 {
-    double p0 = 1.0, p1 = d[b0] - x;
+    double p0 = 1.0, p1 = d(b0) - x;
     int ex = 0, cnt = 0;
     // an exact zero counts as a sign change (the quotient form's -pivmin)
     auto nz = [](double p, double prev) {
@@ -439,7 +441,7 @@ __device__ __forceinline__ TriPoly tri_poly(const double *d, const double *e2, i
     for (; k + 4 <= b1 + 1; k += 4) {
         double dk[4], ek[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) { dk[u] = d[k + u]; ek[u] = e2[k + u - 1]; }
+        for (int u = 0; u < 4; ++u) { dk[u] = d(k + u); ek[u] = e2(k + u - 1); }
 #pragma unroll
         for (int u = 0; u < 4; ++u) step(dk[u], ek[u]);
         const int e1 = (__double2hiint(p1) >> 20) & 0x7FF, e0 = (__double2hiint(p0) >> 20) & 0x7FF;
@@ -458,13 +460,88 @@ __device__ __forceinline__ TriPoly tri_poly(const double *d, const double *e2, i
             ex -= sft;
         }
     }
-    for (; k <= b1; ++k) step(d[k], e2[k - 1]);
+    for (; k <= b1; ++k) step(d(k), e2(k - 1));
     TriPoly r;
     const int e1 = (__double2hiint(p1) >> 20) & 0x7FF;
     r.m = __hiloint2double((__double2hiint(p1) & (int)0x800FFFFFu) | (1023 << 20), __double2loint(p1));
     r.ex = ex + e1 - 1023;
     r.cnt = cnt;
     return r;
+}
+
+// Eigenvalue j of the block [b0, b1], known to lie in [glo, ghi] and thought to lie in [a, z],
+// to `atol`.
+template <typename D, typename E>
+__device__ __forceinline__ double tri_close(D d, E e2, int b0, int b1, int j, double a, double z, double glo, double ghi,
+                                            double tnorm, double atol)
+{
+    const double eps = eps_of<double>(), pivmin = DBL_MIN;
+    TriPoly pa = tri_poly(d, e2, b0, b1, a), pz = tri_poly(d, e2, b0, b1, z);
+    double h = 64.0 * (double)eps_of<float>() * tnorm;
+    for (int t = 0; t < 16 && pa.cnt > j && a > glo; ++t, h *= 64.0) {
+        z = a;
+        pz = pa;
+        a = fmax(glo, a - h);
+        pa = tri_poly(d, e2, b0, b1, a);
+    }
+    h = 64.0 * (double)eps_of<float>() * tnorm;
+    for (int t = 0; t < 16 && pz.cnt <= j && z < ghi; ++t, h *= 64.0) {
+        a = z;
+        pa = pz;
+        z = fmin(ghi, z + h);
+        pz = tri_poly(d, e2, b0, b1, z);
+    }
+    double wa = 1.0, wz = 1.0;   // Illinois weights of the two values
+    int side = 0;                // which end moved last (+1 a, -1 z), doubled when twice in a row
+    double width2 = 2.0 * (z - a);   // width two steps ago
+    for (int it = 0; it < 256; ++it) {
+        const double width = z - a, mid = a + 0.5 * width;
+        const double tol = fmax(atol, 2.0 * eps * fmax(fabs(a), fabs(z))) + pivmin;
+        if (!(width > tol) || mid <= a || mid >= z) break;
+        double x = mid;
+        const bool one = pz.cnt - pa.cnt == 1;
+        if (one && !(it & 1 && width > 0.5 * width2)) {
+            // zero of the line through the weighted values (they differ in sign)
+            const int de = max(-1000, min(1000, pz.ex - pa.ex));
+            const double fa = fabs(pa.m) * wa, fz = scalbn(fabs(pz.m) * wz, de);
+            x = a + width * (fa / (fa + fz));
+            // at least half a tolerance inside, so that the far end comes in too
+            x = fmin(fmax(x, a + 0.5 * tol), z - 0.5 * tol);
+            if (!(x > a && x < z)) x = mid;
+        }
+        if (it & 1) width2 = width;
+        const TriPoly p = tri_poly(d, e2, b0, b1, x);
+        if (p.cnt <= j) {
+            a = x;
+            pa = p;
+            wa = 1.0;
+            if (side > 0) wz *= 0.5;
+            side = 1;
+        } else {
+            z = x;
+            pz = p;
+            wz = 1.0;
+            if (side < 0) wa *= 0.5;
+            side = -1;
+        }
+    }
+    return a + 0.5 * (z - a);
+}
+
+// The same for a block that is smaller than the matrix by more than the shared copies' scale
+// can serve: from d and e themselves, scaled by 2^-sx for this block (whose numbers
+// lo, hi, tnorm are in that scale).
+__device__ __noinline__ double tri_close_small(const double *dg, const double *eg, int sx, int b0, int b1, int j, double lo,
+                                               double hi, double tnorm)
+{
+    const double sc = scalbn(1.0, -sx), atol = eps_of<double>() * tnorm;
+    const double glo = lo - 2.0 * atol - DBL_MIN, ghi = hi + 2.0 * atol + DBL_MIN;
+    auto d = [&](int k) { return dg[k] * sc; };
+    auto e2 = [&](int k) {
+        const double e = eg[k] * sc;
+        return e * e;
+    };
+    return tri_close(d, e2, b0, b1, j, glo, ghi, glo, ghi, tnorm, atol);
 }
 
 // Scaled copies of d and e^2 in FP64 and FP32 and the split flags, 25 n bytes: in
@@ -507,16 +584,21 @@ __global__ void k_tri_bisect64(const double *dd, const double *ee, double *lamlo
     double tnorm = 0, lo = 1e300, hi = -1e300, emax2 = 0;
     block_bounds(dg, eg, valid, b0, b1, lo, hi, tnorm, emax2);
     if (!valid) return;
-    lo *= sc;
-    hi *= sc;
-    tnorm *= sc;
-    const double eps = eps_of<double>(), atol = eps * tnorm, pivmin = DBL_MIN;
     const int j = r - b0;
-    const double glo = lo - 2.0 * atol - pivmin, ghi = hi + 2.0 * atol + pivmin;
     double lam;
-    if (b0 == b1) {
+    if (b0 != b1 && tnorm > 0 && tnorm * sc < 0x1p-100) {
+        frexp(tnorm, &sx);
+        sx = max(-900, sx);
+        const double bs = scalbn(1.0, -sx);
+        lam = tri_close_small(dg, eg, sx, b0, b1, j, lo * bs, hi * bs, tnorm * bs);
+    } else if (b0 == b1) {
         lam = d[b0];
     } else {
+        lo *= sc;
+        hi *= sc;
+        tnorm *= sc;
+        const double eps = eps_of<double>(), atol = eps * tnorm, pivmin = DBL_MIN;
+        const double glo = lo - 2.0 * atol - pivmin, ghi = hi + 2.0 * atol + pivmin;
         double a = glo, z = ghi;
         if (tnorm > 1e-30) {   // FP32's range holds the block
             float fa = (float)glo, fz = (float)ghi;
@@ -529,56 +611,7 @@ __global__ void k_tri_bisect64(const double *dd, const double *ee, double *lamlo
             a = fmax(glo, (double)fa - m);
             z = fmin(ghi, (double)fz + m);
         }
-        TriPoly pa = tri_poly(d, e2, b0, b1, a), pz = tri_poly(d, e2, b0, b1, z);
-        double h = 64.0 * (double)eps_of<float>() * tnorm;
-        for (int t = 0; t < 16 && pa.cnt > j && a > glo; ++t, h *= 64.0) {
-            z = a;
-            pz = pa;
-            a = fmax(glo, a - h);
-            pa = tri_poly(d, e2, b0, b1, a);
-        }
-        h = 64.0 * (double)eps_of<float>() * tnorm;
-        for (int t = 0; t < 16 && pz.cnt <= j && z < ghi; ++t, h *= 64.0) {
-            a = z;
-            pa = pz;
-            z = fmin(ghi, z + h);
-            pz = tri_poly(d, e2, b0, b1, z);
-        }
-        double wa = 1.0, wz = 1.0;   // Illinois weights of the two values
-        int side = 0;                // which end moved last (+1 a, -1 z), doubled when twice in a row
-        double width2 = 2.0 * (z - a);   // width two steps ago
-        for (int it = 0; it < 256; ++it) {
-            const double width = z - a, mid = a + 0.5 * width;
-            const double tol = fmax(atol, 2.0 * eps * fmax(fabs(a), fabs(z))) + pivmin;
-            if (!(width > tol) || mid <= a || mid >= z) break;
-            double x = mid;
-            const bool one = pz.cnt - pa.cnt == 1;
-            if (one && !(it & 1 && width > 0.5 * width2)) {
-                // zero of the line through the weighted values (they differ in sign)
-                const int de = max(-1000, min(1000, pz.ex - pa.ex));
-                const double fa = fabs(pa.m) * wa, fz = scalbn(fabs(pz.m) * wz, de);
-                x = a + width * (fa / (fa + fz));
-                // at least half a tolerance inside, so that the far end comes in too
-                x = fmin(fmax(x, a + 0.5 * tol), z - 0.5 * tol);
-                if (!(x > a && x < z)) x = mid;
-            }
-            if (it & 1) width2 = width;
-            const TriPoly p = tri_poly(d, e2, b0, b1, x);
-            if (p.cnt <= j) {
-                a = x;
-                pa = p;
-                wa = 1.0;
-                if (side > 0) wz *= 0.5;
-                side = 1;
-            } else {
-                z = x;
-                pz = p;
-                wz = 1.0;
-                if (side < 0) wa *= 0.5;
-                side = -1;
-            }
-        }
-        lam = a + 0.5 * (z - a);
+        lam = tri_close([&](int k) { return d[k]; }, [&](int k) { return e2[k]; }, b0, b1, j, a, z, glo, ghi, tnorm, atol);
     }
     lamloc[(long)b * n + r] = scalbn(lam, sx);
     blk[((long)b * n + r) * 2 + 0] = b0;
