@@ -66,3 +66,13 @@ def test_small_blocks_have_their_own_scale(ctx, n, size):
     w = np.linalg.eigvalsh(H[0][n // 2:, n // 2:] / size)
     got = np.sort(e[0][np.argsort(np.abs(e[0]))[:n - n // 2]]) / size
     assert np.abs(got - w).max() <= 32 * n * 2.0 ** -53 * np.abs(w).max()
+
+
+@pytest.mark.parametrize("n", [2, 9, 33, 64, 160])
+@pytest.mark.parametrize("precision,size", [(abi.PREC_MIXED, s) for s in (1e-18, 1e-22, 1e-24, 1e-30)] +
+                         [(abi.PREC_FP64, s) for s in (1e-24, 1e-155, 1e-165, 1e-200)])
+def test_couplings_whose_squares_vanish(ctx, n, precision, size):
+    """Levels coupled by so little that the squares of a whole column are no longer numbers of the form's range."""
+    G = _hermitian(n, np.random.default_rng(n)) * size
+    G[np.arange(n), np.arange(n)] = np.cos(np.arange(n))
+    _check(ctx, [G], precision)

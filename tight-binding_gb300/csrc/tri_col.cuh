@@ -107,7 +107,7 @@ __device__ __forceinline__ void tc_reflector(double2 al, double xn2, double2 &ta
 {
     tau = scale = make_double2(0, 0);
     beta = al.x;
-    if (xn2 == 0 && al.y == 0) return;
+    if ((xn2 == 0 && al.y == 0) || tp_vanishes(al, xn2)) return;
     const double N = fma(al.y, al.y, fma(al.x, al.x, xn2));
     int e = ((__double2hiint(N) >> 20) & 0x7FF) - 1023;
     double g, y;   // sqrt(N), 1 / sqrt(N)
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(32 * TC_WARPS, 2) k_tri_mv(EigWork<T> w, int i
             const C2 al = col[base];
             C2 tau = zero, scale = zero;
             T beta = al.x;
-            if (xn2 != T(0) || al.y != T(0)) {
+            if ((xn2 != T(0) || al.y != T(0)) && !tp_vanishes(al, xn2)) {
                 T bb, rb;
                 tc_root(al.x * al.x + al.y * al.y + xn2, bb, rb);
                 if (al.x >= T(0)) { bb = -bb; rb = -rb; }

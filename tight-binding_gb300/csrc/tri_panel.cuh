@@ -39,6 +39,19 @@ constexpr int TP_RANKS = 8;   // tiles t mod TP_RANKS are summed first, whatever
 // values per lane of one butterfly (16: 16 warps fit an SM)
 template <typename T> struct TpNV { static constexpr int v = 16; };
 
+// A column whose elements' squares fall out of the range (2^-63 in FP32, 2^-511 in FP64) is
+// left as it is: its reflector would be a quotient of zeros.  xn2: |x|^2 of the elements
+// below al.  (FP64 on the exponents: the narrow pipe stays out of the column's chain.)
+__device__ __forceinline__ bool tp_vanishes(float2 al, float xn2)
+{
+    return fmaxf(fabsf(al.x), fabsf(al.y)) < 0x1p-63f && xn2 < 0x1p-126f;
+}
+__device__ __forceinline__ bool tp_vanishes(double2 al, double xn2)
+{
+    const int hi = 0x7FFFFFFF;
+    return max(__double2hiint(al.x) & hi, __double2hiint(al.y) & hi) < (1023 - 511) << 20 && __double2hiint(xn2) < 1 << 20;
+}
+
 // Transpose-reduce over the warp: lane l holds x[0..NV); afterwards x[0] of
 // lane l is sum over all lanes of x[u] with u = l >> (5 - log2 NV) (lanes that
 // share u hold the same total).
@@ -360,7 +373,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_tri_panel(EigWork<T> w, in
         tau = zero;
         {
             const T xnorm = sqrt(xn2);
-            if (xnorm == T(0) && al.y == T(0)) {
+            if ((xnorm == T(0) && al.y == T(0)) || tp_vanishes(al, xn2)) {
                 beta = (double)al.x;
             } else {
                 T bb = sqrt(al.x * al.x + al.y * al.y + xnorm * xnorm);
