@@ -68,7 +68,7 @@ int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int n, int k, i
                               int ldb, double *C, int ldc, size_t scratch);
 
 /* One digit product (1 the refinement's, 2 the FP64 GEMM's) of order n >= 128 on zeros,
- * one of whose barrier waits is sure to run out, after a millisecond: returns
+ * one of whose barrier waits is sure to run out, after two seconds: returns
  * NRLTB_E_TIMEOUT if the kernel raised its own fault flag and no other (and clears it),
  * NRLTB_OK if it did not. */
 int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int batch);

@@ -36,12 +36,11 @@ def _scratch(m, n, k, matrices):
 @pytest.mark.parametrize("kernel", [1, 2])
 @pytest.mark.parametrize("n,batch", [(128, 1), (160, 300), (385, 5)])
 def test_wait_that_runs_out_is_reported_and_leaves_nothing_behind(ctx, kernel, n, batch):
-    """The wait for an accumulator that is never said to be empty: the kernel gives up within its limit, says so,
+    """The wait for an accumulator that is never said to be empty: the kernel gives up after its two seconds, says so,
     and the products after it are those before it, bit for bit."""
     A, B = _operands(n, n, n, 3)
     before = _zgemm(ctx, A, B)
-    for _ in range(3):
-        assert ctx.lib.nrltb_bench_wait_runs_out(ctx.h, kernel, n, batch) == abi.NRLTB_E_TIMEOUT
+    assert ctx.lib.nrltb_bench_wait_runs_out(ctx.h, kernel, n, batch) == abi.NRLTB_E_TIMEOUT
     assert np.array_equal(_zgemm(ctx, A, B), before)
 
 

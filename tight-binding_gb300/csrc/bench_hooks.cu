@@ -369,9 +369,6 @@ extern "C" int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int 
     cudaStream_t s = nrltb_ctx_stream_internal(ctx);
     const size_t nn = (size_t)n * n * batch;
     const size_t scratch = kernel == 1 ? ozaki_work_bytes(n, batch) : zgemm64_scratch_bytes(n, batch);
-    TcWait wait;
-    wait.ns = 1000000;
-    wait.hold = 1;
     DevBufs d;
     for (int q = 0; q < 3; ++q)
         if (cudaMalloc(&d.p[q], sizeof(double2) * nn) != cudaSuccess) return NRLTB_E_NOMEM;
@@ -382,13 +379,13 @@ extern "C" int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int 
     const double2 *A = (const double2 *)d.p[0], *B = (const double2 *)d.p[1];
     if (kernel == 1) {
         OzakiX ox = ozaki_prepare_x(s, (float2 *)d.p[1], n, batch, d.p[3]);
-        ox.wait = wait;
+        ox.hold = 1;
         ozaki_gemm(s, ox, A, (double2 *)d.p[2]);
     } else {
         ZScratch zs;
         zs.p = d.p[3];
         zs.bytes = scratch;
-        zs.wait = wait;
+        zs.hold = 1;
         zgemm<double>(s, n, n, n, batch, one, A, n, (long)n * n, 0, B, n, (long)n * n, 0, zero, (double2 *)d.p[2], n,
                       (long)n * n, 0, 0, 0, zs);
     }

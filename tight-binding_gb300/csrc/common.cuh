@@ -192,13 +192,6 @@ extern thread_local long long *g_launch_counter;
 // concurrent contexts never see each other's faults.
 extern thread_local unsigned *g_fault_word;
 
-// Limit of a tcgen05 kernel's barrier waits; hold (tests): arrivals that the barrier of an
-// emptied accumulator waits for in vain, so that the wait for it runs out.
-struct TcWait {
-    unsigned long long ns = 2000000000ull;
-    int hold = 0;
-};
-
 // Kernel-class timing (off unless a context enables it): CUDA events on the
 // launching stream around each launch of a timed class, with the launch's
 // algorithmic work (flops or bytes), summed by nrltb_bench_kernel_stats.

@@ -7,6 +7,7 @@
 
 namespace nrltb {
 
+constexpr unsigned long long OZ_WAIT_NS = 2000000000ull;   // (as an argument it cost the products 2 to 3 %)
 constexpr int OZ_MA = 128;                // rows of A (and of the product) per CTA: tensor-memory lanes
 // instruction descriptor, kind::f16: D f32 (bits 4-5 = 1), A and B bf16
 // (bits 7-9, 10-12 = 1), both K-major, N >> 3 at bits 17-22, M >> 4 at 24-28
@@ -106,15 +107,15 @@ __device__ __forceinline__ unsigned long long oz_ns()
     return t;
 }
 
-// wait for the phase of the given parity, at most `ns` or until another
+// wait for the phase of the given parity, at most OZ_WAIT_NS or until another
 // role has given up (abort flag)
-__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity, volatile int *abort, unsigned long long ns)
+__device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity, volatile int *abort)
 {
     if (oz_try(bar, parity)) return true;
     const unsigned long long t0 = oz_ns();
     for (;;) {
         if (oz_try(bar, parity)) return true;
-        if (*abort || oz_ns() - t0 > ns) return false;
+        if (*abort || oz_ns() - t0 > OZ_WAIT_NS) return false;
     }
 }
 
@@ -122,8 +123,9 @@ __device__ __forceinline__ bool oz_wait(uint32_t bar, uint32_t parity, volatile 
 // copies or MMAs of its own in flight would have them write into the next one's memory
 static __device__ __noinline__ void oz_drain(uint32_t bar, uint32_t parity)
 {
+    if (oz_try(bar, parity)) return;
     const unsigned long long t0 = oz_ns();
-    while (!oz_try(bar, parity) && oz_ns() - t0 < 2000000000ull) {}
+    while (!oz_try(bar, parity) && oz_ns() - t0 < OZ_WAIT_NS) {}
 }
 
 __device__ __forceinline__ void oz_expect(uint32_t bar, uint32_t bytes)

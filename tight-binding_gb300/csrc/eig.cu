@@ -637,16 +637,17 @@ __device__ inline unsigned hash_bits(unsigned a, unsigned b)
     h ^= h >> 15; h *= 0x2C1B3C6Du; h ^= h >> 12; h *= 0x297A2D39u; h ^= h >> 15;
     return h & 0xFFFFFFu;
 }
-// m 2^-23 - 1 in [-1, 1) for a 24-bit m: exact in FP32 as in FP64, so the FP32
-// form gives the same values without the FP64 pipe
-template <typename TB> __device__ inline TB hash_unit(unsigned a, unsigned b);
-template <> __device__ inline double hash_unit<double>(unsigned a, unsigned b)
+// (m 2^-23 - 1) size in [-size, size) for a 24-bit m and a power of two: exact in FP32 as in
+// FP64, so the FP32 form gives the same values without the FP64 pipe
+template <typename TB> __device__ inline TB hash_unit(unsigned a, unsigned b, TB size)
 {
-    return (double)hash_bits(a, b) / (double)0x800000 - 1.0;
+    return (TB)hash_bits(a, b) * (size * TB(1.0 / 8388608.0)) - size;
 }
-template <> __device__ inline float hash_unit<float>(unsigned a, unsigned b)
+// 2^e, |e| < 1000 (FP32: 120)
+template <typename TB> __device__ inline TB pow2_of(int e)
 {
-    return (float)hash_bits(a, b) * (1.0f / 8388608.0f) - 1.0f;
+    if constexpr (sizeof(TB) == 8) return __hiloint2double((1023 + e) << 20, 0);
+    else return __int_as_float((127 + e) << 23);
 }
 
 // An array of one thread whose elements are `st` apart (thread-interleaved
@@ -739,8 +740,7 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
     const double tn = fmax(tnorm, sizeof(TB) == 8 ? 0x1p-900 : 0x1p-80);
     const TB tiny = eps_of<TB>() * TB(2) * TB(tn);
     const int ex = (__double2hiint(tn) >> 20) - 1023;
-    const bool far = ex < -range || ex > range;
-    const TB size = far ? TB(__hiloint2double((1023 + ex - (sizeof(TB) == 8 ? 51 : 22)) << 20, 0)) : TB(1);
+    const TB size = (ex < -range || ex > range) ? pow2_of<TB>(ex - (sizeof(TB) == 8 ? 51 : 22)) : TB(1);
     const TB lam = TB(L[r]);
     auto pivot = [&](TB g) { return (fabs(g) < tiny) ? ((g < TB(0)) ? -tiny : tiny) : g; };
     const unsigned seed = (unsigned)(b * 7919 + r);
@@ -754,12 +754,7 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
         // forward: factor (dgttrf) and apply P, L; element k + 1 of the
         // right-hand side is the previous iterate scaled by inv (the random
         // start in the first iteration)
-        auto rhs = [&](int k) {
-            if (it > 0) return v[k] * inv;
-            TB h = hash_unit<TB>(seed, (unsigned)k);
-            if (far) h *= size;
-            return h;
-        };
+        auto rhs = [&](int k) { return it == 0 ? hash_unit<TB>(seed, (unsigned)k, size) : v[k] * inv; };
         TB dcur = Dk(b0) - lam, ducur = (len > 1) ? Ek(b0) : TB(0);
         TB vc = rhs(0);
         for (int kb = 0; kb < len - 1; kb += INV_BLK) {
@@ -838,8 +833,7 @@ __global__ void k_tri_invit(const double *dd, const double *ee, const double *la
             }
         }
         nrm = sqrt(nrm);
-        inv = (nrm > TB(0)) ? TB(1) / nrm : TB(0);
-        if (far && it < iters - 1) inv *= size;
+        inv = (nrm > TB(0)) ? (it < iters - 1 ? size : TB(1)) / nrm : TB(0);
     }
     // sign convention: largest component positive
     (void)kmax;

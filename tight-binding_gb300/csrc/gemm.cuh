@@ -332,7 +332,7 @@ void zgemm_simt(cudaStream_t s, int m, int n, int k, int batch, typename cplx<T>
 struct ZScratch {
     void *p = nullptr;
     size_t bytes = 0;
-    TcWait wait;
+    int hold = 0;   // tests: arrivals that the barriers of emptied accumulators wait for in vain
 };
 constexpr size_t ZGEMM64_SCRATCH_MAX = (size_t)6 << 30;
 size_t zgemm64_scratch_bytes(int n, int batch);

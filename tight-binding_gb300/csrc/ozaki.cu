@@ -252,7 +252,7 @@ __device__ __forceinline__ void df_add(float &hi, float &lo, float v)
 template <int SA>
 __global__ void __maxnreg__(96)
 k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, const int *exX, double2 *Y, int n,
-          int np, int batch, unsigned *fault, TcWait wait)
+          int np, int batch, unsigned *fault, int hold)
 {
     extern __shared__ __align__(16) unsigned char oz_raw[];
     const int KC = np / OZ_BK, NJ = np / OZ_NX, NI = np / OZ_MA;
@@ -293,7 +293,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
             // level-empty: one arrive per fold warp
             const bool fold = q >= 2 * OZ_NXS + 2 * OZ_NAS + OZ_NBUF && q < OZ_NBAR;
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar0 + 8u * q),
-                         "r"(fold ? OZ_FOLD_WARPS + wait.hold : 1) : "memory");
+                         "r"(fold ? OZ_FOLD_WARPS + hold : 1) : "memory");
         }
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -322,7 +322,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
                 const unsigned char *gX = tile_x(t), *gA = tile_a(t);
                 for (int kc = 0; kc < KC && ok; ++kc) {
                     const int g = ti * KC + kc, jx = g % OZ_NXS, ux = g / OZ_NXS;
-                    if (ux > 0 && !(ok = oz_wait(empty_x(jx), (ux - 1) & 1, abort, wait.ns))) break;
+                    if (ux > 0 && !(ok = oz_wait(empty_x(jx), (ux - 1) & 1, abort))) break;
                     oz_expect(full_x(jx), OZ_XSTAGE);
                     nx = g + 1;
                     for (int q = 0; q < OZ_SB; ++q)
@@ -337,7 +337,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
                         if (qa + OZ_APF < QA) oz_prefetch_l2(gA + (long)(qa + OZ_APF) * OZ_ABLK, OZ_ABLK);
                         else if (tn < ntiles && qa + OZ_APF - QA < QA)
                             oz_prefetch_l2(tile_a(tn) + (long)(qa + OZ_APF - QA) * OZ_ABLK, OZ_ABLK);
-                        if (ua > 0 && !(ok = oz_wait(empty_a(ia), (ua - 1) & 1, abort, wait.ns))) break;
+                        if (ua > 0 && !(ok = oz_wait(empty_a(ia), (ua - 1) & 1, abort))) break;
                         oz_expect(full_a(ia), OZ_ABLK);
                         na = qg + 1;
                         oz_bulk(oz_saddr(sA + ia * OZ_ABLK), gA + (long)qa * OZ_ABLK, OZ_ABLK, full_a(ia));
@@ -358,10 +358,10 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
             for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
                 for (int kc = 0; kc < KC && ok; ++kc, ++g) {
                     const int jx = g % OZ_NXS, ux = g / OZ_NXS;
-                    if (!(ok = oz_wait(full_x(jx), ux & 1, abort, wait.ns))) break;
+                    if (!(ok = oz_wait(full_x(jx), ux & 1, abort))) break;
                     for (int sdig = 0; sdig < SA; ++sdig) {
                         const int qg = g * SA + sdig, ia = qg % OZ_NAS, ua = qg / OZ_NAS;
-                        if (!(ok = oz_wait(full_a(ia), ua & 1, abort, wait.ns))) break;
+                        if (!(ok = oz_wait(full_a(ia), ua & 1, abort))) break;
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t ar = sa0 + ia * OZ_ABLK, ai = ar + OZ_MA * 128;
                         for (int tdig = 0; tdig < OZ_SB; ++tdig) {
@@ -371,7 +371,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
                             const bool first = sdig == (L > 2 ? L - 2 : 0);
                             if (first && ql >= OZ_NBUF) {
                                 // the fold of level ql - OZ_NBUF has emptied this buffer
-                                if (!(ok = oz_wait(tempty(buf), ((ql - OZ_NBUF) / OZ_NBUF) & 1, abort, wait.ns))) break;
+                                if (!(ok = oz_wait(tempty(buf), ((ql - OZ_NBUF) / OZ_NBUF) & 1, abort))) break;
                                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             }
                             // X block rows: [-Xi | Xr | Xi]; w1 = [Xr | Xi], w2 = [-Xi | Xr]
@@ -401,7 +401,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
             if (ok && g > 0) {
                 // the last commit has landed: every MMA of the CTA has finished
                 const int jx = (g - 1) % OZ_NXS, ux = (g - 1) / OZ_NXS;
-                ok = oz_wait(empty_x(jx), ux & 1, abort, wait.ns);
+                ok = oz_wait(empty_x(jx), ux & 1, abort);
             }
             if (!ok) {
                 *abort = 1;
@@ -425,7 +425,7 @@ k_oz_gemm(const unsigned char *DA, const unsigned char *DX, const int *exA, cons
 #pragma unroll 1
                 for (int L = 0; L < NL; ++L) {
                     const int ql = g * NL + L, buf = ql % OZ_NBUF;
-                    ok = __all_sync(0xffffffffu, oz_wait(tfull(buf), (ql / OZ_NBUF) & 1, abort, wait.ns));
+                    ok = __all_sync(0xffffffffu, oz_wait(tfull(buf), (ql / OZ_NBUF) & 1, abort));
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const float w = ldexpf(1.0f, -8 * (L + 2));
@@ -546,7 +546,7 @@ template <int SA> static void ozaki_product(cudaStream_t s, const OzakiX &ox, co
     const int grid = (int)std::min<long>(ntiles, oz_device_sms());
     cudaEvent_t ev = kt_begin(s);
     NRLTB_LAUNCH(k_oz_gemm<SA>, grid, OZ_THREADS, OZ_SMEM, s, DA, (const unsigned char *)ox.DX, exA, ox.exX, Y, n,
-                 np, batch, g_fault_word, ox.wait);
+                 np, batch, g_fault_word, ox.hold);
     kt_end(ev, s, KC_DIGIT_GEMM, 8.0 * n * (double)n * n * batch);
 }
 

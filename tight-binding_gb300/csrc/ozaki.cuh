@@ -10,7 +10,7 @@ struct OzakiX {
     __nv_bfloat16 *DA, *DX;    // digit planes of A (reused for each A) and of X
     int *exA, *exX;            // per-row (A) and per-column (X) binary exponents
     int n, np, batch;          // order, order padded to a multiple of 128, matrices
-    TcWait wait;               // of the product kernel
+    int hold = 0;              // tests: arrivals that the barriers of emptied accumulators wait for in vain
 };
 
 size_t ozaki_work_bytes(int n, int batch);

@@ -81,7 +81,7 @@ struct ZProduct {
     int order, per, gb;   // tile order, tiles of one matrix, matrices of a group
     double2 *C;
     long ldc, sC;
-    TcWait wait;
+    int hold;             // ZScratch
 };
 }  // namespace
 
@@ -397,7 +397,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
     if (tid == 0) {
         for (int q = 0; q < Z_NBAR; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar0 + 8u * q),
-                         "r"(q >= 2 * ZD + 4 && q < 2 * ZD + 8 ? Z_FOLD + g.wait.hold : 1) : "memory");
+                         "r"(q >= 2 * ZD + 4 && q < 2 * ZD + 8 ? Z_FOLD + g.hold : 1) : "memory");
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -422,7 +422,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                 const unsigned char *px = g.DX + (((long)b * g.nt + jt) * g.kc) * ZD * Z_TILE;
                 for (int kc = c0; kc < c1 && ok; ++kc, ++c)
                     for (int p = ZD - 1; p >= 0; --p) {
-                        if (c > 0 && !(ok = oz_wait(empty(p), (c - 1) & 1, abort, g.wait.ns))) {
+                        if (c > 0 && !(ok = oz_wait(empty(p), (c - 1) & 1, abort))) {
                             stop = p + 1;
                             break;
                         }
@@ -463,7 +463,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                     for (int L = ZL - 1; L >= 0; --L) {
                         if (!ok) break;
                         const int q = 7 - L, buf = q & 3, use = 2 * c + (q >> 2);
-                        if (use > 0) ok = oz_wait(tempty(buf), (use - 1) & 1, abort, g.wait.ns);
+                        if (use > 0) ok = oz_wait(tempty(buf), (use - 1) & 1, abort);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                         const uint32_t tl = tmem + 128u * buf;
                         // pairs (sd, L - sd) from the middle outwards: the slots that the
@@ -475,7 +475,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                             const int sd = (u & 1) ? mid - (u + 1) / 2 : mid + u / 2, td = L - sd;
                             if (L == ZL - 1 || (L == ZL - 2 && (sd == 0 || td == 0))) {
                                 // first reads of this chunk's slots
-                                if (ok) ok = oz_wait(full(sd), c & 1, abort, g.wait.ns) && oz_wait(full(td), c & 1, abort, g.wait.ns);
+                                if (ok) ok = oz_wait(full(sd), c & 1, abort) && oz_wait(full(td), c & 1, abort);
                                 if (!ok) break;
                                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                             }
@@ -491,7 +491,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
                     }
                 }
             }
-            if (ok && c > 0) ok = oz_wait(empty(0), (c - 1) & 1, abort, g.wait.ns);   // every MMA has finished
+            if (ok && c > 0) ok = oz_wait(empty(0), (c - 1) & 1, abort);   // every MMA has finished
             if (!ok) {
                 *abort = 1;
                 atomicOr(fault ? fault : &g_z64_fault, 1u);
@@ -542,7 +542,7 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
 #pragma unroll
                 for (int lp = 0; lp < 4; ++lp) {
                     const int buf = (2 * lp) & 3, use = 2 * c + (lp >> 1);
-                    if (ok) ok = oz_wait(tfull(buf), use & 1, abort, g.wait.ns) && oz_wait(tfull(buf + 1), use & 1, abort, g.wait.ns);
+                    if (ok) ok = oz_wait(tfull(buf), use & 1, abort) && oz_wait(tfull(buf + 1), use & 1, abort);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -746,7 +746,7 @@ bool zgemm64_launch(cudaStream_t s, const GemmArgs<double> &g, const ZScratch &z
         p.C = g.C + b0 * g.sC;
         p.ldc = g.ldc;
         p.sC = g.sC;
-        p.wait = zs.wait;
+        p.hold = zs.hold;
         p.order = g.triC == 1   ? Z_LOWER
                   : g.triA == 1 ? Z_ROWS_DOWN
                   : g.triA == 2 ? Z_ROWS_UP
