@@ -67,7 +67,7 @@ int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int n, int k, i
                               int triB, int triC, double alpha, double beta, const double *A, int lda, const double *B,
                               int ldb, double *C, int ldc, size_t scratch);
 
-/* One digit product (1 the refinement's, 2 the FP64 GEMM's) of order n >= 128 on zeros,
+/* One product (0 the FP32 GEMM's, 1 the refinement's, 2 the FP64 GEMM's) of order n >= 128 on zeros,
  * one of whose barrier waits is sure to run out, after two seconds: returns
  * NRLTB_E_TIMEOUT if the kernel raised its own fault flag and no other (and clears it),
  * NRLTB_OK if it did not. */

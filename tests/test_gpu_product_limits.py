@@ -1,4 +1,4 @@
-"""The digit products at their limits: barrier waits that run out, digit scratch for a part of the batch."""
+"""The tensor-core products at their limits: barrier waits that run out, digit scratch for a part of the batch."""
 import ctypes as C
 
 import numpy as np
@@ -33,8 +33,9 @@ def _scratch(m, n, k, matrices):
     return ((mt + nt) * kc * 7 * 16384 + 8 * (mt * 128 + nt * 64)) * matrices + 1024
 
 
-@pytest.mark.parametrize("kernel", [1, 2])
-@pytest.mark.parametrize("n,batch", [(128, 1), (160, 300), (385, 5)])
+# (the FP32 product's CTAs wait one wave after another: no batch above one wave)
+@pytest.mark.parametrize("kernel,n,batch", [(0, 128, 1), (0, 385, 5)] +
+                         [(k, n, batch) for k in (1, 2) for n, batch in ((128, 1), (160, 300), (385, 5))])
 def test_wait_that_runs_out_is_reported_and_leaves_nothing_behind(ctx, kernel, n, batch):
     """The wait for an accumulator that is never said to be empty: the kernel gives up after its two seconds, says so,
     and the products after it are those before it, bit for bit."""

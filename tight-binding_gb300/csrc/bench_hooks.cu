@@ -365,10 +365,10 @@ extern "C" int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int 
 // one product on zeros whose wait for an emptied accumulator runs out
 extern "C" int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int batch)
 {
-    if (!ctx || (kernel != 1 && kernel != 2) || n < 128 || batch < 1) return NRLTB_E_ARG;
+    if (!ctx || kernel < 0 || kernel > 2 || n < 128 || batch < 1) return NRLTB_E_ARG;
     cudaStream_t s = nrltb_ctx_stream_internal(ctx);
     const size_t nn = (size_t)n * n * batch;
-    const size_t scratch = kernel == 1 ? ozaki_work_bytes(n, batch) : zgemm64_scratch_bytes(n, batch);
+    const size_t scratch = kernel == 0 ? 256 : kernel == 1 ? ozaki_work_bytes(n, batch) : zgemm64_scratch_bytes(n, batch);
     DevBufs d;
     for (int q = 0; q < 3; ++q)
         if (cudaMalloc(&d.p[q], sizeof(double2) * nn) != cudaSuccess) return NRLTB_E_NOMEM;
@@ -377,7 +377,11 @@ extern "C" int nrltb_bench_wait_runs_out(nrltb_ctx *ctx, int kernel, int n, int 
               cudaMemsetAsync(d.p[1], 0, sizeof(double2) * nn, s) == cudaSuccess;
     const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
     const double2 *A = (const double2 *)d.p[0], *B = (const double2 *)d.p[1];
-    if (kernel == 1) {
+    if (kernel == 0) {
+        zgemm_umma_launch(s, gemm_args<float>(n, n, n, batch, make_float2(1, 0), (const float2 *)A, n, (long)n * n, 0,
+                                              (const float2 *)B, n, (long)n * n, 0, make_float2(0, 0), (float2 *)d.p[2], n,
+                                              (long)n * n, 0, 0, 0), 1);
+    } else if (kernel == 1) {
         OzakiX ox = ozaki_prepare_x(s, (float2 *)d.p[1], n, batch, d.p[3]);
         ox.hold = 1;
         ozaki_gemm(s, ox, A, (double2 *)d.p[2]);

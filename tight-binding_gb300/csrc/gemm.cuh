@@ -199,7 +199,8 @@ __global__ static void __launch_bounds__(ZGEMM_SMALL_THREADS) zgemm_small_kernel
 // op(A) = A (gemm_umma.cu), mma.sync otherwise (gemm_tc.cu)
 void zgemm_tc_launch(cudaStream_t s, const GemmArgs<float> &g);
 bool zgemm_umma_supported(const GemmArgs<float> &g);
-void zgemm_umma_launch(cudaStream_t s, const GemmArgs<float> &g);
+// hold (tests): arrivals that the barrier of the MMAs waits for in vain
+void zgemm_umma_launch(cudaStream_t s, const GemmArgs<float> &g, int hold = 0);
 // fault flag of the tcgen05 kernel (a barrier wait that ran out); clear resets it
 unsigned zgemm_umma_fault(bool clear);
 

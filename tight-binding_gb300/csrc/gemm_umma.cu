@@ -32,7 +32,7 @@ constexpr int UM_THREADS = 256;
 constexpr int UM_APL = UM_BM * 128;          // one A plane: 128 rows x 32 TF32 (128 B)
 constexpr int UM_BPL = 2 * UM_BN * 128;      // one B plane: rows Br | Bi
 constexpr int UM_STAGE = 4 * UM_APL + 2 * UM_BPL;   // A: re h, re l, im h, im l; B: h, l
-constexpr int UM_SMEM = UM_STAGE + 1024 + 64;        // one stage, alignment slack, barrier
+constexpr int UM_SMEM = UM_STAGE + 1024 + 64;        // one stage, alignment slack, barriers
 constexpr uint32_t UM_TMEM_COLS = 256;               // P | Q
 constexpr unsigned long long UM_WAIT_NS = 2000000000ull;
 
@@ -97,6 +97,12 @@ __device__ bool um_wait(uint32_t bar, uint32_t parity)
     }
 }
 
+// the barrier's arrival once every MMA issued so far has finished
+__device__ __forceinline__ void um_commit(uint32_t bar)
+{
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void um_ld16(uint32_t taddr, float v[16])
 {
     uint32_t r[16];
@@ -141,7 +147,7 @@ __device__ __forceinline__ void um_put4(unsigned char *ph, unsigned char *pl, ui
 }
 
 template <int TB>   // 1: op(B) = B^H
-__global__ void __launch_bounds__(UM_THREADS, 2) zgemm_umma_kernel(GemmArgs<float> g, int va, int vb, unsigned *fault)
+__global__ void __launch_bounds__(UM_THREADS, 2) zgemm_umma_kernel(GemmArgs<float> g, int va, int vb, unsigned *fault, int hold)
 {
     extern __shared__ __align__(16) unsigned char um_raw[];
     const int b = blockIdx.z;
@@ -163,7 +169,7 @@ __global__ void __launch_bounds__(UM_THREADS, 2) zgemm_umma_kernel(GemmArgs<floa
     const uint32_t raw_s = um_smem_addr(um_raw);
     unsigned char *base = um_raw + (((raw_s + 1023u) & ~1023u) - raw_s);
     uint64_t *bar = (uint64_t *)(base + UM_STAGE);
-    uint32_t *tslot = (uint32_t *)(bar + 1);
+    uint32_t *tslot = (uint32_t *)(bar + 2);
     const uint32_t bar0 = um_smem_addr(bar);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -173,7 +179,8 @@ __global__ void __launch_bounds__(UM_THREADS, 2) zgemm_umma_kernel(GemmArgs<floa
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar0) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar0), "r"(1 + hold) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar0 + 8u) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -309,8 +316,7 @@ __global__ void __launch_bounds__(UM_THREADS, 2) zgemm_umma_kernel(GemmArgs<floa
                 um_mma(tp, arh, bh, 1u);
                 um_mma(tq, aih, bh, 1u);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                         :: "r"(bar0) : "memory");
+            um_commit(bar0);
         }
     }
     if (!fail && nk > 0) {
@@ -319,9 +325,12 @@ __global__ void __launch_bounds__(UM_THREADS, 2) zgemm_umma_kernel(GemmArgs<floa
         if (__syncthreads_or(!ok)) fail = true;
     }
     if (fail) {
-        if (tid == 0) atomicOr(fault ? fault : &g_umma_fault, 1u);
-        // give MMAs still in flight a second bounded wait before the memory is released
-        if (tid == 0 && nk > 0) um_wait(bar0, (nk - 1) & 1);
+        // MMAs still in flight finish, on a barrier of their own, before the memory is released
+        if (tid == 0) {
+            atomicOr(fault ? fault : &g_umma_fault, 1u);
+            um_commit(bar0 + 8u);
+            um_wait(bar0 + 8u, 0);
+        }
     } else {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int q = warp & 3, h = warp >> 2;
@@ -386,7 +395,7 @@ bool zgemm_umma_supported(const GemmArgs<float> &g)
     return g.opA == 0;
 }
 
-void zgemm_umma_launch(cudaStream_t s, const GemmArgs<float> &g)
+void zgemm_umma_launch(cudaStream_t s, const GemmArgs<float> &g, int hold)
 {
     smem_attr_at_least(g.opB ? (const void *)zgemm_umma_kernel<1> : (const void *)zgemm_umma_kernel<0>, UM_SMEM);
     dim3 grid(cdiv(g.m, UM_BM), cdiv(g.n, UM_BN), g.batch);
@@ -394,8 +403,8 @@ void zgemm_umma_launch(cudaStream_t s, const GemmArgs<float> &g)
     // 16-byte aligned: an aligned base, even leading dimension and batch stride
     const int va = ((uintptr_t)g.A % 16 == 0) && g.lda % 2 == 0 && g.sA % 2 == 0;
     const int vb = ((uintptr_t)g.B % 16 == 0) && g.ldb % 2 == 0 && g.sB % 2 == 0;
-    if (g.opB) NRLTB_LAUNCH(zgemm_umma_kernel<1>, grid, UM_THREADS, UM_SMEM, s, g, va, vb, g_fault_word);
-    else NRLTB_LAUNCH(zgemm_umma_kernel<0>, grid, UM_THREADS, UM_SMEM, s, g, va, vb, g_fault_word);
+    if (g.opB) NRLTB_LAUNCH(zgemm_umma_kernel<1>, grid, UM_THREADS, UM_SMEM, s, g, va, vb, g_fault_word, hold);
+    else NRLTB_LAUNCH(zgemm_umma_kernel<0>, grid, UM_THREADS, UM_SMEM, s, g, va, vb, g_fault_word, hold);
 }
 
 unsigned zgemm_umma_fault(bool clear)
