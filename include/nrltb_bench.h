@@ -67,6 +67,12 @@ int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int n, int k, i
                               int triB, int triC, double alpha, double beta, const double *A, int lda, const double *B,
                               int ldb, double *C, int ldc, size_t scratch);
 
+/* The FP64 tridiagonalisation's scalars for n values x, y, z (one array after another):
+ * out, n values each: root and reciprocal root of x (tc_root), reciprocal (tc_recip),
+ * CUDA's sqrt(x), 1 / sqrt(x) and 1 / x, and the reflector of (x + i y, |rest|^2 = z)
+ * (tc_reflector): tau, scale (real and imaginary parts) and beta. */
+int nrltb_bench_fp64_scalars(nrltb_ctx *ctx, int n, const double *in, double *out);
+
 /* One product (0 the FP32 GEMM's, 1 the refinement's, 2 the FP64 GEMM's) of order n >= 128 on zeros,
  * one of whose barrier waits is sure to run out, after two seconds: returns
  * NRLTB_E_TIMEOUT if the kernel raised its own fault flag and no other (and clears it),

@@ -39,8 +39,7 @@ def _check(ctx, H, precision, norm=None):
 @pytest.mark.parametrize("precision,n", [(abi.PREC_FP64, n) for n in (1, 2, 9, 20, 64, 128, 200)] +
                          [(abi.PREC_MIXED, n) for n in (1, 2, 9, 16)])
 def test_zero_blocks(ctx, precision, n):
-    u = np.random.default_rng(n).normal(size=n) + 1j
-    H = [np.zeros((n, n), complex), np.outer(u, u.conj())]
+    H = [np.zeros((n, n), complex)]
     if n > 1:
         H += _two_blocks(n, 0.0, n) + _two_blocks(n, 1e-15, n)
     _check(ctx, H, precision)

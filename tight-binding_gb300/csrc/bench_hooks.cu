@@ -6,6 +6,7 @@
 #include "gemm.cuh"
 #include "dfgemm.cuh"
 #include "ozaki.cuh"
+#include "tri_col.cuh"
 
 using namespace nrltb;
 void nrltb_internal_set_error(const char *msg);
@@ -359,6 +360,34 @@ extern "C" int nrltb_bench_zgemm_scratch(nrltb_ctx *ctx, int method, int m, int 
         ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
     }
     cudaFree(z);
+    return ok && cudaGetLastError() == cudaSuccess ? NRLTB_OK : NRLTB_E_CUDA;
+}
+
+// the FP64 scalars of the column chain beside CUDA's own
+__global__ void k_fp64_scalars(const double *in, double *out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = in[i];
+    double s, r, beta;
+    double2 tau, scale;
+    tc_root(x, s, r);
+    tc_reflector(make_double2(x, in[n + i]), in[2 * n + i], tau, scale, beta);
+    const double v[11] = {s, r, tc_recip(x), sqrt(x), 1.0 / sqrt(x), 1.0 / x, tau.x, tau.y, scale.x, scale.y, beta};
+    for (int q = 0; q < 11; ++q) out[(long)q * n + i] = v[q];
+}
+
+extern "C" int nrltb_bench_fp64_scalars(nrltb_ctx *ctx, int n, const double *in, double *out)
+{
+    if (!ctx || n < 1 || !in || !out) return NRLTB_E_ARG;
+    cudaStream_t s = nrltb_ctx_stream_internal(ctx);
+    DevBufs d;
+    if (cudaMalloc(&d.p[0], sizeof(double) * 3 * n) != cudaSuccess || cudaMalloc(&d.p[1], sizeof(double) * 11 * n) != cudaSuccess)
+        return NRLTB_E_NOMEM;
+    bool ok = cudaMemcpyAsync(d.p[0], in, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s) == cudaSuccess;
+    k_fp64_scalars<<<cdiv(n, 128), 128, 0, s>>>((const double *)d.p[0], (double *)d.p[1], n);
+    ok = ok && cudaMemcpyAsync(out, d.p[1], sizeof(double) * 11 * n, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+    ok = cudaStreamSynchronize(s) == cudaSuccess && ok;
     return ok && cudaGetLastError() == cudaSuccess ? NRLTB_OK : NRLTB_E_CUDA;
 }
 

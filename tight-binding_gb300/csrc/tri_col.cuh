@@ -98,7 +98,7 @@ __device__ __forceinline__ void tc_root(float x, float &s, float &r)
 }
 
 // The reflector of (al, x), |x|^2 = xn2: H (al, x) = (beta, 0) with v = (1, scale x).
-// FP64: one chain of 13 operations from the FP32 root and reciprocal, each followed by
+// FP64: one chain of 14 operations from the FP32 root and reciprocal, each followed by
 // one step of third order (relative errors 2^-22 -> 2^-64, then FP64 rounding):
 //   1/sqrt(N):  y + y e (1/2 + 3/8 e),  e = 1 - N y^2;  the root N y takes the same step
 //   1/D:        r + r (e + e^2),        e = 1 - D r
@@ -118,8 +118,8 @@ __device__ __forceinline__ void tc_reflector(double2 al, double xn2, double2 &ta
         e &= ~1;
         const double m = __hiloint2double(__double2hiint(N) - (e << 20), __double2loint(N));   // [1, 4)
         const double y0 = f2d_exact(rsqrtf(d2f_rn(m))), g0 = m * y0, r = fma(-g0, y0, 1.0);
-        const double p = fma(0.375, r, 0.5) * r;
-        g = fma(g0, p, g0);
+        const double p = fma(0.375, r, 0.5) * r, h = 0.5 * fma(m, y0, -g0);   // (half of g0's own rounding)
+        g = g0 + fma(g0, p, h);
         y = fma(y0, p, y0);
         g = __hiloint2double(__double2hiint(g) + ((e / 2) << 20), __double2loint(g));
         y = __hiloint2double(__double2hiint(y) - ((e / 2) << 20), __double2loint(y));

@@ -121,6 +121,7 @@ GPU_SYMBOLS = [
                                                                                 C.c_int]),
     ("nrltb_bench_zgemm_scratch", C.c_int, [_vp] + [C.c_int] * 10 + [C.c_double] * 2 + [_vp, C.c_int, _vp, C.c_int, _vp,
                                                                                     C.c_int, C.c_size_t]),
+    ("nrltb_bench_fp64_scalars", C.c_int, [_vp, C.c_int, _vp, _vp]),
     ("nrltb_bench_wait_runs_out", C.c_int, [_vp, C.c_int, C.c_int, C.c_int]),
     ("nrltb_bench_umma_fault", C.c_int, [C.c_int]),
     ("nrltb_bench_raise_fault_word", C.c_int, [_vp]),
