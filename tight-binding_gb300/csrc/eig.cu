@@ -110,20 +110,11 @@ __global__ void k_from_unit(double2 *Wi, const int *ex, int n)
     for (int r = threadIdx.x; r < n; r += blockDim.x) w[r] = make_double2(w[r].x * d, w[r].y * d);
 }
 
-template <typename C2>
-__global__ void k_convert_h(const double2 *__restrict__ src, C2 *__restrict__ dst, long count)
+__global__ void k_convert_h(const double2 *__restrict__ src, float2 *__restrict__ dst, long count)
 {
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < count; i += (long)gridDim.x * blockDim.x) {
-        double2 v = src[i];
-        C2 o;
-        if constexpr (sizeof(o.x) == 4) {   // rounded with integer operations, off the FP64 pipe
-            o.x = d2f_rn(v.x);
-            o.y = d2f_rn(v.y);
-        } else {
-            o.x = v.x;
-            o.y = v.y;
-        }
-        dst[i] = o;
+        const double2 v = src[i];
+        dst[i] = make_float2(d2f_rn(v.x), d2f_rn(v.y));   // rounded with integer operations, off the FP64 pipe
     }
 }
 
@@ -209,7 +200,8 @@ __global__ void __launch_bounds__(256) k_potrf_diag(EigWork<float> w, int j0, in
 
 // ---------------------------------------------------------------------------
 // Tridiagonal eigenvalues: Sturm-count bisection inside each unreduced block.
-// the same from per-row split flags (split after row k) in shared memory
+// The block of row r from per-row split flags (T splits between rows k and k + 1 where e[k]
+// is negligible: |d_k d_(k+1)| ulp^2 + DBL_MIN >= e_k^2) in shared memory
 __device__ inline void find_block_flags(const unsigned char *sp, int n, int r, int &b0, int &b1)
 {
     b0 = r;
@@ -218,21 +210,6 @@ __device__ inline void find_block_flags(const unsigned char *sp, int n, int r, i
     while (b1 < n - 1 && !sp[b1]) ++b1;
 }
 
-__device__ inline void find_block(const double *d, const double *e, int n, int r, int &b0, int &b1)
-{
-    const double ulp = DBL_EPSILON;
-    auto split = [&](int k) {   // negligible e[k]: split between rows k and k+1
-        return fabs(d[k] * d[k + 1]) * ulp * ulp + DBL_MIN >= e[k] * e[k];
-    };
-    b0 = r;
-    while (b0 > 0 && !split(b0 - 1)) --b0;
-    b1 = r;
-    while (b1 < n - 1 && !split(b1)) ++b1;
-}
-
-template <typename TB> __device__ inline TB tiny_of();
-template <> __device__ inline float tiny_of<float>() { return FLT_MIN; }
-template <> __device__ inline double tiny_of<double>() { return DBL_MIN; }
 // Quotient in the tridiagonal recurrences: FP32 takes the reciprocal-based
 // quotient (2 ulp; |b| stays below 2^126 there), FP64 the IEEE one.  The FP32
 // eigenpairs are refined to FP64 accuracy afterwards.
@@ -337,7 +314,7 @@ __device__ __forceinline__ void octasect(const float *sd, const float *se2, int 
 }
 
 // One thread per (matrix, row r): eigenvalue number r - b0 of r's block, FP32.
-// The matrix's d and e^2 in FP32 and the split flags of find_block are staged
+// The matrix's d and e^2 in FP32 and the split flags of its rows are staged
 // once per CTA in shared memory (2 n floats + n bytes of dynamic shared memory),
 // so the Sturm chains read them without a conversion from FP64 per step and the
 // block search needs no FP64 work (the values are the same).
@@ -353,7 +330,6 @@ __global__ void k_tri_bisect32(const double *dd, const double *ee, double *lamlo
         sd[k] = d2f_rn(d[k]);
         const float ek = d2f_rn(e[k]);
         se2[k] = ek * ek;
-        // find_block's split test, once per row
         ssp[k] = k < n - 1 && fabs(d[k] * d[k + 1]) * DBL_EPSILON * DBL_EPSILON + DBL_MIN >= e[k] * e[k];
     }
     __syncthreads();
@@ -364,7 +340,7 @@ __global__ void k_tri_bisect32(const double *dd, const double *ee, double *lamlo
     block_bounds(d, e, valid, b0, b1, lo, hi, tnorm, emax2);
     if (!valid) return;
     const float eps = eps_of<float>();
-    const float pivmin = tiny_of<float>() * float(fmax(1.0, emax2));
+    const float pivmin = FLT_MIN * float(fmax(1.0, emax2));
     const float atol = eps * float(tnorm);
     const int j = r - b0;
     float a = float(lo) - 2.f * atol - pivmin, z = float(hi) + 2.f * atol + pivmin;
@@ -605,7 +581,7 @@ __global__ void k_tri_bisect64(const double *dd, const double *ee, double *lamlo
             const float w = 4.f * eps_of<float>() * (float)tnorm;
             fa -= w;
             fz += w;
-            octasect(sd, se2, b0, b1, j, eps_of<float>() * (float)tnorm, tiny_of<float>(), fa, fz);
+            octasect(sd, se2, b0, b1, j, eps_of<float>() * (float)tnorm, FLT_MIN, fa, fz);
             // the FP32 interval widened by its own error, then checked
             const double m = 4.0 * (double)eps_of<float>() * tnorm;
             a = fmax(glo, (double)fa - m);
@@ -1160,15 +1136,14 @@ __global__ void __launch_bounds__(256) k_inv_pair(EigWork<T> w)
 
 // Rows t0.. of the panel's V columns j0..j0+jb into columns 0..jb and
 // 2 EIG_NB.. of VW (W sits in between), for the merged trailing update
-template <typename C2>
-__global__ void k_copy_vpanel(const C2 *V, long ld, long ms, C2 *VW, long ldw, long wps, int t0, int j0, int jb,
+__global__ void k_copy_vpanel(const float2 *V, long ld, long ms, float2 *VW, long ldw, long wps, int t0, int j0, int jb,
                               int rem)
 {
     const long e = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (e >= (long)rem * jb) return;
     const int b = blockIdx.y, r = (int)(e % rem), c = (int)(e / rem);
-    const C2 v = V[b * ms + t0 + r + (long)(j0 + c) * ld];
-    C2 *o = VW + b * wps + t0 + r;
+    const float2 v = V[b * ms + t0 + r + (long)(j0 + c) * ld];
+    float2 *o = VW + b * wps + t0 + r;
     o[(long)c * ldw] = v;
     o[(long)(2 * EIG_NB + c) * ldw] = v;
 }
@@ -1242,8 +1217,8 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
     // 0. inputs in working precision: S -> L, H -> A (A is free until step 3)
     int *const ex = (int *)w.d;   // FP64: exponents of D, until step 4
     if constexpr (sizeof(T) == 4) {
-        NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, S, w.L, cnt);
-        NRLTB_LAUNCH(k_convert_h<C2>, 1184, 256, 0, s, H, w.A, cnt);
+        NRLTB_LAUNCH(k_convert_h, 1184, 256, 0, s, S, w.L, cnt);
+        NRLTB_LAUNCH(k_convert_h, 1184, 256, 0, s, H, w.A, cnt);
     } else {
         NRLTB_LAUNCH(k_unit_exp, cdiv((long)n * B, 128), 128, 0, s, S, ex, n, B);
         NRLTB_LAUNCH(k_to_unit, dim3((unsigned)std::min(cdiv((long)n * n, 256), 512), B), 256, 0, s, S, H, w.L, w.A, ex, n);
@@ -1320,7 +1295,7 @@ void eig_solve(cudaStream_t s, EigWork<T> &w, const double2 *H, const double2 *S
             if (jb == EIG_NB) {
                 // A -= [Vp Wp] [Wp Vp]^H in one rank-64 update: Vp copied on both sides of W
                 if constexpr (sizeof(T) == 4)
-                    NRLTB_LAUNCH(k_copy_vpanel<C2>, dim3(cdiv((long)rem * jb, 256), B), 256, 0, s, w.V, ld, ms, w.VW,
+                    NRLTB_LAUNCH(k_copy_vpanel, dim3(cdiv((long)rem * jb, 256), B), 256, 0, s, w.V, ld, ms, w.VW,
                                  (long)n, w.wps, t0, j0, jb, rem);
                 else
                     NRLTB_LAUNCH(k_scale_vpanel, dim3(jb, B), 256, 0, s, w.V, ld, ms, w.VW, (long)n, w.wps, t0, j0, rem);

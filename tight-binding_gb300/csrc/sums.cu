@@ -76,7 +76,7 @@ __device__ __forceinline__ int count_below(const double *e, int m, double x)
 constexpr int FERMI_CL = 8, FERMI_THREADS = 128, FERMI_ROW_MIN = 64;
 constexpr int FERMI_WARPS = FERMI_CL * FERMI_THREADS / 32;
 
-struct FermiSlot { double v[6]; };
+struct FermiSlot { double v[5]; };   // the edges; a Newton step's two sums take four
 
 // The CTA's two sums into its slot; the cluster's totals to every thread.  A merge is eight
 // dependent FP64 operations, so the two sums are merged side by side, one by each half of a

@@ -36,8 +36,7 @@ namespace nrltb {
 constexpr int TP_STRIPS = 8;  // column strips of a row tile's mat-vec, each summed by itself
 constexpr int TP_RANKS = 8;   // tiles t mod TP_RANKS are summed first, whatever the cluster size
 
-// values per lane of one butterfly (16: 16 warps fit an SM)
-template <typename T> struct TpNV { static constexpr int v = 16; };
+constexpr int TP_NV = 16;     // values per lane of one butterfly (16: 16 warps fit an SM)
 
 // A column whose elements' squares fall out of the range (2^-63 in FP32, 2^-511 in FP64) is
 // left as it is: its reflector would be a quotient of zeros.  xn2: |x|^2 of the elements
@@ -157,7 +156,7 @@ __device__ __forceinline__ void tp_strip(const typename cplx<T>::t *A, long ld, 
                                          int lane)
 {
     typedef typename cplx<T>::t C2;
-    constexpr int NV = TpNV<T>::v;
+    constexpr int NV = TP_NV;
     // columns [u0, u0 + 8) of the half h of the strip's tile S, zero outside the trailing matrix
     auto fetch = [&](C2 (&a)[8], int S, int h, int u0) {
         const bool trans = S > R, diag = S == R;
@@ -221,9 +220,8 @@ __device__ __forceinline__ void tp_strip(const typename cplx<T>::t *A, long ld, 
         }
         if (has_upper) {
             tp_butterfly<NV>(x, lane);
-            constexpr int sh = (NV == 32) ? 0 : (NV == 16 ? 1 : 2);
-            if ((lane & ((1 << sh) - 1)) == 0) {
-                C2 &dst = yp[h * NV + (lane >> sh)];
+            if ((lane & 1) == 0) {   // two lanes hold each sum
+                C2 &dst = yp[h * NV + (lane >> 1)];
                 dst = cadd(dst, x[0]);
             }
         }
@@ -236,7 +234,7 @@ __global__ void __launch_bounds__(32 * NW, 16 / NW) k_tri_panel(EigWork<T> w, in
 {
     typedef typename cplx<T>::t C2;
     namespace cg = cooperative_groups;
-    constexpr int NV = TpNV<T>::v, NR = TP_RANKS / CL;   // ranks of this CTA
+    constexpr int NV = TP_NV, NR = TP_RANKS / CL;   // ranks of this CTA
     extern __shared__ __align__(16) unsigned char tp_raw[];
     cg::cluster_group cluster = cg::this_cluster();
     const int q = (int)cluster.block_rank();

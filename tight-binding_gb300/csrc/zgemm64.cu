@@ -581,7 +581,6 @@ __global__ void __maxnreg__(96) k_z_gemm(ZProduct g, unsigned *fault)
             const int i = it * Z_BM + 32 * q4 + lane, j0 = jt * Z_BN + 16 * h;
             const int ei = g.exA[(long)b * g.mt * Z_BM + i];
             const bool badrow = ei == Z_BAD;
-            const int fj = g.exX[(long)b * g.nt * Z_BN + j0 + (lane & 15)];
             double2 *cp = g.C + b * g.sC + i;
             double2 old[2];
 #pragma unroll
