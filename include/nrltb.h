@@ -42,6 +42,10 @@ extern "C" {
 #define NRLTB_K_TIMEOUT       4  /* a bounded device wait gave up                    */
 
 /* ---- precision forms ---------------------------------------------------- */
+/* Both give eigenvalues to a small multiple of their rounding unit times the norm of
+ * the matrix, not of each eigenvalue: the small ones of a graded matrix have fewer
+ * correct digits.  (FP64 products of order 16 and up carry 55 bits below the largest
+ * element of a row or column, on the tensor cores.) */
 #define NRLTB_PREC_FP64   0      /* plain FP64 drop-in                              */
 #define NRLTB_PREC_MIXED  1      /* FP32 eigensolve + FP64-accurate refinement      */
 

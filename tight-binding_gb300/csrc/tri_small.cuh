@@ -38,9 +38,10 @@ inline size_t ts_smem(int n, int nt)
            sizeof(int) * 2 + (size_t)n;
 }
 
-// shares of the columns for a mat-vec of order m on nt threads: where an SM holds one matrix
-// (n > 96), as many as there are threads, for warps to cover each other's latencies (n = 108:
-// 1.61 -> 1.39 ms with 16 warps); else, with other matrices to do that, the rounds of warps
+// shares of the columns for a mat-vec of order m on nt threads: above n = 96, where an SM holds two
+// matrices at most, as many as there are threads, for warps to cover each other's latencies (16
+// warps against 8 of the other rule, n = 108: 4 to 121 matrices 1.62 -> 1.40 ms, 300 matrices
+// 2.45 -> 2.50, 600 4.89 -> 4.87); else, with other matrices to do that, the rounds of warps
 // over the four quarters times the columns of a share, and the addition of the shares
 __device__ inline int ts_share_count(int m, int nt)
 {

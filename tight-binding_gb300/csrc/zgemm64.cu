@@ -7,10 +7,15 @@
 // and written as an integer below 2^55 in ZD = 7 balanced base-256 digits (one
 // rounding, 2^-56 of the row's or column's largest element, as against 2^-53 of
 // the element itself).  A digit product is an integer that FP32 accumulation
-// sums exactly, so the only further errors are the dropped digit pairs s + t > 7
-// (below 2^-58 of row maximum x column maximum per term) and the last rounding:
-// the sum over k has none, where an FMA chain rounds k times.  Errors against
-// extended precision are in tests/test_gpu_kernel_edges.py.
+// sums exactly, so the further errors are the dropped digit pairs s + t > 7
+// (below 2^-58 of row maximum x column maximum per term), the unit of the
+// 64-bit sums, to which every chunk of 32 k is rounded twice (below), and the
+// last rounding.  In all below K 2^-51 row maximum x column maximum, which
+// tests/test_gpu_kernel_edges.py holds against extended precision; an FMA chain
+// has K 2^-52 of the sum of |a| |b|.  So an element far below its row's largest
+// keeps fewer bits than FP64's 53, and below 2^-56 of it none: what a solve
+// needs is accuracy against the norm, and there the two agree (eig.cu's k_unit_exp
+// and k_scale_vpanel see to the scales that would not cancel).
 //
 // Layout.  A chunk is 32 k.  Plane s of A's 128 rows is one 16 KB tile of the
 // 128-byte-swizzled K-major layout, row i = [re digits of 32 k | im digits]; plane
@@ -27,8 +32,9 @@
 // 2^22.9.  Two levels make a 32-bit integer (256 v_(L-1) + v_L, below 1.9e9) and the
 // four of a chunk are shifted into one 64-bit integer per element, whose unit
 // 2^(e_i + f_j + d - 62) leaves room for the whole sum (d from the row's or the
-// columns' sums of magnitudes, whichever is less), so that it never overflows; what
-// falls below the unit is rounded (2^-63 of the bound on the result).
+// columns' sums of magnitudes, whichever is less), so that it never overflows.  The two
+// higher pairs of levels fall below the unit and are rounded to it: half a unit each, K / 32
+// units in all (at K = 1152 36 units of 2^-62 of the bound on the result).
 //
 // Bound: the MMAs, issued by one thread; sixteen fold warps and the producer run
 // beside them.  Measured figures are at zgemm64_supported below.
